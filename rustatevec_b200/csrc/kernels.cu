@@ -400,166 +400,285 @@ __global__ void __launch_bounds__(kThreads) k_ising(R* __restrict__ re, R* __res
 }
 
 // ---------------------------------------------------------------------------------------------
-// Dense k-qubit sweep on CUDA cores (qsv kernels.cu:91-120 gathers one 2^m block per thread into
-// local arrays; here a CTA gathers a tile of 2^K rows x NC columns into shared memory, where the
-// columns are the NCB lowest non-gate bits, so every global access is a contiguous run of at least
-// NC amplitudes; the tile is then a small complex GEMM Y = U X with U staged in shared memory).
+// Dense k-qubit sweep (qsv kernels.cu:91-120 gathers one 2^m block per thread into local arrays).
+// Matrices are packed row-major, interleaved (re, im) in the state's precision, with the gate's bits
+// in ascending order of their state bits (pack_sweep_matrix). Two kernels; launch_dense_of states
+// which one runs where.
 // ---------------------------------------------------------------------------------------------
-struct DenseP {
-  uint32_t hibits[6];   // tile bits above NCB-1 (ascending), K of them
-  uint64_t hioff[64];   // address offset of the high tile bits
-  uint32_t dsthi[64];   // shared-memory offset of the high tile bits
-  uint32_t dstlo[256];  // shared-memory offset of the low NCB address bits
-  uint32_t vecstore;    // 1 when the low LOG address bits are column bits
+
+// Dense sweep on the FP64 matrix instruction (mma.m8n8k4), no shared-memory staging of the state. A
+// warp owns G groups of 8 columns (the lowest non-gate bits) and computes Y^T = X^T W^T with the real
+// 2M x 2M form W = [[Ur, -Ui], [Ui, Ur]] (M = 2^K): the 8 columns are the instruction's rows, the K
+// index of one instruction is the value of the gate's two lowest state bits, and its 8 result columns
+// are those two bits and (re, im). So lane (column, low gate bits) loads, and later stores, exactly
+// its own amplitudes: the accumulator pair of a lane is (re, im) of one of them. A complex128 load or
+// store instruction touches whole 32-byte sectors wherever the gate bits lie, because state bits 0
+// and 1 are always among its 3 column bits and 2 low gate bits. All loads of the warp's 2^K x 8G
+// amplitudes are in flight before the first product, warps never wait for one another, and each
+// matrix fragment (16 bytes of shared memory a lane) feeds 2 G products. complex64 amplitudes are
+// widened on load and rounded once on store.
+//   The scalar tile it replaces was bound by its operands: every FP64 FMA pair needed a broadcast
+// coefficient from shared memory, and tile, product and write-back were separated by block barriers.
+// Bound now: HBM for K <= 4, the FP64 pipe (37 TFLOP/s measured) for K = 5, 6. Measured on 27-qubit
+// complex128 states (4.3 GB moved), mean over low, middle and high gate bits, before -> after:
+//   K = 2: 0.87 -> 0.68 ms, K = 3: 0.94 -> 0.70 ms, K = 4: 1.39 -> 0.75 ms (5.7 TB/s),
+//   K = 5: 2.26 -> 1.20 ms (28.5 TFLOP/s), K = 6: 3.85 -> 2.02 ms (34 TFLOP/s).
+__device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
+struct DenseMmaP {
+  uint32_t q[6];  // gate bits, ascending
 };
 
-// cp.async copies global -> shared (16 bytes cached in L2 only, or one 4- / 8-byte element).
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
-               "l"(src)
-               : "memory");
-}
-template <class R> __device__ __forceinline__ void cp_async_elem(R* dst, const R* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
-               "l"(src), "n"(int(sizeof(R)))
-               : "memory");
+template <class R, int K, int G, int TH, int MINB>
+__global__ void __launch_bounds__(TH, MINB) k_dense_mma(R* __restrict__ re, R* __restrict__ im, uint64_t nitems,
+                                                        const R* __restrict__ u, DenseMmaP p) {
+  constexpr int M = 1 << K, H = M / 4;  // H: values of the gate bits above the two lowest
+  extern __shared__ __align__(16) char smem_raw[];
+  // fragment (r >> 2, s >> 2): lane 8 (r & 3) + 4 part + (s & 3) holds the two values that multiply the
+  // real and the imaginary part of column s for the real (part 0) or imaginary part of row r
+  double2* ws = reinterpret_cast<double2*>(smem_raw);
+  for (int i = threadIdx.x; i < H * H * 32; i += TH) {
+    const int f = i >> 5, r = (f / H) * 4 + ((i >> 3) & 3), s = (f % H) * 4 + (i & 3);
+    const double ar = u[2 * (r * M + s)], ai = u[2 * (r * M + s) + 1];
+    ws[i] = (i & 4) ? make_double2(ai, ar) : make_double2(ar, -ai);
+  }
+  __syncthreads();
+  const uint32_t lane = threadIdx.x & 31u;
+  uint64_t bit[K];
+#pragma unroll
+  for (int j = 0; j < K; ++j) bit[j] = 1ull << p.q[j];
+  const uint64_t low = ((lane & 1u) ? bit[0] : 0ull) + ((lane & 2u) ? bit[1] : 0ull);
+  auto row = [&](int h) {  // address offset of the higher gate bits' value h
+    uint64_t o = 0;
+#pragma unroll
+    for (int j = 2; j < K; ++j)
+      if ((h >> (j - 2)) & 1) o += bit[j];
+    return o;
+  };
+  const uint64_t nwarps = uint64_t(gridDim.x) * (TH / 32);
+#pragma unroll 1
+  for (uint64_t w = blockIdx.x * uint64_t(TH / 32) + (threadIdx.x >> 5); w < nitems; w += nwarps) {
+    uint64_t base[G];
+    R x[G][2 * H];
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      uint64_t a = (w * G + g) * 8 + (lane >> 2);
+#pragma unroll
+      for (int j = 0; j < K; ++j) {
+        const uint64_t lo = a & (bit[j] - 1ull);
+        a = ((a - lo) << 1) | lo;
+      }
+      base[g] = a + low;
+#pragma unroll
+      for (int h = 0; h < H; ++h) {
+        x[g][2 * h] = re[base[g] + row(h)];
+        x[g][2 * h + 1] = im[base[g] + row(h)];
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < H; ++r) {
+      double y[G][2];
+#pragma unroll
+      for (int g = 0; g < G; ++g) y[g][0] = y[g][1] = 0.0;
+#pragma unroll
+      for (int h = 0; h < H; ++h) {
+        const double2 b = ws[(r * H + h) * 32 + lane];
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          mma_f64(y[g], double(x[g][2 * h]), b.x);
+          mma_f64(y[g], double(x[g][2 * h + 1]), b.y);
+        }
+      }
+      // in place: a lane stores only addresses that it has loaded itself
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        re[base[g] + row(r)] = R(y[g][0]);
+        im[base[g] + row(r)] = R(y[g][1]);
+      }
+    }
+  }
 }
 
-// DB: two tile buffers, the gather of tile i + grid (cp.async) in flight while tile i is
-// multiplied and written back; otherwise one buffer, gathered with vector loads.
-template <class R, int K, int NCB, bool DB>
-__global__ void __launch_bounds__(kThreads) k_dense(R* __restrict__ re, R* __restrict__ im,
-                                                    uint64_t ntiles, const R* __restrict__ ut,
-                                                    DenseP p) {
-  constexpr int M = 1 << K, NC = 1 << NCB, N = VecT<R>::N;
-  constexpr int RG = kThreads / NC;  // row groups
-  constexpr int RPT = M / RG;        // rows per thread
-  constexpr int NB = DB ? 2 : 1;     // tile buffers
-  static_assert(RG * NC == kThreads && RPT * RG == M, "tile shape");
-  extern __shared__ __align__(16) char smem_raw[];
-  R* xbuf = reinterpret_cast<R*>(smem_raw);  // buffer b: re [M * NC], im [M * NC]
-  R* us = xbuf + NB * 2 * M * NC;            // [s][r] complex interleaved
-  uint32_t* dlo = reinterpret_cast<uint32_t*>(us + 2 * M * M);
-  uint32_t* dhi = dlo + NC;
-  uint64_t* hio = reinterpret_cast<uint64_t*>(dhi + M);  // 8-byte aligned: NC + M is even
-  for (int i = threadIdx.x; i < 2 * M * M; i += kThreads) us[i] = ut[i];
-  for (int i = threadIdx.x; i < NC; i += kThreads) dlo[i] = p.dstlo[i];
-  for (int i = threadIdx.x; i < M; i += kThreads) {
-    dhi[i] = p.dsthi[i];
-    hio[i] = p.hioff[i];
-  }
-  const int col = threadIdx.x % NC, rg = threadIdx.x / NC;
-  const bool vs = p.vecstore != 0;
-  auto tile_base = [&](uint64_t tile) {
-    uint64_t base = tile << NCB;
+// complex64 dense sweep of K = 2..4 on paired FP32 FMAs, large states. A thread holds the 2^K rows of 4
+// columns in registers and walks the matrix two or more rows a step: one broadcast coefficient from
+// shared memory feeds 8 paired FMAs. Loads and stores are 16-byte vectors (state bits 0 and 1 are
+// always in the thread: L0 / L1 say which of them are gate bits; as many further column bits, `ext`,
+// above the lanes then make up the 4 columns). The lanes are the lowest remaining bits. Where state
+// bit 2 is a gate bit (L2) a lane's vectors would be half sectors 32 bytes apart, so a lane pair loads
+// whole sectors, trading bit 2 against the lowest lane bit, and swaps back with shuffles.
+//   Before, each product of the shared-memory tile needed one operand from shared memory for every
+// two FMAs and three block barriers a tile. Bound now: HBM (K = 2, 3); FP32 FMA issue together with
+// HBM (K = 4: 240 of 380 us are FMA issue). Measured on 27-qubit states (2.1 GB moved), mean over low,
+// middle and high gate bits, before -> after: K = 2: 0.50 -> 0.36 ms, K = 3: 0.59 -> 0.38 ms,
+// K = 4: 0.77 -> 0.45 ms (0.58 -> 0.38 ms with the gate bits above bit 6).
+struct DenseColP {
+  uint32_t ins[6], nins;  // the register bits (gate bits and state bits 0, 1), ascending
+  uint32_t zero;          // 0: see `fresh`
+  uint64_t hi[4];         // address of the gate bits that are not in the vector
+  uint64_t ext[2];        // address of the extra column bits
+};
+
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ void fma2(f32x2& d, f32x2 a, f32x2 b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+
+template <int K, int L0, int L1, int L2, int TH>
+__global__ void __launch_bounds__(TH, 1) k_dense_cols(float* __restrict__ re, float* __restrict__ im, uint64_t nitems,
+                                                      const float2* __restrict__ u, const __grid_constant__ DenseColP p) {
+  constexpr int M = 1 << K, NL = L0 + L1, NH = K - NL, VH = 1 << NH, NX = 1 << NL, RV = 1 << NL;
+  constexpr int VB = (L2 || (K == 4 && NL == 0)) ? 2 : 1;  // vectors (groups of RV rows) a step
+  constexpr int RB = RV * VB;
+  __shared__ __align__(16) float2 us[M * M];
+  for (int i = threadIdx.x; i < M * M; i += TH) us[i] = u[i];
+  __syncthreads();
+  const uint32_t lane = threadIdx.x & 31u;
+  auto insert = [&](uint64_t x) {
 #pragma unroll
-    for (int j = 0; j < K; ++j) {
-      const uint32_t b = p.hibits[j];
-      const uint64_t lo = base & ((1ull << b) - 1ull);
-      base = ((base - lo) << 1) | lo;
-    }
-    return base;
+    for (int j = 0; j < 6; ++j)
+      if (j < int(p.nins)) {
+        const uint64_t lo = x & ((1ull << p.ins[j]) - 1ull);
+        x = ((x - lo) << 1) | lo;
+      }
+    return x;
   };
-  // the tile's gather into buffer b: contiguous runs of >= NC amplitudes, scattered into the
-  // (row, column) tile layout
-  auto gather = [&](uint64_t base, int b) {
-    R* xr = xbuf + b * 2 * M * NC;
-    R* xi = xr + M * NC;
-    for (int v = threadIdx.x; v < M * NC / N; v += kThreads) {
-      const int t = v * N, tlo = t & (NC - 1), thi = t >> NCB;
-      const uint64_t a = base + hio[thi] + uint64_t(tlo);
-      if constexpr (DB) {
-        if (vs) {
-          const uint32_t d = dlo[tlo] + dhi[thi];
-          cp_async16(xr + d, re + a);
-          cp_async16(xi + d, im + a);
-        } else {
+  const bool up = L2 && (lane & 1u);
+  const uint64_t lane_bit = insert(1);  // state bit of the lowest lane bit
+  const uint64_t lane_off = L2 ? insert(lane & ~1u) + (up ? p.hi[0] : 0ull) : insert(lane);
+  // register bit 0 of the higher rows: with L2 it walks the lane bit's two columns in memory
+  const uint64_t first = L2 ? lane_bit : p.hi[0];
+  auto ext = [&](int x) { return ((x & 1) ? p.ext[0] : 0ull) + ((x & 2) ? p.ext[1] : 0ull); };
+  // vector element e of vector (row group, x): its row within the group and its column
+  auto elem_row = [](int e) { return L0 && L1 ? e : L0 ? (e & 1) : L1 ? (e >> 1) : 0; };
+  auto elem_col = [](int e, int x) { return L0 && L1 ? x : L0 ? ((e >> 1) | (x << 1)) : L1 ? ((e & 1) | (x << 1)) : e; };
+  auto swap = [&](float& v0, float& v1) {  // lane pair: v0 <-> the other lane's v1 crosswise
+    const float got = __shfl_xor_sync(0xffffffffu, up ? v0 : v1, 1);
+    if (up) v0 = got;
+    else v1 = got;
+  };
+  // Column pairs that are not adjacent in a loaded vector (L0) move to their register pair once, here:
+  // without an operation of its own the assembler repeats the moves in every step (K = 4: 0.60 against
+  // 0.46 ms).
+  auto fresh = [&](float v) { return L0 && !L2 ? __uint_as_float(__float_as_uint(v) ^ p.zero) : v; };
+  const uint64_t nwarps = uint64_t(gridDim.x) * (TH / 32);
+#pragma unroll 1
+  for (uint64_t w = blockIdx.x * uint64_t(TH / 32) + (threadIdx.x >> 5); w < nitems; w += nwarps) {
+    const uint64_t base = insert(w << (5 + NL)) + lane_off;
+    asm volatile("" ::: "memory");  // the matrix stays in shared memory (hoisted, it would spill)
+    float xr[M][4], xi[M][4];
 #pragma unroll
-          for (int e = 0; e < N; ++e) {
-            const uint32_t d = dlo[tlo + e] + dhi[thi];
-            cp_async_elem(xr + d, re + a + e);
-            cp_async_elem(xi + d, im + a + e);
-          }
-        }
-      } else {
-        R vr[N], vi[N];
-        vld(re + a, vr);
-        vld(im + a, vi);
-        if (vs) {
-          const uint32_t d = dlo[tlo] + dhi[thi];
-          vst(xr + d, vr);
-          vst(xi + d, vi);
-        } else {
+    for (int v = 0; v < VH; ++v)
 #pragma unroll
-          for (int e = 0; e < N; ++e) {
-            const uint32_t d = dlo[tlo + e] + dhi[thi];
-            xr[d] = vr[e];
-            xi[d] = vi[e];
-          }
+      for (int x = 0; x < NX; ++x) {
+        uint64_t a = base + ext(x) + ((v & 1) ? first : 0ull);
+#pragma unroll
+        for (int j = 1; j < NH; ++j)
+          if ((v >> j) & 1) a += p.hi[j];
+        float fr[4], fi[4];
+        vld(re + a, fr);
+        vld(im + a, fi);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          xr[(v << NL) | elem_row(e)][elem_col(e, x)] = fr[e];
+          xi[(v << NL) | elem_row(e)][elem_col(e, x)] = fi[e];
         }
       }
-    }
-  };
-  __syncthreads();  // tables ready
-  if constexpr (DB) {
-    if (blockIdx.x < ntiles) gather(tile_base(blockIdx.x), 0);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  }
-  int cur = 0;
-  for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, cur ^= NB - 1) {
-    const uint64_t base = tile_base(tile);
-    if constexpr (DB) {
-      // the next tile's gather goes into the other buffer (its last reads ended at the barrier
-      // closing the previous iteration); then wait for this tile's group only
-      const uint64_t nxt = tile + gridDim.x;
-      if (nxt < ntiles) gather(tile_base(nxt), cur ^ 1);
-      asm volatile("cp.async.commit_group;" ::: "memory");
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-    } else {
-      gather(base, 0);
-    }
-    __syncthreads();
-    R* xr = xbuf + cur * 2 * M * NC;
-    R* xi = xr + M * NC;
-    R ar[RPT], ai[RPT];
+    if constexpr (L2) {
 #pragma unroll
-    for (int r = 0; r < RPT; ++r) ar[r] = ai[r] = R(0);
-#pragma unroll 4
-    for (int s = 0; s < M; ++s) {
-      const R vr = xr[s * NC + col], vi = xi[s * NC + col];
-      const R* u = us + 2 * (s * M + rg * RPT);
+      for (int r = 0; r < M; ++r)
+        if (!((r >> NL) & 1))
 #pragma unroll
-      for (int r = 0; r < RPT; ++r) cmac(ar[r], ai[r], u[2 * r], u[2 * r + 1], vr, vi);
+          for (int c = 0; c < 4; ++c) {
+            swap(xr[r][c], xr[r | RV][c]);
+            swap(xi[r][c], xi[r | RV][c]);
+          }
     }
-    __syncthreads();
+    f32x2 pr[M][2], pi[M][2];
 #pragma unroll
-    for (int r = 0; r < RPT; ++r) {
-      xr[(rg * RPT + r) * NC + col] = ar[r];
-      xi[(rg * RPT + r) * NC + col] = ai[r];
-    }
-    __syncthreads();
-    for (int v = threadIdx.x; v < M * NC / N; v += kThreads) {
-      const int t = v * N, tlo = t & (NC - 1), thi = t >> NCB;
-      const uint64_t a = base + hio[thi] + uint64_t(tlo);
-      R vr[N], vi[N];
-      if (vs) {
-        const uint32_t d = dlo[tlo] + dhi[thi];
-        vld(xr + d, vr);
-        vld(xi + d, vi);
-      } else {
+    for (int s = 0; s < M; ++s)
 #pragma unroll
-        for (int e = 0; e < N; ++e) {
-          const uint32_t d = dlo[tlo + e] + dhi[thi];
-          vr[e] = xr[d];
-          vi[e] = xi[d];
-        }
+      for (int c = 0; c < 2; ++c) {
+        pr[s][c] = pack2(fresh(xr[s][2 * c]), fresh(xr[s][2 * c + 1]));
+        pi[s][c] = pack2(fresh(xi[s][2 * c]), fresh(xi[s][2 * c + 1]));
       }
-      vst(re + a, vr);
-      vst(im + a, vi);
+#pragma unroll 1
+    for (int v0 = 0; v0 < VH; v0 += VB) {
+      f32x2 rr[RB][2], ii[RB][2], ri[RB][2];  // sums of ar xr, ai xi, ar xi + ai xr
+#pragma unroll
+      for (int q = 0; q < RB; ++q)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) rr[q][c] = ii[q][c] = ri[q][c] = 0ull;
+      const float2* um = us + (v0 << NL) * M;
+#pragma unroll
+      for (int s = 0; s < M; ++s)
+#pragma unroll
+        for (int q = 0; q < RB; ++q) {
+          const float2 g = um[q * M + s];
+          const f32x2 ar = pack2(g.x, g.x), ai = pack2(g.y, g.y);
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            fma2(rr[q][c], ar, pr[s][c]);
+            fma2(ii[q][c], ai, pi[s][c]);
+            fma2(ri[q][c], ar, pi[s][c]);
+            fma2(ri[q][c], ai, pr[s][c]);
+          }
+        }
+      float yr[RB][4], yi[RB][4];
+#pragma unroll
+      for (int q = 0; q < RB; ++q)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const float2 a = unpack2(rr[q][c]), b = unpack2(ii[q][c]), d = unpack2(ri[q][c]);
+          yr[q][2 * c] = a.x - b.x;
+          yr[q][2 * c + 1] = a.y - b.y;
+          yi[q][2 * c] = d.x;
+          yi[q][2 * c + 1] = d.y;
+        }
+      if constexpr (L2) {
+#pragma unroll
+        for (int q = 0; q < RV; ++q)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            swap(yr[q][c], yr[q + RV][c]);
+            swap(yi[q][c], yi[q + RV][c]);
+          }
+      }
+      uint64_t group = 0;  // address of this step's first row group
+      if (VB == 1 && (v0 & 1)) group += first;
+#pragma unroll
+      for (int j = 1; j < NH; ++j)
+        if ((v0 >> j) & 1) group += p.hi[j];
+      // in place: a thread stores only the vectors that it has loaded itself
+#pragma unroll
+      for (int v = 0; v < VB; ++v)
+#pragma unroll
+        for (int x = 0; x < NX; ++x) {
+          const uint64_t a = base + ext(x) + group + (v ? first : 0ull);
+          float fr[4], fi[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            fr[e] = yr[v * RV + elem_row(e)][elem_col(e, x)];
+            fi[e] = yi[v * RV + elem_row(e)][elem_col(e, x)];
+          }
+          vst(re + a, fr);
+          vst(im + a, fi);
+        }
     }
-    __syncthreads();  // this buffer's reads are done before a later gather reuses it
   }
-  if constexpr (DB) asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 // Small-state fallback: one 2^K block per thread (gather, matvec, scatter).
@@ -568,7 +687,6 @@ __global__ void k_dense_small(R* __restrict__ re, R* __restrict__ im, uint64_t n
                               const R* __restrict__ ut, Enum en, uint32_t q0, uint32_t q1,
                               uint32_t q2, uint32_t q3, uint32_t q4, uint32_t q5) {
   constexpr int M = 1 << K;
-  const R* __restrict__ us = ut;  // small states only: the matrix stays in L1/L2
   const uint32_t qs[6] = {q0, q1, q2, q3, q4, q5};
   for (uint64_t w = gtid(); w < nblocks; w += gstride()) {
     const uint64_t base = enum_base(w, 0, en);
@@ -585,7 +703,7 @@ __global__ void k_dense_small(R* __restrict__ re, R* __restrict__ im, uint64_t n
     for (int r = 0; r < M; ++r) {
       R yr = 0, yi = 0;
 #pragma unroll
-      for (int s = 0; s < M; ++s) cmac(yr, yi, us[2 * (s * M + r)], us[2 * (s * M + r) + 1], xr[s], xi[s]);
+      for (int s = 0; s < M; ++s) cmac(yr, yi, ut[2 * (r * M + s)], ut[2 * (r * M + s) + 1], xr[s], xi[s]);
       uint64_t idx = base;
 #pragma unroll
       for (int j = 0; j < K; ++j) idx |= uint64_t((r >> j) & 1) << qs[j];
@@ -891,100 +1009,134 @@ void launch_diag(const LaunchEnv& env, R* re, R* im, uint32_t n, const Sweep& s)
   check_launch();
 }
 
-// Dense-kernel tile width per (precision, K): NCB column bits. complex128 gates of <= 3 qubits take
-// 256 columns (a CTA loads, multiplies and stores its tile in turn, so a larger tile keeps more
-// bytes in flight per SM; measured 2-19 % faster at 30 qubits, while wider gates measured mixed).
-template <class R> constexpr int dense_ncb(int K) {
-  return sizeof(R) == 4 ? 7 : (K <= 3 ? 8 : (K == 6 ? 5 : 6));
+// Launch shape of k_dense_mma for K gate bits: column groups of 8 a warp works on at a time, threads a
+// block, blocks an SM. More groups keep more bytes in flight and use each matrix fragment more often,
+// as far as registers allow (27-qubit complex128 states, gate bits 10..17: K = 4 0.99 / 0.78 / 0.71 ms
+// with 1 / 2 / 4 groups, K = 3 0.81 / 0.74 ms with 2 / 4, K = 5 1.27 / 1.24 ms with 1 / 2).
+struct DenseMmaShape {
+  int groups, threads, blocks;
+};
+constexpr DenseMmaShape dense_mma_shape(int K) {
+  return K == 2 ? DenseMmaShape{8, 128, 3}
+         : K == 3 ? DenseMmaShape{4, 128, 4}
+         : K == 4 ? DenseMmaShape{4, 128, 3}
+         : K == 5 ? DenseMmaShape{2, 128, 3}
+                  : DenseMmaShape{1, 512, 1};
 }
 
-// Double-buffered gathers where the sweep is memory-bound (k <= 4); the compute-bound k = 5, 6
-// CUDA-core tiles keep one buffer and twice the blocks per SM.
-template <class R> constexpr bool dense_db(int K) { return K <= 4; }
-
-template <class R, int K>
-size_t dense_smem_bytes() {
-  constexpr int M = 1 << K, NC = 1 << dense_ncb<R>(K), NB = dense_db<R>(K) ? 2 : 1;
-  return size_t(2) * NB * M * NC * sizeof(R) + size_t(2) * M * M * sizeof(R) + (NC + M) * 4 + M * 8;
+template <class R, int K, int G, int TH, int MINB>
+void launch_dense_mma_shape(const LaunchEnv& env, R* re, R* im, uint64_t ngroups, const R* u, const DenseMmaP& p) {
+  constexpr size_t smem = size_t(32) << (2 * K);
+  auto kern = k_dense_mma<R, K, G, TH, MINB>;
+  QSVB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  const uint64_t items = ngroups / G;
+  kern<<<grid_for(items, TH / 32, env.num_sms, MINB), TH, smem, env.stream>>>(re, im, items, u, p);
+  check_launch();
 }
 
 template <class R, int K>
-void launch_dense_k(const LaunchEnv& env, R* re, R* im, uint32_t n, const Sweep& s, const R* ut) {
-  constexpr int NCB = dense_ncb<R>(K);
-  constexpr int M = 1 << K, NC = 1 << NCB, LOG = VecT<R>::LOG;
-  if (n < uint32_t(K + NCB)) {
-    std::vector<uint32_t> fixed(s.q, s.q + K);
+void launch_dense_mma(const LaunchEnv& env, R* re, R* im, uint32_t n, const uint32_t* q, const R* u) {
+  DenseMmaP p{};
+  std::copy(q, q + K, p.q);
+  constexpr DenseMmaShape sh = dense_mma_shape(K);
+  const uint64_t ngroups = 1ull << (n - K - 3);
+  // several groups a warp only once every resident warp has an item of its own; below that, one group
+  // a warp in small blocks spreads the state over more SMs
+  if (ngroups / sh.groups >= uint64_t(env.num_sms) * sh.blocks * (sh.threads / 32))
+    launch_dense_mma_shape<R, K, sh.groups, sh.threads, sh.blocks>(env, re, im, ngroups, u, p);
+  else if constexpr (K < 6)
+    launch_dense_mma_shape<R, K, 1, 64, 4>(env, re, im, ngroups, u, p);
+  else
+    launch_dense_mma_shape<R, K, 1, 128, 1>(env, re, im, ngroups, u, p);
+}
+
+// k_dense_cols holds 2^K x 4 amplitudes a thread: one block of as many warps as the registers allow
+// (K = 4 with all gate bits above bit 1: 12 warps 0.38 ms, 8 warps 0.41 ms; with shuffles or more rows a
+// step 8 warps win, 0.44-0.47 against 0.44-0.51 ms).
+constexpr int dense_cols_threads(int K, int nlow, int l2) {
+  return K == 4 ? (nlow == 0 && l2 == 0 ? 384 : 256) : 512;
+}
+
+template <int K, int L0, int L1, int L2>
+void launch_dense_cols_at(const LaunchEnv& env, float* re, float* im, uint32_t n, const float* u, const DenseColP& p) {
+  constexpr int TH = dense_cols_threads(K, L0 + L1, L2);
+  const uint64_t items = 1ull << (n - K - 7);
+  k_dense_cols<K, L0, L1, L2, TH><<<grid_for(items, TH / 32, env.num_sms, 1), TH, 0, env.stream>>>(
+      re, im, items, reinterpret_cast<const float2*>(u), p);
+  check_launch();
+}
+
+template <int K>
+void launch_dense_cols(const LaunchEnv& env, float* re, float* im, uint32_t n, const uint32_t* q, const float* u) {
+  auto has = [&](uint32_t b) { return std::find(q, q + K, b) != q + K; };
+  const bool l0 = has(0), l1 = has(1), l2 = has(2);
+  const uint32_t nlow = uint32_t(l0) + uint32_t(l1);
+  DenseColP p{};
+  std::vector<uint32_t> ins(q, q + K);
+  for (uint32_t b = 0; b < 2; ++b)
+    if (!has(b)) ins.push_back(b);
+  std::sort(ins.begin(), ins.end());
+  p.nins = uint32_t(ins.size());
+  std::copy(ins.begin(), ins.end(), p.ins);
+  for (uint32_t j = nlow; j < uint32_t(K); ++j) p.hi[j - nlow] = 1ull << q[j];
+  for (uint32_t j = 0; j < nlow; ++j) {  // the extra columns lie above the 5 lane bits
+    uint64_t x = 1ull << (5 + j);
+    for (uint32_t b : ins) {
+      const uint64_t lo = x & ((1ull << b) - 1ull);
+      x = ((x - lo) << 1) | lo;
+    }
+    p.ext[j] = x;
+  }
+  if (l0 && l1) launch_dense_cols_at<K, 1, 1, 0>(env, re, im, n, u, p);  // a thread has whole sectors
+  else if (l0 && l2) launch_dense_cols_at<K, 1, 0, 1>(env, re, im, n, u, p);
+  else if (l0) launch_dense_cols_at<K, 1, 0, 0>(env, re, im, n, u, p);
+  else if (l1 && l2) launch_dense_cols_at<K, 0, 1, 1>(env, re, im, n, u, p);
+  else if (l1) launch_dense_cols_at<K, 0, 1, 0>(env, re, im, n, u, p);
+  else if (l2) launch_dense_cols_at<K, 0, 0, 1>(env, re, im, n, u, p);
+  else launch_dense_cols_at<K, 0, 0, 0>(env, re, im, n, u, p);
+}
+
+// Which kernel runs a dense sweep:
+//  * fewer than 8 columns: one block of amplitudes per thread;
+//  * complex64 with K <= 4 once every resident warp has 2^K x 128 amplitudes of its own (n >= 21 or 22):
+//    paired FP32 FMAs;
+//  * everything else: the FP64 matrix instruction. That is complex128, complex64 states below that
+//    size (a warp there needs only 2^K x 8 amplitudes, so more SMs take part) and complex64 K = 5, 6 on
+//    CUDA cores (27 qubits: 1.20 ms against 1.20 (K = 5) and 2.02 against 2.09 ms (K = 6) for an FP32
+//    shared-memory tile, with one rounding instead of 2^(K+1)).
+template <class R, int K>
+void launch_dense_of(const LaunchEnv& env, R* re, R* im, uint32_t n, const Sweep& s, const R* u) {
+  uint32_t q[K];
+  std::copy(s.q, s.q + K, q);
+  std::sort(q, q + K);
+  if (n < uint32_t(K + 3)) {
     const uint64_t nb = 1ull << (n - K);
-    uint32_t q[6] = {0, 0, 0, 0, 0, 0};
-    for (int j = 0; j < K; ++j) q[j] = s.q[j];
+    uint32_t v[6] = {0, 0, 0, 0, 0, 0};
+    std::copy(q, q + K, v);
     k_dense_small<R, K><<<grid_for(nb, 128, env.num_sms), 128, 0, env.stream>>>(
-        re, im, nb, ut, make_enum(fixed, 0), q[0], q[1], q[2], q[3], q[4], q[5]);
+        re, im, nb, u, make_enum(std::vector<uint32_t>(q, q + K), 0), v[0], v[1], v[2], v[3], v[4], v[5]);
     check_launch();
     return;
   }
-  // tile bits: gate bits + the NCB lowest non-gate bits
-  int gate_rank[64];
-  for (int b = 0; b < 64; ++b) gate_rank[b] = -1;
-  for (int j = 0; j < K; ++j) gate_rank[s.q[j]] = j;
-  int col_rank[64];
-  std::vector<uint32_t> tbits;
-  int ncol = 0;
-  for (uint32_t b = 0; b < n; ++b) {
-    col_rank[b] = -1;
-    if (gate_rank[b] >= 0) tbits.push_back(b);
-    else if (ncol < NCB) {
-      col_rank[b] = ncol++;
-      tbits.push_back(b);
+  if constexpr (sizeof(R) == 4 && K <= 4) {
+    if (n >= uint32_t(K + 7) &&
+        (1ull << (n - K - 7)) >= uint64_t(env.num_sms) * (dense_cols_threads(K, 0, 0) / 32)) {
+      launch_dense_cols<K>(env, re, im, n, q, u);
+      return;
     }
   }
-  auto contrib = [&](uint32_t b) -> uint32_t {
-    return gate_rank[b] >= 0 ? (uint32_t(1) << gate_rank[b]) * NC : (uint32_t(1) << col_rank[b]);
-  };
-  DenseP p{};
-  for (int j = 0; j < NCB; ++j) QSVB_REQUIRE(tbits[j] == uint32_t(j), "dense tile: low bits not contiguous");
-  for (int j = 0; j < K; ++j) p.hibits[j] = tbits[NCB + j];
-  for (int h = 0; h < M; ++h) {
-    uint64_t off = 0;
-    uint32_t d = 0;
-    for (int j = 0; j < K; ++j)
-      if ((h >> j) & 1) {
-        off |= 1ull << p.hibits[j];
-        d += contrib(p.hibits[j]);
-      }
-    p.hioff[h] = off;
-    p.dsthi[h] = d;
-  }
-  for (int l = 0; l < NC; ++l) {
-    uint32_t d = 0;
-    for (int b = 0; b < NCB; ++b)
-      if ((l >> b) & 1) d += contrib(uint32_t(b));
-    p.dstlo[l] = d;
-  }
-  p.vecstore = 1;
-  for (int b = 0; b < LOG; ++b)
-    if (gate_rank[b] >= 0) p.vecstore = 0;
-  const uint64_t ntiles = 1ull << (n - K - NCB);
-  const size_t smem = dense_smem_bytes<R, K>();
-  constexpr bool DB = dense_db<R>(K);
-  QSVB_CK(cudaFuncSetAttribute(k_dense<R, K, NCB, DB>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-  QSVB_CK(cudaFuncSetAttribute(k_dense<R, K, NCB, DB>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                               int(cudaSharedmemCarveoutMaxShared)));
-  int occ = 1;
-  QSVB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_dense<R, K, NCB, DB>, kThreads, smem));
-  const unsigned grid = unsigned(std::max<uint64_t>(1, std::min<uint64_t>(ntiles, uint64_t(env.num_sms) * std::max(occ, 1))));
-  k_dense<R, K, NCB, DB><<<grid, kThreads, smem, env.stream>>>(re, im, ntiles, ut, p);
-  check_launch();
+  launch_dense_mma<R, K>(env, re, im, n, q, u);
 }
 
 template <class R>
 void launch_dense(const LaunchEnv& env, R* re, R* im, uint32_t n, const Sweep& s, const void* dev_mat) {
   const R* ut = static_cast<const R*>(dev_mat);
   switch (s.m) {
-    case 2: launch_dense_k<R, 2>(env, re, im, n, s, ut); break;
-    case 3: launch_dense_k<R, 3>(env, re, im, n, s, ut); break;
-    case 4: launch_dense_k<R, 4>(env, re, im, n, s, ut); break;
-    case 5: launch_dense_k<R, 5>(env, re, im, n, s, ut); break;
-    case 6: launch_dense_k<R, 6>(env, re, im, n, s, ut); break;
+    case 2: launch_dense_of<R, 2>(env, re, im, n, s, ut); break;
+    case 3: launch_dense_of<R, 3>(env, re, im, n, s, ut); break;
+    case 4: launch_dense_of<R, 4>(env, re, im, n, s, ut); break;
+    case 5: launch_dense_of<R, 5>(env, re, im, n, s, ut); break;
+    case 6: launch_dense_of<R, 6>(env, re, im, n, s, ut); break;
     default: throw Error(QSVB_E_INVALID, "dense sweep arity must be 2..6");
   }
 }
@@ -1059,11 +1211,19 @@ size_t sweep_matrix_bytes(const Sweep& s, int dtype) {
 
 void pack_sweep_matrix(const Sweep& s, int dtype, void* dst) {
   if (s.kind == SK_DENSE) {
-    const size_t M = size_t(1) << s.m;
-    for (size_t r = 0; r < M; ++r)
-      for (size_t c = 0; c < M; ++c) {
-        const cd v = s.mat[r * M + c];
-        const size_t o = 2 * (c * M + r);  // transposed: [s][r]
+    const uint32_t M = 1u << s.m;
+    uint32_t rank[6] = {};  // the kernels take the gate's bits in the order of their state bits
+    for (uint32_t j = 0; j < s.m; ++j)
+      for (uint32_t i = 0; i < s.m; ++i) rank[j] += s.q[i] < s.q[j];
+    auto sorted = [&](uint32_t x) {
+      uint32_t o = 0;
+      for (uint32_t j = 0; j < s.m; ++j) o |= ((x >> j) & 1u) << rank[j];
+      return o;
+    };
+    for (uint32_t r = 0; r < M; ++r)
+      for (uint32_t c = 0; c < M; ++c) {
+        const cd v = s.mat[size_t(r) * M + c];
+        const size_t o = 2 * (size_t(sorted(r)) * M + sorted(c));
         if (dtype == QSVB_C128) {
           static_cast<double*>(dst)[o] = v.real();
           static_cast<double*>(dst)[o + 1] = v.imag();

@@ -1,0 +1,60 @@
+"""Dense CUDA-core sweeps at every size class of their launch rule: states with fewer columns than one
+matrix-instruction tile, one column group a warp, several groups a warp, and gate bits low, high,
+spread and in descending order.
+
+Tolerance: each output is a sum of 2^(k+1) products whose absolute values add up to at most
+|row| |x| <= 1 (unitary row, normalised state), so with unit roundoff u the sum is off by at most
+2^(k+1) u, plus u for the rounding of the matrix and of the input each and one for the store."""
+import numpy as np
+import pytest
+
+from rustatevec_b200 import Plan, PLAN_AS_GIVEN, ENGINE_CUDA_CORE
+from rustatevec_b200 import _lib as L
+from rustatevec_b200 import gate as G
+from rustatevec_b200.circuit import Circuit
+
+from helpers import max_abs_diff, numpy_run
+
+pytestmark = pytest.mark.gpu
+UNIT = {"f64": 2.0 ** -53, "f32": 2.0 ** -24}
+
+
+def unitary(k, rng):
+    z = rng.normal(size=(1 << k, 1 << k)) + 1j * rng.normal(size=(1 << k, 1 << k))
+    return np.linalg.qr(z)[0]
+
+
+def placements(n, k, rng):
+    spread = sorted(rng.choice(n, size=k, replace=False).tolist())
+    out = [list(range(k)), list(range(n - k, n)), spread, spread[::-1]]
+    if n >= k + 3:  # the bits around a 16-byte vector, a 32-byte sector and a warp's row
+        out += [[0] + list(range(n - k + 1, n)), [1] + list(range(n - k + 1, n)), [2] + list(range(n - k + 1, n)),
+                list(range(1, k + 1)), list(range(2, k + 2)), [0, 2] + list(range(n - k + 2, n)),
+                [1, 2] + list(range(n - k + 2, n)), [0, 1] + list(range(n - k + 2, n))]
+    return out
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+@pytest.mark.parametrize("k", [2, 3, 4, 5, 6])
+@pytest.mark.parametrize("n", [6, 8, 9, 10, 11, 13, 17, 21])
+def test_dense_sweep_every_size_class(be64, be32, precision, k, n):
+    be = be64 if precision == "f64" else be32
+    rng = np.random.default_rng(100 * k + n)
+    qsets = placements(n, k, rng)
+    if n >= 17:  # the large states: one launch class, every placement once across the sizes
+        qsets = qsets[:3] + [qsets[3 + n % (len(qsets) - 3)]]
+    st = be.alloc(n)
+    for qs in qsets:
+        if len(set(qs)) < k:
+            continue
+        psi = rng.normal(size=1 << n) + 1j * rng.normal(size=1 << n)
+        psi = (psi / np.linalg.norm(psi)).astype(np.complex128 if precision == "f64" else np.complex64)
+        c = Circuit(n)
+        c.push(G.DenseGate(k, unitary(k, rng)), qs)
+        plan = Plan(be, c, L.make_opts(PLAN_AS_GIVEN, k, ENGINE_CUDA_CORE))
+        assert plan.stats()["by_kind"] == {"dense": 1}
+        be.upload(st, psi.real, psi.imag)
+        plan.run(st)
+        err = max_abs_diff(numpy_run(c, psi), be.download(st).as_complex())
+        assert err <= (2 ** (k + 1) + 4) * UNIT[precision], (qs, err)
+    st.free()
