@@ -96,7 +96,8 @@ typedef struct qsvb_plan_opts {
 /* What a plan does, for reports and rooflines. */
 typedef struct qsvb_plan_stats {
   uint64_t n_gates_in;        /* gates in the input circuit */
-  uint64_t n_sweeps;          /* kernel sweeps launched per run */
+  uint64_t n_sweeps;          /* sweeps of the plan; a run launches one kernel for each, except for diagonal
+                                 sweeps that a dense sweep's kernel carries along */
   uint64_t n_sweeps_by_kind[10]; /* 1q, ctrl1q, diag, phase, dense CUDA-core, dense TC, tile pass,
                                    other, tensor-core chain pass, tile permutation */
   double algorithmic_bytes;   /* sum over sweeps of 2 * (amplitudes the sweep may change) * bytes/amp */

@@ -105,10 +105,10 @@ void* ring_upload(qsvb_ctx* c, const void* src, size_t bytes) {
   return dst;
 }
 
-void run_sweep(qsvb_ctx* c, qsvb_state* st, const Sweep& s, const void* dev_mat) {
+void run_sweep(qsvb_ctx* c, qsvb_state* st, const Sweep& s, const void* dev_mat, bool tail = false) {
   by_dtype(st->dtype, [&](auto r) {
     using R = decltype(r);
-    launch_sweep<R>(c->env(), static_cast<R*>(st->re), static_cast<R*>(st->im), st->n_qubits, s, dev_mat);
+    launch_sweep<R>(c->env(), static_cast<R*>(st->re), static_cast<R*>(st->im), st->n_qubits, s, dev_mat, tail);
   });
 }
 
@@ -127,6 +127,8 @@ qsvb_plan* build_plan(qsvb_ctx* c, const qsvb_circuit* circ, int dtype, const qs
   p->sweeps = plan_sweeps(gates_from_circuit(circ), circ->n_qubits, p->opts, dtype);
   p->stats.n_gates_in = circ->n_gates;
   sweep_costs(p->sweeps, circ->n_qubits, dtype, &p->stats);
+  // (as given: one sweep per gate, in order)
+  if (p->opts.planner != QSVB_PLAN_AS_GIVEN) attach_diagonals(p->sweeps, circ->n_qubits);
   // one device block holding every sweep's matrix, uploaded once
   size_t total = 0;
   for (const Sweep& s : p->sweeps) {
@@ -176,8 +178,9 @@ qsvb_plan* build_plan(qsvb_ctx* c, const qsvb_circuit* circ, int dtype, const qs
 
 void launch_plan(qsvb_ctx* c, qsvb_plan* p, qsvb_state* st) {
   for (size_t i = 0; i < p->sweeps.size(); ++i) {
+    if (p->sweeps[i].carried) continue;
     const void* m = sweep_matrix_bytes(p->sweeps[i], p->dtype) ? p->d_mats + p->mat_offset[i] : nullptr;
-    run_sweep(c, st, p->sweeps[i], m);
+    run_sweep(c, st, p->sweeps[i], m, true);
   }
 }
 

@@ -14,6 +14,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 #include "qsvb_internal.h"
 
@@ -26,10 +27,12 @@ constexpr int kThreads = 256;
 template <class R> struct VecT;
 template <> struct VecT<float> {
   using T = float4;
+  using Pair = float2;
   static constexpr int N = 4, LOG = 2;
 };
 template <> struct VecT<double> {
   using T = double2;
+  using Pair = double2;
   static constexpr int N = 2, LOG = 1;
 };
 
@@ -401,9 +404,10 @@ __global__ void __launch_bounds__(kThreads) k_ising(R* __restrict__ re, R* __res
 
 // ---------------------------------------------------------------------------------------------
 // Dense k-qubit sweep (qsv kernels.cu:91-120 gathers one 2^m block per thread into local arrays).
-// Matrices are packed row-major, interleaved (re, im) in the state's precision, with the gate's bits
-// in ascending order of their state bits (pack_sweep_matrix). Two kernels; launch_dense_of states
-// which one runs where.
+// Matrices are packed row-major, interleaved (re, im) in the state's precision; the classifier lists a
+// dense gate's qubits in ascending order. Two kernels; launch_dense_of states which one runs where.
+// Either can multiply its result by a diagonal sweep's factors before the write-back (`Tail`, chosen
+// by attach_diagonals), which saves that sweep's own read and write of the state.
 // ---------------------------------------------------------------------------------------------
 
 // Dense sweep on the FP64 matrix instruction (mma.m8n8k4), no shared-memory staging of the state. A
@@ -423,19 +427,57 @@ __global__ void __launch_bounds__(kThreads) k_ising(R* __restrict__ re, R* __res
 // complex128 states (4.3 GB moved), mean over low, middle and high gate bits, before -> after:
 //   K = 2: 0.87 -> 0.68 ms, K = 3: 0.94 -> 0.70 ms, K = 4: 1.39 -> 0.75 ms (5.7 TB/s),
 //   K = 5: 2.26 -> 1.20 ms (28.5 TFLOP/s), K = 6: 3.85 -> 2.02 ms (34 TFLOP/s).
+//
+// Tail: the diagonal D applied after the dense product, in the order and the rounding of a separate
+// diagonal sweep (the product rounded to R, then one complex multiply in R), so results are the same
+// bit for bit. Bits of the sub-index that must be 1 for D to act (`need`) are honoured per amplitude.
+// Cost at 27 qubits: K = 2, 3 within 0.03 ms of the plain sweep; K = 4 complex64 0.37 -> 0.49 ms and
+// complex128 0.72 -> 0.91 ms, against 0.36 and 0.73 ms for the diagonal sweep that it replaces.
+template <class R> struct Tail {
+  uint32_t q[6];  // state bit of each sub-index bit (63: unused)
+  uint32_t need;
+  uint32_t m;
+  // sub-index bits that an offset brings in, so that a thread extracts them from its address once:
+  // the gate's bits (in the kernel's order), and the group bits (k_dense_mma) or extra columns and
+  // vector elements (k_dense_cols)
+  uint32_t gate[6], grp[3], ext[2], elem[2];
+  R d[128];  // interleaved (re, im), 2^m entries
+};
+
+template <class R> __device__ __forceinline__ uint32_t tail_index(const Tail<R>& t, uint64_t a) {
+  uint32_t s = 0;
+#pragma unroll
+  for (int j = 0; j < 6; ++j) s |= uint32_t((a >> t.q[j]) & 1ull) << j;
+  return s;
+}
+
+template <class R, class R2>
+__device__ __forceinline__ void tail_apply(const R2* tab, uint32_t need, uint32_t sub, R& xr, R& xi) {
+  const R2 d = tab[sub];
+  const R a = xr, c = xi;
+  const bool acts = (sub & need) == need;  // (selected, not branched on)
+  xr = acts ? fma(d.x, a, -d.y * c) : a;
+  xi = acts ? fma(d.x, c, d.y * a) : c;
+}
+
 __device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
                : "+d"(c[0]), "+d"(c[1])
                : "d"(a), "d"(b));
 }
 
+struct NoTail {};
+template <class R, bool TAIL> using TailIf = std::conditional_t<TAIL, Tail<R>, NoTail>;
+
 struct DenseMmaP {
-  uint32_t q[6];  // gate bits, ascending
+  uint64_t bit[6];  // address of the gate bits, ascending
+  uint64_t grp[3];  // address of the column bits that number a warp's groups
 };
 
-template <class R, int K, int G, int TH, int MINB>
+template <class R, int K, int G, int TH, int MINB, bool TAIL>
 __global__ void __launch_bounds__(TH, MINB) k_dense_mma(R* __restrict__ re, R* __restrict__ im, uint64_t nitems,
-                                                        const R* __restrict__ u, DenseMmaP p) {
+                                                        const R* __restrict__ u, DenseMmaP p,
+                                                        const __grid_constant__ TailIf<R, TAIL> t) {
   constexpr int M = 1 << K, H = M / 4;  // H: values of the gate bits above the two lowest
   extern __shared__ __align__(16) char smem_raw[];
   // fragment (r >> 2, s >> 2): lane 8 (r & 3) + 4 part + (s & 3) holds the two values that multiply the
@@ -446,39 +488,47 @@ __global__ void __launch_bounds__(TH, MINB) k_dense_mma(R* __restrict__ re, R* _
     const double ar = u[2 * (r * M + s)], ai = u[2 * (r * M + s) + 1];
     ws[i] = (i & 4) ? make_double2(ai, ar) : make_double2(ar, -ai);
   }
+  __shared__ __align__(16) typename VecT<R>::Pair tab[TAIL ? 64 : 1];
+  if constexpr (TAIL)
+    for (int i = threadIdx.x; i < (1 << t.m); i += TH) tab[i] = {t.d[2 * i], t.d[2 * i + 1]};
   __syncthreads();
   const uint32_t lane = threadIdx.x & 31u;
-  uint64_t bit[K];
-#pragma unroll
-  for (int j = 0; j < K; ++j) bit[j] = 1ull << p.q[j];
-  const uint64_t low = ((lane & 1u) ? bit[0] : 0ull) + ((lane & 2u) ? bit[1] : 0ull);
+  const uint64_t low = ((lane & 1u) ? p.bit[0] : 0ull) + ((lane & 2u) ? p.bit[1] : 0ull);
   auto row = [&](int h) {  // address offset of the higher gate bits' value h
     uint64_t o = 0;
 #pragma unroll
     for (int j = 2; j < K; ++j)
-      if ((h >> (j - 2)) & 1) o += bit[j];
+      if ((h >> (j - 2)) & 1) o += p.bit[j];
+    return o;
+  };
+  auto group = [&](int g) {
+    uint64_t o = 0;
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      if ((g >> j) & 1) o += p.grp[j];
     return o;
   };
   const uint64_t nwarps = uint64_t(gridDim.x) * (TH / 32);
 #pragma unroll 1
   for (uint64_t w = blockIdx.x * uint64_t(TH / 32) + (threadIdx.x >> 5); w < nitems; w += nwarps) {
-    uint64_t base[G];
+    uint64_t base = w * (G * 8) + (lane >> 2);
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const uint64_t lo = base & (p.bit[j] - 1ull);
+      base = ((base - lo) << 1) | lo;
+    }
+    // (the group bits lie between the columns' and w's, so they are zero in it)
+    base += low;
+    uint32_t tsub = 0;  // tail sub-index of this lane's row 0 in group 0
+    if constexpr (TAIL) tsub = tail_index(t, base);
     R x[G][2 * H];
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-      uint64_t a = (w * G + g) * 8 + (lane >> 2);
-#pragma unroll
-      for (int j = 0; j < K; ++j) {
-        const uint64_t lo = a & (bit[j] - 1ull);
-        a = ((a - lo) << 1) | lo;
-      }
-      base[g] = a + low;
+    for (int g = 0; g < G; ++g)
 #pragma unroll
       for (int h = 0; h < H; ++h) {
-        x[g][2 * h] = re[base[g] + row(h)];
-        x[g][2 * h + 1] = im[base[g] + row(h)];
+        x[g][2 * h] = re[base + group(g) + row(h)];
+        x[g][2 * h + 1] = im[base + group(g) + row(h)];
       }
-    }
 #pragma unroll
     for (int r = 0; r < H; ++r) {
       double y[G][2];
@@ -496,8 +546,19 @@ __global__ void __launch_bounds__(TH, MINB) k_dense_mma(R* __restrict__ re, R* _
       // in place: a lane stores only addresses that it has loaded itself
 #pragma unroll
       for (int g = 0; g < G; ++g) {
-        re[base[g] + row(r)] = R(y[g][0]);
-        im[base[g] + row(r)] = R(y[g][1]);
+        R yr = R(y[g][0]), yi = R(y[g][1]);
+        if constexpr (TAIL) {
+          uint32_t sub = tsub;
+#pragma unroll
+          for (int j = 2; j < K; ++j)
+            if ((r >> (j - 2)) & 1) sub |= t.gate[j];
+#pragma unroll
+          for (int j = 0; j < 3; ++j)
+            if ((g >> j) & 1) sub |= t.grp[j];
+          tail_apply(tab, t.need, sub, yr, yi);
+        }
+        re[base + group(g) + row(r)] = yr;
+        im[base + group(g) + row(r)] = yi;
       }
     }
   }
@@ -513,8 +574,8 @@ __global__ void __launch_bounds__(TH, MINB) k_dense_mma(R* __restrict__ re, R* _
 //   Before, each product of the shared-memory tile needed one operand from shared memory for every
 // two FMAs and three block barriers a tile. Bound now: HBM (K = 2, 3); FP32 FMA issue together with
 // HBM (K = 4: 240 of 380 us are FMA issue). Measured on 27-qubit states (2.1 GB moved), mean over low,
-// middle and high gate bits, before -> after: K = 2: 0.50 -> 0.36 ms, K = 3: 0.59 -> 0.38 ms,
-// K = 4: 0.77 -> 0.45 ms (0.58 -> 0.38 ms with the gate bits above bit 6).
+// middle and high gate bits, before -> after: K = 2: 0.50 -> 0.35 ms, K = 3: 0.59 -> 0.37 ms,
+// K = 4: 0.77 -> 0.43 ms (0.58 -> 0.39 ms with the gate bits above bit 6).
 struct DenseColP {
   uint32_t ins[6], nins;  // the register bits (gate bits and state bits 0, 1), ascending
   uint32_t zero;          // 0: see `fresh`
@@ -537,14 +598,18 @@ __device__ __forceinline__ void fma2(f32x2& d, f32x2 a, f32x2 b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
 }
 
-template <int K, int L0, int L1, int L2, int TH>
+template <int K, int L0, int L1, int L2, int TH, bool TAIL>
 __global__ void __launch_bounds__(TH, 1) k_dense_cols(float* __restrict__ re, float* __restrict__ im, uint64_t nitems,
-                                                      const float2* __restrict__ u, const __grid_constant__ DenseColP p) {
+                                                      const float2* __restrict__ u, const __grid_constant__ DenseColP p,
+                                                      const __grid_constant__ TailIf<float, TAIL> t) {
   constexpr int M = 1 << K, NL = L0 + L1, NH = K - NL, VH = 1 << NH, NX = 1 << NL, RV = 1 << NL;
   constexpr int VB = (L2 || (K == 4 && NL == 0)) ? 2 : 1;  // vectors (groups of RV rows) a step
   constexpr int RB = RV * VB;
   __shared__ __align__(16) float2 us[M * M];
   for (int i = threadIdx.x; i < M * M; i += TH) us[i] = u[i];
+  __shared__ __align__(16) float2 tab[TAIL ? 64 : 1];
+  if constexpr (TAIL)
+    for (int i = threadIdx.x; i < (1 << t.m); i += TH) tab[i] = make_float2(t.d[2 * i], t.d[2 * i + 1]);
   __syncthreads();
   const uint32_t lane = threadIdx.x & 31u;
   auto insert = [&](uint64_t x) {
@@ -579,6 +644,8 @@ __global__ void __launch_bounds__(TH, 1) k_dense_cols(float* __restrict__ re, fl
   for (uint64_t w = blockIdx.x * uint64_t(TH / 32) + (threadIdx.x >> 5); w < nitems; w += nwarps) {
     const uint64_t base = insert(w << (5 + NL)) + lane_off;
     asm volatile("" ::: "memory");  // the matrix stays in shared memory (hoisted, it would spill)
+    uint32_t tsub = 0;  // tail sub-index of the thread's first amplitude
+    if constexpr (TAIL) tsub = tail_index(t, base);
     float xr[M][4], xi[M][4];
 #pragma unroll
     for (int v = 0; v < VH; ++v)
@@ -662,6 +729,12 @@ __global__ void __launch_bounds__(TH, 1) k_dense_cols(float* __restrict__ re, fl
 #pragma unroll
       for (int j = 1; j < NH; ++j)
         if ((v0 >> j) & 1) group += p.hi[j];
+      uint32_t gsub = tsub;
+      if constexpr (TAIL) {
+#pragma unroll
+        for (int j = 0; j < NH; ++j)
+          if ((v0 >> j) & 1) gsub |= t.gate[j];
+      }
       // in place: a thread stores only the vectors that it has loaded itself
 #pragma unroll
       for (int v = 0; v < VB; ++v)
@@ -673,6 +746,9 @@ __global__ void __launch_bounds__(TH, 1) k_dense_cols(float* __restrict__ re, fl
           for (int e = 0; e < 4; ++e) {
             fr[e] = yr[v * RV + elem_row(e)][elem_col(e, x)];
             fi[e] = yi[v * RV + elem_row(e)][elem_col(e, x)];
+            if constexpr (TAIL)
+              tail_apply(tab, t.need, gsub | (v ? t.gate[0] : 0u) | ((x & 1) ? t.ext[0] : 0u) |
+                         ((x & 2) ? t.ext[1] : 0u) | ((e & 1) ? t.elem[0] : 0u) | ((e & 2) ? t.elem[1] : 0u), fr[e], fi[e]);
           }
           vst(re + a, fr);
           vst(im + a, fi);
@@ -1024,30 +1100,52 @@ constexpr DenseMmaShape dense_mma_shape(int K) {
                   : DenseMmaShape{1, 512, 1};
 }
 
-template <class R, int K, int G, int TH, int MINB>
-void launch_dense_mma_shape(const LaunchEnv& env, R* re, R* im, uint64_t ngroups, const R* u, const DenseMmaP& p) {
+template <class R, int K, int G, int TH, int MINB, bool TAIL>
+void launch_dense_mma_shape(const LaunchEnv& env, R* re, R* im, uint64_t ngroups, const R* u, const DenseMmaP& p,
+                            const TailIf<R, TAIL>& t) {
   constexpr size_t smem = size_t(32) << (2 * K);
-  auto kern = k_dense_mma<R, K, G, TH, MINB>;
+  auto kern = k_dense_mma<R, K, G, TH, MINB, TAIL>;
   QSVB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   const uint64_t items = ngroups / G;
-  kern<<<grid_for(items, TH / 32, env.num_sms, MINB), TH, smem, env.stream>>>(re, im, items, u, p);
+  kern<<<grid_for(items, TH / 32, env.num_sms, MINB), TH, smem, env.stream>>>(re, im, items, u, p, t);
   check_launch();
 }
 
-template <class R, int K>
-void launch_dense_mma(const LaunchEnv& env, R* re, R* im, uint32_t n, const uint32_t* q, const R* u) {
+// The value with zero bits inserted at the ascending positions q (layout.rs:70-86).
+inline uint64_t insert_bits(uint64_t x, const uint32_t* q, size_t count) {
+  for (size_t j = 0; j < count; ++j) {
+    const uint64_t lo = x & ((1ull << q[j]) - 1ull);
+    x = ((x - lo) << 1) | lo;
+  }
+  return x;
+}
+
+template <class R> uint32_t tail_bits(const Tail<R>& t, uint64_t address) {
+  uint32_t s = 0;
+  for (uint32_t j = 0; j < t.m; ++j) s |= uint32_t((address >> t.q[j]) & 1u) << j;
+  return s;
+}
+
+template <class R, int K, bool TAIL>
+void launch_dense_mma(const LaunchEnv& env, R* re, R* im, uint32_t n, const uint32_t* q, const R* u,
+                      TailIf<R, TAIL> t) {
   DenseMmaP p{};
-  std::copy(q, q + K, p.q);
+  for (int j = 0; j < K; ++j) p.bit[j] = 1ull << q[j];
+  for (int j = 0; j < 3; ++j) p.grp[j] = insert_bits(8ull << j, q, K);
+  if constexpr (TAIL) {
+    for (int j = 0; j < K; ++j) t.gate[j] = tail_bits(t, p.bit[j]);
+    for (int j = 0; j < 3; ++j) t.grp[j] = tail_bits(t, p.grp[j]);
+  }
   constexpr DenseMmaShape sh = dense_mma_shape(K);
   const uint64_t ngroups = 1ull << (n - K - 3);
   // several groups a warp only once every resident warp has an item of its own; below that, one group
   // a warp in small blocks spreads the state over more SMs
   if (ngroups / sh.groups >= uint64_t(env.num_sms) * sh.blocks * (sh.threads / 32))
-    launch_dense_mma_shape<R, K, sh.groups, sh.threads, sh.blocks>(env, re, im, ngroups, u, p);
+    launch_dense_mma_shape<R, K, sh.groups, sh.threads, sh.blocks, TAIL>(env, re, im, ngroups, u, p, t);
   else if constexpr (K < 6)
-    launch_dense_mma_shape<R, K, 1, 64, 4>(env, re, im, ngroups, u, p);
+    launch_dense_mma_shape<R, K, 1, 64, 4, TAIL>(env, re, im, ngroups, u, p, t);
   else
-    launch_dense_mma_shape<R, K, 1, 128, 1>(env, re, im, ngroups, u, p);
+    launch_dense_mma_shape<R, K, 1, 128, 1, TAIL>(env, re, im, ngroups, u, p, t);
 }
 
 // k_dense_cols holds 2^K x 4 amplitudes a thread: one block of as many warps as the registers allow
@@ -1057,17 +1155,19 @@ constexpr int dense_cols_threads(int K, int nlow, int l2) {
   return K == 4 ? (nlow == 0 && l2 == 0 ? 384 : 256) : 512;
 }
 
-template <int K, int L0, int L1, int L2>
-void launch_dense_cols_at(const LaunchEnv& env, float* re, float* im, uint32_t n, const float* u, const DenseColP& p) {
+template <int K, int L0, int L1, int L2, bool TAIL>
+void launch_dense_cols_at(const LaunchEnv& env, float* re, float* im, uint32_t n, const float* u, const DenseColP& p,
+                          const TailIf<float, TAIL>& t) {
   constexpr int TH = dense_cols_threads(K, L0 + L1, L2);
   const uint64_t items = 1ull << (n - K - 7);
-  k_dense_cols<K, L0, L1, L2, TH><<<grid_for(items, TH / 32, env.num_sms, 1), TH, 0, env.stream>>>(
-      re, im, items, reinterpret_cast<const float2*>(u), p);
+  k_dense_cols<K, L0, L1, L2, TH, TAIL><<<grid_for(items, TH / 32, env.num_sms, 1), TH, 0, env.stream>>>(
+      re, im, items, reinterpret_cast<const float2*>(u), p, t);
   check_launch();
 }
 
-template <int K>
-void launch_dense_cols(const LaunchEnv& env, float* re, float* im, uint32_t n, const uint32_t* q, const float* u) {
+template <int K, bool TAIL>
+void launch_dense_cols(const LaunchEnv& env, float* re, float* im, uint32_t n, const uint32_t* q, const float* u,
+                       TailIf<float, TAIL> t) {
   auto has = [&](uint32_t b) { return std::find(q, q + K, b) != q + K; };
   const bool l0 = has(0), l1 = has(1), l2 = has(2);
   const uint32_t nlow = uint32_t(l0) + uint32_t(l1);
@@ -1079,21 +1179,21 @@ void launch_dense_cols(const LaunchEnv& env, float* re, float* im, uint32_t n, c
   p.nins = uint32_t(ins.size());
   std::copy(ins.begin(), ins.end(), p.ins);
   for (uint32_t j = nlow; j < uint32_t(K); ++j) p.hi[j - nlow] = 1ull << q[j];
-  for (uint32_t j = 0; j < nlow; ++j) {  // the extra columns lie above the 5 lane bits
-    uint64_t x = 1ull << (5 + j);
-    for (uint32_t b : ins) {
-      const uint64_t lo = x & ((1ull << b) - 1ull);
-      x = ((x - lo) << 1) | lo;
-    }
-    p.ext[j] = x;
+  // the extra columns lie above the 5 lane bits
+  for (uint32_t j = 0; j < nlow; ++j) p.ext[j] = insert_bits(1ull << (5 + j), p.ins, p.nins);
+  if constexpr (TAIL) {
+    for (uint32_t j = 0; j < 2; ++j) t.ext[j] = tail_bits(t, p.ext[j]), t.elem[j] = tail_bits(t, 1ull << j);
+    for (uint32_t j = 0; j < uint32_t(K) - nlow; ++j) t.gate[j] = tail_bits(t, p.hi[j]);
+    // bit 0 of the kernel's row groups: see `first`
+    if (l2 && nlow < 2) t.gate[0] = tail_bits(t, insert_bits(1, p.ins, p.nins));
   }
-  if (l0 && l1) launch_dense_cols_at<K, 1, 1, 0>(env, re, im, n, u, p);  // a thread has whole sectors
-  else if (l0 && l2) launch_dense_cols_at<K, 1, 0, 1>(env, re, im, n, u, p);
-  else if (l0) launch_dense_cols_at<K, 1, 0, 0>(env, re, im, n, u, p);
-  else if (l1 && l2) launch_dense_cols_at<K, 0, 1, 1>(env, re, im, n, u, p);
-  else if (l1) launch_dense_cols_at<K, 0, 1, 0>(env, re, im, n, u, p);
-  else if (l2) launch_dense_cols_at<K, 0, 0, 1>(env, re, im, n, u, p);
-  else launch_dense_cols_at<K, 0, 0, 0>(env, re, im, n, u, p);
+  if (l0 && l1) launch_dense_cols_at<K, 1, 1, 0, TAIL>(env, re, im, n, u, p, t);  // a thread has whole sectors
+  else if (l0 && l2) launch_dense_cols_at<K, 1, 0, 1, TAIL>(env, re, im, n, u, p, t);
+  else if (l0) launch_dense_cols_at<K, 1, 0, 0, TAIL>(env, re, im, n, u, p, t);
+  else if (l1 && l2) launch_dense_cols_at<K, 0, 1, 1, TAIL>(env, re, im, n, u, p, t);
+  else if (l1) launch_dense_cols_at<K, 0, 1, 0, TAIL>(env, re, im, n, u, p, t);
+  else if (l2) launch_dense_cols_at<K, 0, 0, 1, TAIL>(env, re, im, n, u, p, t);
+  else launch_dense_cols_at<K, 0, 0, 0, TAIL>(env, re, im, n, u, p, t);
 }
 
 // Which kernel runs a dense sweep:
@@ -1104,39 +1204,48 @@ void launch_dense_cols(const LaunchEnv& env, float* re, float* im, uint32_t n, c
 //    size (a warp there needs only 2^K x 8 amplitudes, so more SMs take part) and complex64 K = 5, 6 on
 //    CUDA cores (27 qubits: 1.20 ms against 1.20 (K = 5) and 2.02 against 2.09 ms (K = 6) for an FP32
 //    shared-memory tile, with one rounding instead of 2^(K+1)).
-template <class R, int K>
+template <class R, int K, bool TAIL>
 void launch_dense_of(const LaunchEnv& env, R* re, R* im, uint32_t n, const Sweep& s, const R* u) {
-  uint32_t q[K];
-  std::copy(s.q, s.q + K, q);
-  std::sort(q, q + K);
+  const uint32_t* q = s.q;  // ascending
   if (n < uint32_t(K + 3)) {
-    const uint64_t nb = 1ull << (n - K);
-    uint32_t v[6] = {0, 0, 0, 0, 0, 0};
-    std::copy(q, q + K, v);
-    k_dense_small<R, K><<<grid_for(nb, 128, env.num_sms), 128, 0, env.stream>>>(
-        re, im, nb, u, make_enum(std::vector<uint32_t>(q, q + K), 0), v[0], v[1], v[2], v[3], v[4], v[5]);
-    check_launch();
-    return;
+    if constexpr (!TAIL) {  // (attach_diagonals leaves such states alone)
+      const uint64_t nb = 1ull << (n - K);
+      k_dense_small<R, K><<<grid_for(nb, 128, env.num_sms), 128, 0, env.stream>>>(
+          re, im, nb, u, make_enum(std::vector<uint32_t>(q, q + K), 0), q[0], q[1], q[2], q[3], q[4], q[5]);
+      check_launch();
+      return;
+    }
+    throw Error(QSVB_E_INVALID, "dense sweep with a tail needs at least 8 columns");
+  }
+  TailIf<R, TAIL> t{};
+  if constexpr (TAIL) {
+    t.m = s.tail_m;
+    t.need = s.tail_need;
+    for (uint32_t j = 0; j < 6; ++j) t.q[j] = j < s.tail_m ? s.tail_q[j] : 63u;
+    for (size_t i = 0; i < s.tail.size(); ++i) {
+      t.d[2 * i] = R(s.tail[i].real());
+      t.d[2 * i + 1] = R(s.tail[i].imag());
+    }
   }
   if constexpr (sizeof(R) == 4 && K <= 4) {
     if (n >= uint32_t(K + 7) &&
         (1ull << (n - K - 7)) >= uint64_t(env.num_sms) * (dense_cols_threads(K, 0, 0) / 32)) {
-      launch_dense_cols<K>(env, re, im, n, q, u);
+      launch_dense_cols<K, TAIL>(env, re, im, n, q, u, t);
       return;
     }
   }
-  launch_dense_mma<R, K>(env, re, im, n, q, u);
+  launch_dense_mma<R, K, TAIL>(env, re, im, n, q, u, t);
 }
 
-template <class R>
+template <class R, bool TAIL>
 void launch_dense(const LaunchEnv& env, R* re, R* im, uint32_t n, const Sweep& s, const void* dev_mat) {
-  const R* ut = static_cast<const R*>(dev_mat);
+  const R* u = static_cast<const R*>(dev_mat);
   switch (s.m) {
-    case 2: launch_dense_of<R, 2>(env, re, im, n, s, ut); break;
-    case 3: launch_dense_of<R, 3>(env, re, im, n, s, ut); break;
-    case 4: launch_dense_of<R, 4>(env, re, im, n, s, ut); break;
-    case 5: launch_dense_of<R, 5>(env, re, im, n, s, ut); break;
-    case 6: launch_dense_of<R, 6>(env, re, im, n, s, ut); break;
+    case 2: launch_dense_of<R, 2, TAIL>(env, re, im, n, s, u); break;
+    case 3: launch_dense_of<R, 3, TAIL>(env, re, im, n, s, u); break;
+    case 4: launch_dense_of<R, 4, TAIL>(env, re, im, n, s, u); break;
+    case 5: launch_dense_of<R, 5, TAIL>(env, re, im, n, s, u); break;
+    case 6: launch_dense_of<R, 6, TAIL>(env, re, im, n, s, u); break;
     default: throw Error(QSVB_E_INVALID, "dense sweep arity must be 2..6");
   }
 }
@@ -1212,18 +1321,10 @@ size_t sweep_matrix_bytes(const Sweep& s, int dtype) {
 void pack_sweep_matrix(const Sweep& s, int dtype, void* dst) {
   if (s.kind == SK_DENSE) {
     const uint32_t M = 1u << s.m;
-    uint32_t rank[6] = {};  // the kernels take the gate's bits in the order of their state bits
-    for (uint32_t j = 0; j < s.m; ++j)
-      for (uint32_t i = 0; i < s.m; ++i) rank[j] += s.q[i] < s.q[j];
-    auto sorted = [&](uint32_t x) {
-      uint32_t o = 0;
-      for (uint32_t j = 0; j < s.m; ++j) o |= ((x >> j) & 1u) << rank[j];
-      return o;
-    };
     for (uint32_t r = 0; r < M; ++r)
       for (uint32_t c = 0; c < M; ++c) {
         const cd v = s.mat[size_t(r) * M + c];
-        const size_t o = 2 * (size_t(sorted(r)) * M + sorted(c));
+        const size_t o = 2 * (size_t(r) * M + c);
         if (dtype == QSVB_C128) {
           static_cast<double*>(dst)[o] = v.real();
           static_cast<double*>(dst)[o + 1] = v.imag();
@@ -1249,13 +1350,16 @@ void pack_sweep_matrix(const Sweep& s, int dtype, void* dst) {
 }
 
 template <class R>
-void launch_sweep(const LaunchEnv& env, R* re, R* im, uint32_t n, const Sweep& s, const void* dev_mat) {
+void launch_sweep(const LaunchEnv& env, R* re, R* im, uint32_t n, const Sweep& s, const void* dev_mat, bool tail) {
   switch (s.kind) {
     case SK_1Q: launch_pair<R>(env, re, im, n, s.target, nullptr, 0, s.mat); break;
     case SK_CTRL: launch_pair<R>(env, re, im, n, s.target, s.ctrl, s.nctrl, s.mat); break;
     case SK_DIAG: launch_diag<R>(env, re, im, n, s); break;
     case SK_PHASE: launch_phase<R>(env, re, im, n, s, dev_mat); break;
-    case SK_DENSE: launch_dense<R>(env, re, im, n, s, dev_mat); break;
+    case SK_DENSE:
+      if (tail && s.tail_m) launch_dense<R, true>(env, re, im, n, s, dev_mat);
+      else launch_dense<R, false>(env, re, im, n, s, dev_mat);
+      break;
     case SK_DENSE_TC:
       if constexpr (sizeof(R) == 4) {
         launch_tc_dense(env, reinterpret_cast<float*>(re), reinterpret_cast<float*>(im), n, s, dev_mat);
@@ -1331,7 +1435,7 @@ void launch_probabilities(const LaunchEnv& e, const R* re, const R* im, uint64_t
 }
 
 #define QSVB_INST(R)                                                                                   \
-  template void launch_sweep<R>(const LaunchEnv&, R*, R*, uint32_t, const Sweep&, const void*);       \
+  template void launch_sweep<R>(const LaunchEnv&, R*, R*, uint32_t, const Sweep&, const void*, bool); \
   template void launch_init_basis<R>(const LaunchEnv&, R*, R*, uint32_t, uint64_t);                   \
   template void launch_init_gaussian<R>(const LaunchEnv&, R*, R*, uint32_t, uint64_t);                \
   template void launch_scale<R>(const LaunchEnv&, R*, R*, uint32_t, const double*);                   \

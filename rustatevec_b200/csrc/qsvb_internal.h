@@ -121,6 +121,14 @@ struct Sweep {
   // the last matrix's columns 0, 1 land on output tile positions 0, 1 (16-byte epilogue stores)
   uint8_t chain_bk[kChainMaxMats] = {};
   uint8_t chain_evec = 0;
+  // set by attach_diagonals: a dense sweep's tail (a diagonal on tail_m qubits, sub-index bit j <->
+  // tail_q[j], applied after the product where every bit of tail_need is 1), and the diagonal sweeps
+  // that such tails carry (launch_plan skips them)
+  uint32_t tail_m = 0;
+  uint32_t tail_q[6] = {0, 0, 0, 0, 0, 0};
+  uint32_t tail_need = 0;
+  std::vector<cd> tail;
+  bool carried = false;
 };
 
 std::vector<Gate> gates_from_circuit(const qsvb_circuit* c);
@@ -171,6 +179,9 @@ template <class F> void parallel_ranges(size_t n, size_t min_items, F&& fn) {
 // Tensor-core chain passes with qubit relabelling, then the permutation passes that restore every
 // qubit to its own state bit (chain_planner.cpp). max_mats: matrices per pass (1..3).
 std::vector<Sweep> plan_chain(const std::vector<Gate>& in, uint32_t n, uint32_t max_mats);
+// Lets dense sweeps carry diagonal sweeps in their write-back (Sweep::tail); the list of sweeps and
+// their costs stay as planned.
+void attach_diagonals(std::vector<Sweep>& sw, uint32_t n);
 void sweep_costs(const std::vector<Sweep>& sw, uint32_t n, int dtype, qsvb_plan_stats* st);
 qsvb_plan_opts default_opts();
 
@@ -186,10 +197,11 @@ template <class R> void launch_init_basis(const LaunchEnv& e, R* re, R* im, uint
 template <class R> void launch_init_gaussian(const LaunchEnv& e, R* re, R* im, uint32_t n, uint64_t seed);
 template <class R> void launch_scale(const LaunchEnv& e, R* re, R* im, uint32_t n, const double* d_norm);
 
-// One sweep. `dev_mat` points to the sweep's device-side matrix block (dense kinds only) laid out
+// One sweep, with its tail when `tail` is set. `dev_mat` points to the sweep's device-side matrix block (dense kinds only) laid out
 // by pack_dense_matrix(); other kinds carry their coefficients by value.
 template <class R>
-void launch_sweep(const LaunchEnv& e, R* re, R* im, uint32_t n, const Sweep& s, const void* dev_mat);
+void launch_sweep(const LaunchEnv& e, R* re, R* im, uint32_t n, const Sweep& s, const void* dev_mat,
+                  bool tail = false);
 // Device bytes the sweep's matrix block needs (0 when the coefficients travel by value).
 size_t sweep_matrix_bytes(const Sweep& s, int dtype);
 void pack_sweep_matrix(const Sweep& s, int dtype, void* host_dst);

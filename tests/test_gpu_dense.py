@@ -8,7 +8,7 @@ Tolerance: each output is a sum of 2^(k+1) products whose absolute values add up
 import numpy as np
 import pytest
 
-from rustatevec_b200 import Plan, PLAN_AS_GIVEN, ENGINE_CUDA_CORE
+from rustatevec_b200 import Plan, PLAN_AS_GIVEN, PLAN_GREEDY, ENGINE_CUDA_CORE
 from rustatevec_b200 import _lib as L
 from rustatevec_b200 import gate as G
 from rustatevec_b200.circuit import Circuit
@@ -57,4 +57,55 @@ def test_dense_sweep_every_size_class(be64, be32, precision, k, n):
         plan.run(st)
         err = max_abs_diff(numpy_run(c, psi), be.download(st).as_complex())
         assert err <= (2 ** (k + 1) + 4) * UNIT[precision], (qs, err)
+    st.free()
+
+
+def diagonal(m, rng, controls=0):
+    """A random diagonal on m qubits that acts only where the lowest `controls` bits are 1."""
+    d = np.exp(1j * rng.uniform(0, 2 * np.pi, size=1 << m))
+    d[(np.arange(1 << m) & ((1 << controls) - 1)) != (1 << controls) - 1] = 1.0
+    return np.diag(d)
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+@pytest.mark.parametrize("k,n", [(2, 5), (2, 11), (3, 11), (4, 11), (5, 11), (6, 11), (2, 21), (3, 22), (4, 22), (5, 20)])
+def test_diagonal_carried_by_a_dense_sweep(be64, be32, precision, k, n):
+    """A dense sweep that multiplies by the following diagonal gives the two sweeps' own bits (to rounding
+    where the diagonal went into the matrix); with a second diagonal moved back past a sweep on other
+    qubits, the circuit is right to rounding."""
+    be = be64 if precision == "f64" else be32
+    rng = np.random.default_rng(10 * k + n)
+    st = be.alloc(n)
+    qsets = placements(n, k, rng)
+    for i, qs in enumerate(qsets if n < 17 else qsets[::4]):
+        if len(set(qs)) < k:
+            continue
+        m = 1 + i % 4
+        psi = rng.normal(size=1 << n) + 1j * rng.normal(size=1 << n)
+        psi = (psi / np.linalg.norm(psi)).astype(np.complex128 if precision == "f64" else np.complex64)
+        c = Circuit(n)
+        c.push(G.DenseGate(k, unitary(k, rng)), qs)
+        inside = i % 3 == 2  # on the dense gate's own qubits: multiplied into its matrix
+        dq = rng.permutation(qs)[:m].tolist() if inside else rng.choice(n, size=m, replace=False).tolist()
+        m = len(dq)
+        inside = set(dq) <= set(qs)
+        c.push(G.DenseGate(m, diagonal(m, rng, controls=i % 2)), dq)
+        got = []
+        for planner in (PLAN_AS_GIVEN, PLAN_GREEDY):  # (a width cap of 1 leaves the gates apart)
+            plan = Plan(be, c, L.make_opts(planner, 1, ENGINE_CUDA_CORE))
+            assert plan.stats()["by_kind"] == {"dense": 1, "diag": 1}
+            be.upload(st, psi.real, psi.imag)
+            plan.run(st)
+            got.append(be.download(st).as_complex())
+        if inside:
+            assert max_abs_diff(got[0], got[1]) <= 2 * (2 ** (k + 1) + 8) * UNIT[precision], (qs, dq)
+        else:
+            assert np.array_equal(got[0], got[1]), (qs, dq)
+        rest = [q for q in range(n) if q not in qs][:2]
+        c.push(G.DenseGate(2, unitary(2, rng)), rest)
+        c.push(G.DenseGate(2, diagonal(2, rng)), [qs[0], qs[-1]])
+        be.upload(st, psi.real, psi.imag)
+        Plan(be, c, L.make_opts(PLAN_GREEDY, 1, ENGINE_CUDA_CORE)).run(st)
+        err = max_abs_diff(numpy_run(c, psi), be.download(st).as_complex())
+        assert err <= (2 ** (k + 1) + 2 ** 3 + 20) * UNIT[precision], (qs, m, err)
     st.free()
