@@ -280,6 +280,7 @@ int qsvb_destroy(qsvb_ctx* c) {
     if (c->d_mat_ring) cudaFree(c->d_mat_ring);
     if (c->d_exec_mats) cudaFree(c->d_exec_mats);
     if (c->d_prob) cudaFree(c->d_prob);
+    if (c->d_sample) cudaFree(c->d_sample);
     if (c->d_err) cudaFree(c->d_err);
     for (int i = 0; i < 2; ++i) {
       if (c->h_pin[i]) cudaFreeHost(c->h_pin[i]);

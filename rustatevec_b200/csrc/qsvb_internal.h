@@ -269,6 +269,8 @@ struct qsvb_ctx {
   size_t exec_mats_cap = 0;
   void* d_prob = nullptr;         // probability staging chunk
   size_t prob_cap = 0;
+  char* d_sample = nullptr;       // sampling scratch (sample.cu)
+  size_t sample_cap = 0;
   int* d_err = nullptr;           // device error flag (bounded waits)
   void* h_pin[2] = {nullptr, nullptr};      // pinned host ring for large device -> host copies
   cudaEvent_t pin_ev[2] = {nullptr, nullptr};
