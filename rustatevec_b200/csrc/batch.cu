@@ -57,29 +57,59 @@ constexpr long long kSpinBudget = 1ll << 32;  // default dependency-wait budget,
 constexpr uint32_t kStageBytes = 32768;       // shared memory for one pass's program
 // The same for tile sweeps: small enough for five blocks per SM (larger programs are read from
 // global memory through L1).
-constexpr uint32_t kTileStageBytes = 8192;
+constexpr uint32_t kTileStageBytes = 7680;
 constexpr int kTileHi = 128;  // address / swizzle table entries of tile sweeps (<= 12 local bits)
 
+// A phase's program is a list of rounds. A round is straight-line code over the register bits j in
+// ascending order (run_round): for each j an optional point of diagonals (a table of one factor per
+// register slot, and diagonals on single register bits whose entries depend on bits of the thread's group
+// index) and an optional 1-qubit gate on bit j, then the CX gates from register bit j to j + 1, ascending.
+// OP_ROUND is the round's header; its gates and diagonals follow in the order in which it reaches them.
+// What does not fit (other CX gates, 2-qubit matrices, OP_D1T, OP_DT) comes first in a round of its own.
+//   Why rounds: one instruction at a time through a jump on (operation, register bit), the 2^RB
+// amplitudes met in registers at the end of some 60 branches, and the compiler moved them all to common
+// registers after every instruction: of 373 instructions an amplitude in QFT(26)'s first pass 72 were
+// arithmetic, 160 moves and integer operations, and the jumps stalled on top.
+//
 // OP_D1T: a diagonal on one register bit whose two entries depend on one bit of the tile index
 // (a 2-qubit diagonal with one qubit outside the tile); OP_DT: a phase that depends only on tile
-// bits (a diagonal whose qubits are all outside the tile), applied to every amplitude.
-// OP_D1P / OP_DTP: the same as OP_D1 / OP_DT with coefficients computed once per tile from a
-// phase sum over tile bits (tile sweeps merge runs of diagonal gates into them).
+// bits (a diagonal whose qubits are all outside the tile), applied to every amplitude. Tile sweeps
+// merge those with unit-modulus entries into phase sums over the tile bits and these into the slot tables,
+// which are then computed once per tile.
 enum BatchOp : uint32_t {
-  OP_PHASE = 0, OP_1Q = 1, OP_D1 = 2, OP_CX = 3, OP_2Q = 4, OP_D2 = 5, OP_D1T = 6, OP_DT = 7, OP_D1P = 8, OP_DTP = 9,
-  OP_DTAB = 10,  // the product of a phase's diagonal gates: one factor per register slot
-  OP_1QR = 11,   // a real 1-qubit gate [[a, b], [c, d]] (RY, H, X): half the work of a general one
-  OP_1QX = 12,   // [[a, i b], [i c, d]] with a..d real (RX, Y): half the work as well
-  OP_D1G = 13    // a diagonal on one register bit whose entries depend on bits of the group index
+  OP_PHASE = 0, OP_ROUND = 1,
+  OP_1Q = 2,
+  OP_1QR = 3,    // a real 1-qubit gate [[a, b], [c, d]] (RY, H, X): half the work of a general one
+  OP_1QX = 4,    // [[a, i b], [i c, d]] with a..d real (RX, Y): half the work as well
+  OP_TAB = 5,    // one factor per register slot (a: the table is one of the tile's, index coef)
+  OP_D1G = 6, OP_D1GH = 7,  // a diagonal on one register bit whose entries depend on bits of the group
+                            // index (H: the 0 side is 1)
+  OP_CX = 8, OP_2Q = 9, OP_D1T = 10, OP_DT = 11,
+  // host only
+  OP_D1 = 12, OP_D2 = 13, OP_D1P = 14, OP_DTP = 15
 };
-constexpr uint32_t kTphSlots = 32;  // per-tile phase operations per pass (tile sweeps)
-constexpr uint32_t kTphSlotR = 12;  // reals per slot (the OP_D1 coefficient block of either precision)
+// OP_ROUND's word a: 2 bits per register bit for its gate (1 real, 2 imaginary off the diagonal, 3
+// general), then the CX gates, whether another operation comes first, and 2 bits per register bit for the
+// table in front of its gate (1: all slots, 2: factors other than 1 only where the register bit below is
+// 1). Word b: 5 bits per register bit, the register bits of the group-dependent diagonals there.
+constexpr uint32_t kRoundCx = 10, kRoundOther = 14, kRoundTab = 15, kRoundBits = 5;
+constexpr uint32_t kTphSlots = 16;  // per-tile phase sums per pass (tile sweeps), and tables made of them
+constexpr uint32_t kTabNone = 255;
+// one such table: its constant factors (index of 2^RB complex FP64 values), the phase sum on each register
+// bit and the one on all slots (kTabNone: none)
+struct TileTab {
+  uint32_t base;
+  uint8_t bit[5], all;
+};
+// reals of a slot table (complex64: per pair of slots the pairs (re), (im), (-im))
+template <class R> constexpr uint32_t tab_reals(uint32_t rb) { return (sizeof(R) == 4 ? 3u : 2u) << rb; }
 
 struct Instr {
   uint32_t op;
-  uint32_t a, b;  // register bits (1Q/D1/D1T: a; CX: a = control, b = target; 2Q/D2: a < b, matrix bit 0 <->
-                  // a); D1T: b = tile bit; DT: b = tile bit of entry bit 0 | (tile bit of entry bit 1
-                  // << 8) | (number of tile bits << 16)
+  uint32_t a, b;  // rounds: see kRoundCx; 1-qubit gates: a = register bit; CX: a = control, b = target; 2Q:
+                  // a < b, matrix bit 0 <-> a; D1G: a = register bit, b = the windows of its tables (gd1g);
+                  // D1T: a = register bit, b = tile bit; DT: b = tile bit of entry bit 0 | (tile bit of
+                  // entry bit 1 << 8) | (number of tile bits << 16)
   uint32_t coef;  // complex index into the coefficient array (OP_PHASE: phase index)
 };
 
@@ -104,6 +134,7 @@ struct PassDev {
   uint32_t phase_off, nphase, coef_off, ncoef;  // the pass's phases and coefficients (complex units)
   uint32_t staged;       // program fits the shared-memory staging area
   uint32_t tph_n, tph_off;  // per-tile phase sums: count and byte offset from this record
+  uint32_t ttab_n, ttab_off, ttab_base;  // slot tables made of them: records, constant factors
 };
 
 struct Item {
@@ -157,79 +188,127 @@ __device__ __forceinline__ void cmac(R& yr, R& yi, R ar, R ai, R xr, R xi) {
   yi = fma(ai, xr, yi);
 }
 
-// ---- register storage of one group: complex64 keeps amplitude pairs (s, s^1) in float2 registers
-// so a gate on any register bit but 0 runs on Blackwell's paired FP32 FMA (two amplitudes per
-// instruction); complex128 keeps one amplitude per register.
+// ---- register storage of one group: complex64 keeps amplitude pairs (s, s^1) side by side so a gate
+// on any register bit but 0 runs on Blackwell's paired FP32 FMA (two amplitudes per instruction);
+// complex128 keeps one amplitude per register. Updates are written in the order that lets each overwrite
+// its own operand.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
 template <class R, int RB> struct Regs;
+// (kept as its two floats: held as 64-bit values, the same program ran 12 % slower in the batched runner)
+struct PairReg {
+  float2 v;
+  __device__ __forceinline__ operator f32x2() const { return pack2(v.x, v.y); }
+  __device__ __forceinline__ PairReg& operator=(f32x2 x) {
+    v = unpack2(x);
+    return *this;
+  }
+};
 template <int RB> struct Regs<float, RB> {
-  float2 r[(1 << RB) / 2], i[(1 << RB) / 2];
-  __device__ __forceinline__ float& re(int s) { return (s & 1) ? r[s >> 1].y : r[s >> 1].x; }
-  __device__ __forceinline__ float& im(int s) { return (s & 1) ? i[s >> 1].y : i[s >> 1].x; }
+  PairReg r[(1 << RB) / 2], i[(1 << RB) / 2];
+  __device__ __forceinline__ float re(int s) const { return (s & 1) ? unpack2(r[s >> 1]).y : unpack2(r[s >> 1]).x; }
+  __device__ __forceinline__ float im(int s) const { return (s & 1) ? unpack2(i[s >> 1]).y : unpack2(i[s >> 1]).x; }
+  __device__ __forceinline__ void set(int s, float a, float b) {
+    const float2 x = unpack2(r[s >> 1]), y = unpack2(i[s >> 1]);
+    r[s >> 1] = (s & 1) ? pack2(x.x, a) : pack2(a, x.y);
+    i[s >> 1] = (s & 1) ? pack2(y.x, b) : pack2(b, y.y);
+  }
+  // the pair h times the factors (pr, pi), npi = -pi
+  __device__ __forceinline__ void mul(int h, f32x2 pr, f32x2 pi, f32x2 npi) {
+    const f32x2 a = mul2(npi, i[h]), b = mul2(pi, r[h]);
+    r[h] = fma2(pr, r[h], a);
+    i[h] = fma2(pr, i[h], b);
+  }
 };
 template <int RB> struct Regs<double, RB> {
   double r[1 << RB], i[1 << RB];
-  __device__ __forceinline__ double& re(int s) { return r[s]; }
-  __device__ __forceinline__ double& im(int s) { return i[s]; }
+  __device__ __forceinline__ double re(int s) const { return r[s]; }
+  __device__ __forceinline__ double im(int s) const { return i[s]; }
+  __device__ __forceinline__ void set(int s, double a, double b) {
+    r[s] = a;
+    i[s] = b;
+  }
 };
+// slot s times (pr, pi)
+template <class R, int RB> __device__ __forceinline__ void mul_slot(Regs<R, RB>& v, int s, R pr, R pi) {
+  const R a = -pi * v.im(s), b = pi * v.re(s);
+  v.set(s, fma(pr, v.re(s), a), fma(pr, v.im(s), b));
+}
 
 // ---- gates on register bits (compile-time bit positions, so the amplitudes stay in registers)
 template <int J, class R, int RB>
 __device__ __forceinline__ void g1q(Regs<R, RB>& v, const R* __restrict__ c) {
   if constexpr (J < RB) {
     if constexpr (std::is_same<R, float>::value) {
-      // complex64 coefficients come pre-broadcast as float2 pairs: for each of a, b, c, d (the 2x2
-      // in row-major order) the pairs (re, re), (im, im), (-im, -im)
-      const float2* cc = reinterpret_cast<const float2*>(c);
+      // complex64 coefficients come pre-broadcast as pairs: for each of a, b, c, d (the 2x2 in
+      // row-major order) the pairs (re, re), (im, im), (-im, -im)
+      const f32x2* cc = reinterpret_cast<const f32x2*>(c);
       if constexpr (J >= 1) {
         // two amplitudes per instruction; same operation order as the scalar path below
         constexpr int HJ = 1 << (J - 1);
-        const float2 A0 = cc[0], A1 = cc[1], NA1 = cc[2], B0 = cc[3], B1 = cc[4], NB1 = cc[5];
-        const float2 C0 = cc[6], C1 = cc[7], NC1 = cc[8], D0 = cc[9], D1 = cc[10], ND1 = cc[11];
+        const f32x2 A0 = cc[0], A1 = cc[1], NA1 = cc[2], B0 = cc[3], B1 = cc[4], NB1 = cc[5];
+        const f32x2 C0 = cc[6], C1 = cc[7], NC1 = cc[8], D0 = cc[9], D1 = cc[10], ND1 = cc[11];
 #pragma unroll
         for (int h = 0; h < (1 << RB) / 2; ++h) {
           if (h & HJ) continue;
           const int t = h | HJ;
-          const float2 xr0 = v.r[h], xi0 = v.i[h], xr1 = v.r[t], xi1 = v.i[t];
-          float2 yr0 = __fmul2_rn(A0, xr0), yi0 = __fmul2_rn(A0, xi0);
-          float2 yr1 = __fmul2_rn(C0, xr0), yi1 = __fmul2_rn(C0, xi0);
-          yr0 = __ffma2_rn(NA1, xi0, yr0);
-          yi0 = __ffma2_rn(A1, xr0, yi0);
-          yr1 = __ffma2_rn(NC1, xi0, yr1);
-          yi1 = __ffma2_rn(C1, xr0, yi1);
-          yr0 = __ffma2_rn(B0, xr1, yr0);
-          yi0 = __ffma2_rn(B0, xi1, yi0);
-          yr1 = __ffma2_rn(D0, xr1, yr1);
-          yi1 = __ffma2_rn(D0, xi1, yi1);
-          yr0 = __ffma2_rn(NB1, xi1, yr0);
-          yi0 = __ffma2_rn(B1, xr1, yi0);
-          yr1 = __ffma2_rn(ND1, xi1, yr1);
-          yi1 = __ffma2_rn(D1, xr1, yi1);
-          v.r[h] = yr0;
-          v.i[h] = yi0;
-          v.r[t] = yr1;
-          v.i[t] = yi1;
+          const f32x2 xr0 = v.r[h], xi0 = v.i[h], xr1 = v.r[t], xi1 = v.i[t];
+          f32x2 yr0 = mul2(A0, xr0), yi0 = mul2(A0, xi0);
+          f32x2 yr1 = mul2(C0, xr0), yi1 = mul2(C0, xi0);
+          yr0 = fma2(NA1, xi0, yr0);
+          yi0 = fma2(A1, xr0, yi0);
+          yr1 = fma2(NC1, xi0, yr1);
+          yi1 = fma2(C1, xr0, yi1);
+          yr0 = fma2(B0, xr1, yr0);
+          yi0 = fma2(B0, xi1, yi0);
+          yr1 = fma2(D0, xr1, yr1);
+          yi1 = fma2(D0, xi1, yi1);
+          v.r[h] = fma2(NB1, xi1, yr0);
+          v.i[h] = fma2(B1, xr1, yi0);
+          v.r[t] = fma2(ND1, xi1, yr1);
+          v.i[t] = fma2(D1, xr1, yi1);
         }
       } else {
-        const float a0 = cc[0].x, a1 = cc[1].x, b0 = cc[3].x, b1 = cc[4].x;
-        const float c0 = cc[6].x, c1 = cc[7].x, d0 = cc[9].x, d1 = cc[10].x;
+        const float a0 = unpack2(cc[0]).x, a1 = unpack2(cc[1]).x, b0 = unpack2(cc[3]).x, b1 = unpack2(cc[4]).x;
+        const float c0 = unpack2(cc[6]).x, c1 = unpack2(cc[7]).x, d0 = unpack2(cc[9]).x, d1 = unpack2(cc[10]).x;
 #pragma unroll
         for (int h = 0; h < (1 << RB) / 2; ++h) {
-          const float xr0 = v.r[h].x, xi0 = v.i[h].x, xr1 = v.r[h].y, xi1 = v.i[h].y;
-          float yr0 = a0 * xr0, yi0 = a0 * xi0, yr1 = c0 * xr0, yi1 = c0 * xi0;
-          yr0 = fmaf(-a1, xi0, yr0);
-          yi0 = fmaf(a1, xr0, yi0);
-          yr1 = fmaf(-c1, xi0, yr1);
-          yi1 = fmaf(c1, xr0, yi1);
-          yr0 = fmaf(b0, xr1, yr0);
-          yi0 = fmaf(b0, xi1, yi0);
-          yr1 = fmaf(d0, xr1, yr1);
-          yi1 = fmaf(d0, xi1, yi1);
-          yr0 = fmaf(-b1, xi1, yr0);
-          yi0 = fmaf(b1, xr1, yi0);
-          yr1 = fmaf(-d1, xi1, yr1);
-          yi1 = fmaf(d1, xr1, yi1);
-          v.r[h] = make_float2(yr0, yr1);
-          v.i[h] = make_float2(yi0, yi1);
+          const float2 xr = unpack2(v.r[h]), xi = unpack2(v.i[h]);
+          float yr0 = a0 * xr.x, yi0 = a0 * xi.x, yr1 = c0 * xr.x, yi1 = c0 * xi.x;
+          yr0 = fmaf(-a1, xi.x, yr0);
+          yi0 = fmaf(a1, xr.x, yi0);
+          yr1 = fmaf(-c1, xi.x, yr1);
+          yi1 = fmaf(c1, xr.x, yi1);
+          yr0 = fmaf(b0, xr.y, yr0);
+          yi0 = fmaf(b0, xi.y, yi0);
+          yr1 = fmaf(d0, xr.y, yr1);
+          yi1 = fmaf(d0, xi.y, yi1);
+          yr0 = fmaf(-b1, xi.y, yr0);
+          yi0 = fmaf(b1, xr.y, yi0);
+          yr1 = fmaf(-d1, xi.y, yr1);
+          yi1 = fmaf(d1, xr.y, yi1);
+          v.r[h] = pack2(yr0, yr1);
+          v.i[h] = pack2(yi0, yi1);
         }
       }
     } else {
@@ -248,14 +327,8 @@ __device__ __forceinline__ void g1q(Regs<R, RB>& v, const R* __restrict__ c) {
         yi0 = fma(b0, xi1, yi0);
         yr1 = fma(d0, xr1, yr1);
         yi1 = fma(d0, xi1, yi1);
-        yr0 = fma(-b1, xi1, yr0);
-        yi0 = fma(b1, xr1, yi0);
-        yr1 = fma(-d1, xi1, yr1);
-        yi1 = fma(d1, xr1, yi1);
-        v.re(s) = yr0;
-        v.im(s) = yi0;
-        v.re(t) = yr1;
-        v.im(t) = yi1;
+        v.set(s, fma(-b1, xi1, yr0), fma(b1, xr1, yi0));
+        v.set(t, fma(-d1, xi1, yr1), fma(d1, xr1, yi1));
       }
     }
   }
@@ -267,71 +340,71 @@ __device__ __forceinline__ void gd1(Regs<R, RB>& v, const R* __restrict__ c) {
     if constexpr (std::is_same<R, float>::value) {
       // pre-broadcast pairs (re, im, -im) for the 0 side and the 1 side of bit J; for J == 0 the
       // pair (s, s^1) straddles bit J, so both sets hold (value at s, value at s^1)
-      const float2* cc = reinterpret_cast<const float2*>(c);
-      const float2 pr0 = cc[0], pi0 = cc[1], npi0 = cc[2], pr1 = cc[3], pi1 = cc[4], npi1 = cc[5];
+      const f32x2* cc = reinterpret_cast<const f32x2*>(c);
 #pragma unroll
-      for (int h = 0; h < (1 << RB) / 2; ++h) {
-        const bool one = J >= 1 && (h & (1 << (J >= 1 ? J - 1 : 0)));
-        const float2 pr = one ? pr1 : pr0, pi = one ? pi1 : pi0, npi = one ? npi1 : npi0;
-        const float2 xr = v.r[h], xi = v.i[h];
-        v.r[h] = __ffma2_rn(pr, xr, __fmul2_rn(npi, xi));
-        v.i[h] = __ffma2_rn(pr, xi, __fmul2_rn(pi, xr));
+      for (int side = 0; side < 2; ++side) {
+        const f32x2 pr = cc[3 * side], pi = cc[3 * side + 1], npi = cc[3 * side + 2];
+#pragma unroll
+        for (int h = 0; h < (1 << RB) / 2; ++h)
+          if ((J >= 1 ? (h >> (J >= 1 ? J - 1 : 0)) & 1 : 0) == side) v.mul(h, pr, pi, npi);
+        if (J == 0) break;
       }
     } else {
-      const R p0r = c[0], p0i = c[1], p1r = c[2], p1i = c[3];
 #pragma unroll
       for (int s = 0; s < (1 << RB); ++s) {
-        const R pr = (s & (1 << J)) ? p1r : p0r, pi = (s & (1 << J)) ? p1i : p0i;
-        const R xr = v.re(s), xi = v.im(s);
-        v.re(s) = fma(pr, xr, -pi * xi);
-        v.im(s) = fma(pr, xi, pi * xr);
+        const int side = (s >> J) & 1;
+        mul_slot<R, RB>(v, s, c[2 * side], c[2 * side + 1]);
       }
     }
   }
 }
 
-// Diagonal on register bit J whose entries depend on bits of this thread's group index gidx (local
-// qubits outside the phase's registers, constant per group): for each set bit k of mask, in
-// ascending order, c holds the four entries of one 2-qubit diagonal (index: register bit | group
-// bit k << 1, complex pairs). The thread multiplies the entries its group bits select, then applies
-// the resulting diag(f0, f1).
-template <int J, class R, int RB>
-__device__ __forceinline__ void gd1g(Regs<R, RB>& v, const R* __restrict__ c, uint32_t mask, uint32_t gidx) {
+// Diagonal on register bit J whose entries depend on bits of this thread's group index (local qubits
+// outside the phase's registers, constant per group): the product of several 2-qubit diagonals, taken
+// from one or two tables that the host multiplied out, each over a window of the index's bits (window:
+// first bit and width of the first table, then of the second, 4 bits each; width 0: none). An entry is the
+// pair (f0, f1) of complex factors of the two sides, or f1 alone when f0 is 1 throughout (HALF: controlled
+// phases). Multiplying the selected entries of every diagonal in each thread instead took up to 8 rounds
+// of two complex products.
+template <class R> using Cplx = std::conditional_t<sizeof(R) == 8, double2, float2>;
+template <class R> __device__ __forceinline__ Cplx<R> cmul(const Cplx<R>& a, const Cplx<R>& b) {
+  return {a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x};
+}
+template <int J, class R, int RB, bool HALF>
+__device__ __forceinline__ void gd1g(Regs<R, RB>& v, const R* __restrict__ c, uint32_t window, uint32_t gidx) {
   if constexpr (J < RB) {
-    R f0r = 1, f0i = 0, f1r = 1, f1i = 0;
-    for (uint32_t mm = mask; mm; mm &= mm - 1u, c += 8) {
-      const R* d = c + 4 * ((gidx >> (__ffs(mm) - 1)) & 1u);
-      const R a0r = d[0], a0i = d[1], a1r = d[2], a1i = d[3];
-      const R t0 = f0r * a0r - f0i * a0i, t1 = f1r * a1r - f1i * a1i;
-      f0i = f0r * a0i + f0i * a0r;
-      f1i = f1r * a1i + f1i * a1r;
-      f0r = t0;
-      f1r = t1;
+    constexpr uint32_t E = HALF ? 1 : 2;
+    const Cplx<R>* tab = reinterpret_cast<const Cplx<R>*>(c);
+    const uint32_t w0 = (window >> 4) & 15u, w1 = (window >> 12) & 15u;
+    const Cplx<R>* t0 = tab + E * ((gidx >> (window & 15u)) & ((1u << w0) - 1u));
+    Cplx<R> f0 = {R(1), R(0)}, f1 = t0[E - 1];
+    if constexpr (!HALF) f0 = t0[0];
+    if (w1) {
+      const Cplx<R>* t1 = tab + E * ((1u << w0) + ((gidx >> ((window >> 8) & 15u)) & ((1u << w1) - 1u)));
+      f1 = cmul<R>(f1, t1[E - 1]);
+      if constexpr (!HALF) f0 = cmul<R>(f0, t1[0]);
     }
     if constexpr (std::is_same<R, float>::value) {
+      if constexpr (J == 0) {  // the pair (2h, 2h+1) straddles bit 0
+        const f32x2 pr = pack2(f0.x, f1.x), pi = pack2(f0.y, f1.y), npi = pack2(-f0.y, -f1.y);
 #pragma unroll
-      for (int h = 0; h < (1 << RB) / 2; ++h) {
-        float2 pr, pi;
-        if constexpr (J == 0) {  // the pair (2h, 2h+1) straddles bit 0
-          pr = make_float2(f0r, f1r);
-          pi = make_float2(f0i, f1i);
-        } else {
-          const bool one = (h >> (J - 1)) & 1;
-          pr = one ? make_float2(f1r, f1r) : make_float2(f0r, f0r);
-          pi = one ? make_float2(f1i, f1i) : make_float2(f0i, f0i);
+        for (int h = 0; h < (1 << RB) / 2; ++h) v.mul(h, pr, pi, npi);
+      } else {
+#pragma unroll
+        for (int side = HALF ? 1 : 0; side < 2; ++side) {
+          const Cplx<R> f = side ? f1 : f0;
+          const f32x2 pr = pack2(f.x, f.x), pi = pack2(f.y, f.y), npi = pack2(-f.y, -f.y);
+#pragma unroll
+          for (int h = 0; h < (1 << RB) / 2; ++h)
+            if (((h >> (J - 1)) & 1) == side) v.mul(h, pr, pi, npi);
         }
-        const float2 npi = make_float2(-pi.x, -pi.y);
-        const float2 xr = v.r[h], xi = v.i[h];
-        v.r[h] = __ffma2_rn(pr, xr, __fmul2_rn(npi, xi));
-        v.i[h] = __ffma2_rn(pr, xi, __fmul2_rn(pi, xr));
       }
     } else {
 #pragma unroll
       for (int s = 0; s < (1 << RB); ++s) {
-        const R pr = (s & (1 << J)) ? f1r : f0r, pi = (s & (1 << J)) ? f1i : f0i;
-        const R xr = v.re(s), xi = v.im(s);
-        v.re(s) = fma(pr, xr, -pi * xi);
-        v.im(s) = fma(pr, xi, pi * xr);
+        const int side = (s >> J) & 1;
+        if (HALF && !side) continue;
+        mul_slot<R, RB>(v, s, side ? f1.x : f0.x, side ? f1.y : f0.y);
       }
     }
   }
@@ -345,10 +418,8 @@ __device__ __forceinline__ void gcx(Regs<R, RB>& v) {
       if (!(s & (1 << J)) || (s & (1 << K))) continue;
       const int t = s | (1 << K);
       const R tr = v.re(s), ti = v.im(s);
-      v.re(s) = v.re(t);
-      v.im(s) = v.im(t);
-      v.re(t) = tr;
-      v.im(t) = ti;
+      v.set(s, v.re(t), v.im(t));
+      v.set(t, tr, ti);
     }
   }
 }
@@ -371,68 +442,54 @@ __device__ __forceinline__ void g2q(Regs<R, RB>& v, const R* __restrict__ c) {
         R yr = 0, yi = 0;
 #pragma unroll
         for (int q = 0; q < 4; ++q) cmac(yr, yi, c[2 * (4 * r + q)], c[2 * (4 * r + q) + 1], xr[q], xi[q]);
-        v.re(idx[r]) = yr;
-        v.im(idx[r]) = yi;
+        v.set(idx[r], yr, yi);
       }
-    }
-  }
-}
-
-template <int J, int K, class R, int RB>
-__device__ __forceinline__ void gd2(Regs<R, RB>& v, const R* __restrict__ c) {
-  if constexpr (J < K && K < RB) {
-#pragma unroll
-    for (int s = 0; s < (1 << RB); ++s) {
-      const int d = ((s >> J) & 1) | (((s >> K) & 1) << 1);
-      const R pr = c[2 * d], pi = c[2 * d + 1];
-      const R xr = v.re(s), xi = v.im(s);
-      v.re(s) = fma(pr, xr, -pi * xi);
-      v.im(s) = fma(pr, xi, pi * xr);
     }
   }
 }
 
 // A 1-qubit gate whose entries are each real or imaginary, on register bit J: X false, the real
 // matrix [[a, b], [c, d]]; X true, [[a, i b], [i c, d]]. Four real multiplies per amplitude instead
-// of eight. Coefficients: complex128 (a, b), (c, d); complex64 float2 pairs broadcast on the host,
+// of eight. Coefficients: complex128 (a, b), (c, d); complex64 pairs broadcast on the host,
 // (a, a), (b, b), (c, c), (d, d) and, for X, (-b, -b), (-c, -c) after them.
 template <int J, class R, int RB, bool X>
 __device__ __forceinline__ void g1qs(Regs<R, RB>& v, const R* __restrict__ c) {
   if constexpr (J < RB) {
     if constexpr (std::is_same<R, float>::value) {
-      const float2* cc = reinterpret_cast<const float2*>(c);
-      const float2 A = cc[0], B = cc[1], Cc = cc[2], D = cc[3];
+      const f32x2* cc = reinterpret_cast<const f32x2*>(c);
+      const f32x2 A = cc[0], B = cc[1], Cc = cc[2], D = cc[3];
       if constexpr (J >= 1) {
         constexpr int HJ = 1 << (J - 1);
 #pragma unroll
         for (int h = 0; h < (1 << RB) / 2; ++h) {
           if (h & HJ) continue;
           const int t = h | HJ;
-          const float2 xr0 = v.r[h], xi0 = v.i[h], xr1 = v.r[t], xi1 = v.i[t];
           if constexpr (X) {
-            const float2 NB = cc[4], NC = cc[5];
-            v.r[h] = __ffma2_rn(NB, xi1, __fmul2_rn(A, xr0));
-            v.i[h] = __ffma2_rn(B, xr1, __fmul2_rn(A, xi0));
-            v.r[t] = __ffma2_rn(D, xr1, __fmul2_rn(NC, xi0));
-            v.i[t] = __ffma2_rn(D, xi1, __fmul2_rn(Cc, xr0));
+            const f32x2 NB = cc[4], NC = cc[5];
+            const f32x2 p = mul2(NC, v.i[h]), q = mul2(Cc, v.r[h]);
+            v.r[h] = fma2(NB, v.i[t], mul2(A, v.r[h]));
+            v.i[h] = fma2(B, v.r[t], mul2(A, v.i[h]));
+            v.r[t] = fma2(D, v.r[t], p);
+            v.i[t] = fma2(D, v.i[t], q);
           } else {
-            v.r[h] = __ffma2_rn(B, xr1, __fmul2_rn(A, xr0));
-            v.i[h] = __ffma2_rn(B, xi1, __fmul2_rn(A, xi0));
-            v.r[t] = __ffma2_rn(D, xr1, __fmul2_rn(Cc, xr0));
-            v.i[t] = __ffma2_rn(D, xi1, __fmul2_rn(Cc, xi0));
+            const f32x2 p = mul2(Cc, v.r[h]), q = mul2(Cc, v.i[h]);
+            v.r[h] = fma2(B, v.r[t], mul2(A, v.r[h]));
+            v.i[h] = fma2(B, v.i[t], mul2(A, v.i[h]));
+            v.r[t] = fma2(D, v.r[t], p);
+            v.i[t] = fma2(D, v.i[t], q);
           }
         }
       } else {
-        const float a = A.x, b = B.x, cs = Cc.x, d = D.x;
+        const float a = unpack2(A).x, b = unpack2(B).x, cs = unpack2(Cc).x, d = unpack2(D).x;
 #pragma unroll
         for (int h = 0; h < (1 << RB) / 2; ++h) {
-          const float xr0 = v.r[h].x, xi0 = v.i[h].x, xr1 = v.r[h].y, xi1 = v.i[h].y;
+          const float2 xr = unpack2(v.r[h]), xi = unpack2(v.i[h]);
           if constexpr (X) {
-            v.r[h] = make_float2(fmaf(-b, xi1, a * xr0), fmaf(d, xr1, -cs * xi0));
-            v.i[h] = make_float2(fmaf(b, xr1, a * xi0), fmaf(d, xi1, cs * xr0));
+            v.r[h] = pack2(fmaf(-b, xi.y, a * xr.x), fmaf(d, xr.y, -cs * xi.x));
+            v.i[h] = pack2(fmaf(b, xr.y, a * xi.x), fmaf(d, xi.y, cs * xr.x));
           } else {
-            v.r[h] = make_float2(fmaf(b, xr1, a * xr0), fmaf(d, xr1, cs * xr0));
-            v.i[h] = make_float2(fmaf(b, xi1, a * xi0), fmaf(d, xi1, cs * xi0));
+            v.r[h] = pack2(fmaf(b, xr.y, a * xr.x), fmaf(d, xr.y, cs * xr.x));
+            v.i[h] = pack2(fmaf(b, xi.y, a * xi.x), fmaf(d, xi.y, cs * xi.x));
           }
         }
       }
@@ -442,17 +499,18 @@ __device__ __forceinline__ void g1qs(Regs<R, RB>& v, const R* __restrict__ c) {
       for (int s = 0; s < (1 << RB); ++s) {
         if (s & (1 << J)) continue;
         const int t = s | (1 << J);
-        const R xr0 = v.re(s), xi0 = v.im(s), xr1 = v.re(t), xi1 = v.im(t);
         if constexpr (X) {
-          v.re(s) = fma(-b, xi1, a * xr0);
-          v.im(s) = fma(b, xr1, a * xi0);
-          v.re(t) = fma(d, xr1, -cs * xi0);
-          v.im(t) = fma(d, xi1, cs * xr0);
+          const R p = -cs * v.i[s], q = cs * v.r[s];
+          v.r[s] = fma(-b, v.i[t], a * v.r[s]);
+          v.i[s] = fma(b, v.r[t], a * v.i[s]);
+          v.r[t] = fma(d, v.r[t], p);
+          v.i[t] = fma(d, v.i[t], q);
         } else {
-          v.re(s) = fma(b, xr1, a * xr0);
-          v.im(s) = fma(b, xi1, a * xi0);
-          v.re(t) = fma(d, xr1, cs * xr0);
-          v.im(t) = fma(d, xi1, cs * xi0);
+          const R p = cs * v.r[s], q = cs * v.i[s];
+          v.r[s] = fma(b, v.r[t], a * v.r[s]);
+          v.i[s] = fma(b, v.i[t], a * v.i[s]);
+          v.r[t] = fma(d, v.r[t], p);
+          v.i[t] = fma(d, v.i[t], q);
         }
       }
     }
@@ -460,30 +518,27 @@ __device__ __forceinline__ void g1qs(Regs<R, RB>& v, const R* __restrict__ c) {
 }
 
 // One factor per register slot (a phase's diagonal gates multiplied out on the host). complex64:
-// per float2 pair h the factors of slots 2h and 2h+1 as (re), (im), (-im) pairs; complex128: one
-// complex per slot.
-template <class R, int RB>
+// per pair h the factors of slots 2h and 2h+1 as (re), (im), (-im) pairs; complex128: one complex per
+// slot. J >= 0: the factors are 1 wherever register bit J is 0, so only the other half is multiplied.
+template <int J, class R, int RB>
 __device__ __forceinline__ void gtab(Regs<R, RB>& v, const R* __restrict__ c) {
   if constexpr (std::is_same<R, float>::value) {
-    const float2* cc = reinterpret_cast<const float2*>(c);
+    const f32x2* cc = reinterpret_cast<const f32x2*>(c);
 #pragma unroll
     for (int h = 0; h < (1 << RB) / 2; ++h) {
-      const float2 pr = cc[3 * h], pi = cc[3 * h + 1], npi = cc[3 * h + 2];
-      const float2 xr = v.r[h], xi = v.i[h];
-      v.r[h] = __ffma2_rn(pr, xr, __fmul2_rn(npi, xi));
-      v.i[h] = __ffma2_rn(pr, xi, __fmul2_rn(pi, xr));
+      if (J >= 1 && !(h & (1 << (J >= 1 ? J - 1 : 0)))) continue;
+      v.mul(h, cc[3 * h], cc[3 * h + 1], cc[3 * h + 2]);
     }
   } else {
 #pragma unroll
     for (int s = 0; s < (1 << RB); ++s) {
-      const R pr = c[2 * s], pi = c[2 * s + 1];
-      const R xr = v.re(s), xi = v.im(s);
-      v.re(s) = fma(pr, xr, -pi * xi);
-      v.im(s) = fma(pr, xi, pi * xr);
+      if (J >= 0 && !(s & (1 << (J >= 0 ? J : 0)))) continue;
+      mul_slot<R, RB>(v, s, c[2 * s], c[2 * s + 1]);
     }
   }
 }
 
+#define QSVB_EACH(g) _Pragma("unroll") for (int g = 0; g < G; ++g)  // the thread's groups stay in registers
 #define QSVB_PAIR_CASES(F, ...)                       \
   case 0 * 8 + 1: F<0, 1, R, RB>(__VA_ARGS__); break; \
   case 0 * 8 + 2: F<0, 2, R, RB>(__VA_ARGS__); break; \
@@ -496,76 +551,21 @@ __device__ __forceinline__ void gtab(Regs<R, RB>& v, const R* __restrict__ c) {
   case 2 * 8 + 4: F<2, 4, R, RB>(__VA_ARGS__); break; \
   case 3 * 8 + 4: F<3, 4, R, RB>(__VA_ARGS__); break;
 
-// Applies one instruction to G groups held by this thread (the dispatch and the coefficient loads
-// are shared; the G independent updates interleave).
+// Applies an operation outside the rounds' pattern to G groups held by this thread.
 template <class R, int RB, int G>
-__device__ __forceinline__ void apply_instr(const Instr& in, Regs<R, RB>* v, const R* __restrict__ coef, uint32_t tile,
-                                            const R* tcoef, const uint32_t* grp) {
+__device__ __forceinline__ void apply_other(const Instr& in, Regs<R, RB>* v, const R* __restrict__ coef, uint32_t tile) {
   const R* c = coef + 2 * size_t(in.coef);
   switch (in.op) {
-    case OP_D1G:
-      switch (in.a) {
-        case 0: for (int g = 0; g < G; ++g) gd1g<0, R, RB>(v[g], c, in.b, grp[g]); break;
-        case 1: for (int g = 0; g < G; ++g) gd1g<1, R, RB>(v[g], c, in.b, grp[g]); break;
-        case 2: for (int g = 0; g < G; ++g) gd1g<2, R, RB>(v[g], c, in.b, grp[g]); break;
-        case 3: for (int g = 0; g < G; ++g) gd1g<3, R, RB>(v[g], c, in.b, grp[g]); break;
-        case 4: for (int g = 0; g < G; ++g) gd1g<4, R, RB>(v[g], c, in.b, grp[g]); break;
-      }
-      break;
-    case OP_DTAB:
-      for (int g = 0; g < G; ++g) gtab<R, RB>(v[g], c);
-      break;
-    case OP_1QR:
-      switch (in.a) {
-        case 0: for (int g = 0; g < G; ++g) g1qs<0, R, RB, false>(v[g], c); break;
-        case 1: for (int g = 0; g < G; ++g) g1qs<1, R, RB, false>(v[g], c); break;
-        case 2: for (int g = 0; g < G; ++g) g1qs<2, R, RB, false>(v[g], c); break;
-        case 3: for (int g = 0; g < G; ++g) g1qs<3, R, RB, false>(v[g], c); break;
-        case 4: for (int g = 0; g < G; ++g) g1qs<4, R, RB, false>(v[g], c); break;
-      }
-      break;
-    case OP_1QX:
-      switch (in.a) {
-        case 0: for (int g = 0; g < G; ++g) g1qs<0, R, RB, true>(v[g], c); break;
-        case 1: for (int g = 0; g < G; ++g) g1qs<1, R, RB, true>(v[g], c); break;
-        case 2: for (int g = 0; g < G; ++g) g1qs<2, R, RB, true>(v[g], c); break;
-        case 3: for (int g = 0; g < G; ++g) g1qs<3, R, RB, true>(v[g], c); break;
-        case 4: for (int g = 0; g < G; ++g) g1qs<4, R, RB, true>(v[g], c); break;
-      }
-      break;
-    case OP_D1P: {
-      c = tcoef + kTphSlotR * in.coef;
-      switch (in.a) {
-        case 0: for (int g = 0; g < G; ++g) gd1<0, R, RB>(v[g], c); break;
-        case 1: for (int g = 0; g < G; ++g) gd1<1, R, RB>(v[g], c); break;
-        case 2: for (int g = 0; g < G; ++g) gd1<2, R, RB>(v[g], c); break;
-        case 3: for (int g = 0; g < G; ++g) gd1<3, R, RB>(v[g], c); break;
-        case 4: for (int g = 0; g < G; ++g) gd1<4, R, RB>(v[g], c); break;
-      }
-      break;
-    }
-    case OP_DTP: {
-      c = tcoef + kTphSlotR * in.coef;
-      const R pr = c[0], pi = c[1];
-      for (int g = 0; g < G; ++g)
-#pragma unroll
-        for (int s = 0; s < (1 << RB); ++s) {
-          const R xr = v[g].re(s), xi = v[g].im(s);
-          v[g].re(s) = fma(pr, xr, -pi * xi);
-          v[g].im(s) = fma(pr, xi, pi * xr);
-        }
-      break;
-    }
     case OP_D1T: {
       // two coefficient blocks (tile bit 0 / 1) in the layout of OP_D1
       constexpr int blk = std::is_same<R, float>::value ? 6 : 2;  // complex entries per block
       c += 2 * blk * ((tile >> in.b) & 1u);
       switch (in.a) {
-        case 0: for (int g = 0; g < G; ++g) gd1<0, R, RB>(v[g], c); break;
-        case 1: for (int g = 0; g < G; ++g) gd1<1, R, RB>(v[g], c); break;
-        case 2: for (int g = 0; g < G; ++g) gd1<2, R, RB>(v[g], c); break;
-        case 3: for (int g = 0; g < G; ++g) gd1<3, R, RB>(v[g], c); break;
-        case 4: for (int g = 0; g < G; ++g) gd1<4, R, RB>(v[g], c); break;
+        case 0: QSVB_EACH(g) gd1<0, R, RB>(v[g], c); break;
+        case 1: QSVB_EACH(g) gd1<1, R, RB>(v[g], c); break;
+        case 2: QSVB_EACH(g) gd1<2, R, RB>(v[g], c); break;
+        case 3: QSVB_EACH(g) gd1<3, R, RB>(v[g], c); break;
+        case 4: QSVB_EACH(g) gd1<4, R, RB>(v[g], c); break;
       }
       break;
     }
@@ -574,40 +574,18 @@ __device__ __forceinline__ void apply_instr(const Instr& in, Regs<R, RB>* v, con
       uint32_t idx = (tile >> (in.b & 255u)) & 1u;
       if (nb == 2) idx |= ((tile >> ((in.b >> 8) & 255u)) & 1u) << 1;
       const R pr = c[2 * idx], pi = c[2 * idx + 1];
-      for (int g = 0; g < G; ++g)
+      QSVB_EACH(g)
 #pragma unroll
-        for (int s = 0; s < (1 << RB); ++s) {
-          const R xr = v[g].re(s), xi = v[g].im(s);
-          v[g].re(s) = fma(pr, xr, -pi * xi);
-          v[g].im(s) = fma(pr, xi, pi * xr);
-        }
+        for (int s = 0; s < (1 << RB); ++s) mul_slot<R, RB>(v[g], s, pr, pi);
       break;
     }
-    case OP_1Q:
-      switch (in.a) {
-        case 0: for (int g = 0; g < G; ++g) g1q<0, R, RB>(v[g], c); break;
-        case 1: for (int g = 0; g < G; ++g) g1q<1, R, RB>(v[g], c); break;
-        case 2: for (int g = 0; g < G; ++g) g1q<2, R, RB>(v[g], c); break;
-        case 3: for (int g = 0; g < G; ++g) g1q<3, R, RB>(v[g], c); break;
-        case 4: for (int g = 0; g < G; ++g) g1q<4, R, RB>(v[g], c); break;
-      }
-      break;
-    case OP_D1:
-      switch (in.a) {
-        case 0: for (int g = 0; g < G; ++g) gd1<0, R, RB>(v[g], c); break;
-        case 1: for (int g = 0; g < G; ++g) gd1<1, R, RB>(v[g], c); break;
-        case 2: for (int g = 0; g < G; ++g) gd1<2, R, RB>(v[g], c); break;
-        case 3: for (int g = 0; g < G; ++g) gd1<3, R, RB>(v[g], c); break;
-        case 4: for (int g = 0; g < G; ++g) gd1<4, R, RB>(v[g], c); break;
-      }
-      break;
     case OP_CX: {
       const uint32_t lo = min(in.a, in.b), hi = max(in.a, in.b);
       const bool fwd = in.a < in.b;  // the control is the lower register bit
       switch (lo * 8 + hi) {
 #define QSVB_CX_CASE(J, K)       \
   case J * 8 + K:                \
-    for (int g = 0; g < G; ++g)       \
+    QSVB_EACH(g)       \
       if (fwd) gcx<J, K, R, RB>(v[g]); \
       else gcx<K, J, R, RB>(v[g]);     \
     break;
@@ -626,84 +604,164 @@ __device__ __forceinline__ void apply_instr(const Instr& in, Regs<R, RB>* v, con
       break;
     }
     case OP_2Q:
-      for (int g = 0; g < G; ++g) switch (in.a * 8 + in.b) { QSVB_PAIR_CASES(g2q, v[g], c) }
+      QSVB_EACH(g) switch (in.a * 8 + in.b) { QSVB_PAIR_CASES(g2q, v[g], c) }
       break;
-    case OP_D2:
-      for (int g = 0; g < G; ++g) switch (in.a * 8 + in.b) { QSVB_PAIR_CASES(gd2, v[g], c) }
-      break;
+  }
+}
+
+// One register bit's part of a round: the diagonals in front of its gate, then the gate. k walks the
+// program; ttab: the tile's slot tables.
+template <int J, class R, int RB, int G>
+__device__ __forceinline__ void round_bit(const Instr& rd, const Instr* prog, uint32_t& k, Regs<R, RB>* v,
+                                          const R* __restrict__ coef, const R* __restrict__ ttab,
+                                          const uint32_t* grp) {
+  if constexpr (J < RB) {
+    const uint32_t tab = (rd.a >> (kRoundTab + 2 * J)) & 3u;
+    if (tab) {
+      const Instr in = prog[k++];
+      const R* c = in.a ? ttab + size_t(in.coef) * tab_reals<R>(RB) : coef + 2 * size_t(in.coef);
+      if (J >= 1 && tab == 2) {
+        QSVB_EACH(g) gtab<(J >= 1 ? J - 1 : 0), R, RB>(v[g], c);
+      } else {
+        QSVB_EACH(g) gtab<-1, R, RB>(v[g], c);
+      }
+    }
+    const uint32_t gm = (rd.b >> (5 * J)) & 31u;
+    if (gm) {
+#define QSVB_GROUP_DIAG(B)                                                                              \
+  if (gm & (1u << B)) {                                                                                 \
+    const Instr in = prog[k++];                                                                         \
+    const R* c = coef + 2 * size_t(in.coef);                                                            \
+    if (in.op == OP_D1GH)                                                                               \
+      QSVB_EACH(g) gd1g<B, R, RB, true>(v[g], c, in.b, grp[g]);                          \
+    else                                                                                                \
+      QSVB_EACH(g) gd1g<B, R, RB, false>(v[g], c, in.b, grp[g]);                         \
+  }
+      QSVB_GROUP_DIAG(0)
+      QSVB_GROUP_DIAG(1)
+      QSVB_GROUP_DIAG(2)
+      QSVB_GROUP_DIAG(3)
+      QSVB_GROUP_DIAG(4)
+#undef QSVB_GROUP_DIAG
+    }
+    const uint32_t kind = (rd.a >> (2 * J)) & 3u;
+    if (kind) {
+      const R* c = coef + 2 * size_t(prog[k++].coef);
+      if (kind == 1) {
+        QSVB_EACH(g) g1qs<J, R, RB, false>(v[g], c);
+      } else if (kind == 2) {
+        QSVB_EACH(g) g1qs<J, R, RB, true>(v[g], c);
+      } else {
+        QSVB_EACH(g) g1q<J, R, RB>(v[g], c);
+      }
+    }
+  }
+}
+
+template <class R, int RB, int G>
+__device__ __forceinline__ void run_rounds(const Instr* prog, uint32_t k, uint32_t kend, Regs<R, RB>* v,
+                                           const R* __restrict__ coef, const R* __restrict__ ttab, uint32_t tile,
+                                           const uint32_t* grp) {
+  while (k < kend) {
+    const Instr rd = prog[k++];
+    if ((rd.a >> kRoundOther) & 1u) {
+      apply_other<R, RB, G>(prog[k++], v, coef, tile);
+      continue;
+    }
+    round_bit<0, R, RB, G>(rd, prog, k, v, coef, ttab, grp);
+    round_bit<1, R, RB, G>(rd, prog, k, v, coef, ttab, grp);
+    round_bit<2, R, RB, G>(rd, prog, k, v, coef, ttab, grp);
+    round_bit<3, R, RB, G>(rd, prog, k, v, coef, ttab, grp);
+    round_bit<4, R, RB, G>(rd, prog, k, v, coef, ttab, grp);
+    const uint32_t cx = (rd.a >> kRoundCx) & 15u;
+    if (cx) {
+      if (cx & 1u)
+        QSVB_EACH(g) gcx<0, 1, R, RB>(v[g]);
+      if (cx & 2u)
+        QSVB_EACH(g) gcx<1, 2, R, RB>(v[g]);
+      if (cx & 4u)
+        QSVB_EACH(g) gcx<2, 3, R, RB>(v[g]);
+      if (cx & 8u)
+        QSVB_EACH(g) gcx<3, 4, R, RB>(v[g]);
+    }
   }
 }
 
 // One register phase for G groups of this thread: load 2^r amplitudes per group from the swizzled
-// tile, apply the phase's instructions, store them back.
+// tile, apply the phase's instructions, store them back. Offsets are bytes (rp: those of the register
+// bits' unit vectors); the imaginary parts lie `im` bytes above the real ones (a constant in tile sweeps,
+// so that an amplitude's two accesses share one address register).
 template <class R, int RB, int G>
-__device__ __forceinline__ void phase_groups(const uint32_t* grp, const PhaseDev& D, const uint32_t* rp, R* xr, R* xi,
-                                             const Instr* pprog, uint32_t kbeg, uint32_t kend, const R* pcoef,
-                                             uint32_t tile, const R* tcoef) {
+__device__ __forceinline__ void phase_groups(const uint32_t* grp, const PhaseDev& D, const uint32_t* rp, char* sm,
+                                             uint32_t im, const Instr* pprog, uint32_t kbeg, uint32_t kend,
+                                             const R* pcoef, uint32_t tile, const R* ttab) {
   constexpr int NV = 1 << RB;
   const uint32_t r = D.r;
   uint32_t p0[G];
   Regs<R, RB> v[G];
+  auto offset = [&](int g, int s) {
+    uint32_t off = p0[g];
 #pragma unroll
-  for (int g = 0; g < G; ++g) p0[g] = uint32_t(D.lo[grp[g] & 31u]) ^ uint32_t(D.hi[grp[g] >> 5]);
-  if (r == uint32_t(RB)) {  // full register tile (every pass with at least RB local qubits)
+    for (int j = 0; j < RB; ++j)
+      if (s & (1 << j)) off ^= rp[j];
+    return off;
+  };
+  auto re = [&](uint32_t off) -> R& { return *reinterpret_cast<R*>(sm + off); };
 #pragma unroll
-    for (int g = 0; g < G; ++g)
+  for (int g = 0; g < G; ++g)
+    p0[g] = (uint32_t(D.lo[grp[g] & 31u]) ^ uint32_t(D.hi[grp[g] >> 5])) * uint32_t(sizeof(R));
+  const bool full = r == uint32_t(RB);  // full register tile (every pass with at least RB local qubits)
 #pragma unroll
-      for (int s = 0; s < NV; ++s) {
-        uint32_t off = p0[g];
+  for (int g = 0; g < G; ++g) {
+    if (full) {
 #pragma unroll
-        for (int j = 0; j < RB; ++j)
-          if (s & (1 << j)) off ^= rp[j];
-        v[g].re(s) = xr[off];
-        v[g].im(s) = xi[off];
+      for (int s = 0; s < NV; s += 2) {
+        const uint32_t o0 = offset(g, s), o1 = offset(g, s + 1);
+        const R a0 = re(o0), b0 = re(o0 + im), a1 = re(o1), b1 = re(o1 + im);
+        if constexpr (sizeof(R) == 4) {
+          v[g].r[s >> 1] = pack2(a0, a1);
+          v[g].i[s >> 1] = pack2(b0, b1);
+        } else {
+          v[g].set(s, a0, b0);
+          v[g].set(s + 1, a1, b1);
+        }
       }
-  } else {
+    } else {
 #pragma unroll
-    for (int g = 0; g < G; ++g)
+      for (int s = 0; s < NV; s += 2) {
+        R a[2] = {R(0), R(0)}, b[2] = {R(0), R(0)};
 #pragma unroll
-      for (int s = 0; s < NV; ++s) {
-        if (uint32_t(s) >> r) continue;
-        uint32_t off = p0[g];
-#pragma unroll
-        for (int j = 0; j < RB; ++j)
-          if (s & (1 << j)) off ^= rp[j];
-        v[g].re(s) = xr[off];
-        v[g].im(s) = xi[off];
+        for (int e = 0; e < 2; ++e)
+          if (!(uint32_t(s + e) >> r)) {
+            a[e] = re(offset(g, s + e));
+            b[e] = re(offset(g, s + e) + im);
+          }
+        if constexpr (sizeof(R) == 4) {
+          v[g].r[s >> 1] = pack2(a[0], a[1]);
+          v[g].i[s >> 1] = pack2(b[0], b[1]);
+        } else {
+          v[g].set(s, a[0], b[0]);
+          v[g].set(s + 1, a[1], b[1]);
+        }
       }
+    }
   }
-  for (uint32_t kk = kbeg; kk < kend; ++kk) apply_instr<R, RB, G>(pprog[kk], v, pcoef, tile, tcoef, grp);
-  if (r == uint32_t(RB)) {
+  run_rounds<R, RB, G>(pprog, kbeg, kend, v, pcoef, ttab, tile, grp);
 #pragma unroll
-    for (int g = 0; g < G; ++g)
+  for (int g = 0; g < G; ++g)
 #pragma unroll
-      for (int s = 0; s < NV; ++s) {
-        uint32_t off = p0[g];
-#pragma unroll
-        for (int j = 0; j < RB; ++j)
-          if (s & (1 << j)) off ^= rp[j];
-        xr[off] = v[g].re(s);
-        xi[off] = v[g].im(s);
-      }
-  } else {
-#pragma unroll
-    for (int g = 0; g < G; ++g)
-#pragma unroll
-      for (int s = 0; s < NV; ++s) {
-        if (uint32_t(s) >> r) continue;
-        uint32_t off = p0[g];
-#pragma unroll
-        for (int j = 0; j < RB; ++j)
-          if (s & (1 << j)) off ^= rp[j];
-        xr[off] = v[g].re(s);
-        xi[off] = v[g].im(s);
-      }
-  }
+    for (int s = 0; s < NV; ++s) {
+      if (!full && (uint32_t(s) >> r)) continue;
+      const uint32_t off = offset(g, s);
+      re(off) = v[g].re(s);
+      re(off + im) = v[g].im(s);
+    }
 }
 
 // HI: entries of the address and swizzle tables (2^(lbits - 5) and 2^(lbits - W) at most); tile
-// sweeps take a smaller table, which leaves room for one more block per SM.
-template <class R, int RB, int W, int NT, int MINB = 1, int GP = 1, int HI = kMaxHi>
+// sweeps take a smaller table, which leaves room for one more block per SM. Their tiles' imaginary parts
+// lie at a constant distance (TILE), the largest tile's size.
+template <class R, int RB, int W, int NT, int MINB = 1, int GP = 1, int HI = kMaxHi, bool TILE = false>
 __global__ void __launch_bounds__(NT, MINB)
     k_batch(const Item* __restrict__ items, uint32_t nitems, const PassDev* __restrict__ passes,
             const PhaseDev* __restrict__ phases, const Instr* __restrict__ prog, const R* __restrict__ coef,
@@ -712,10 +770,12 @@ __global__ void __launch_bounds__(NT, MINB)
             long long* __restrict__ prof, uint32_t fixed, const long long* __restrict__ wait_budget) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   R* xr = reinterpret_cast<R*>(smem_raw);
-  R* xi = xr + (size_t(1) << lbits);  // every pass has nlocal <= lbits
-  uint8_t* stage = reinterpret_cast<uint8_t*>(xi + (size_t(1) << lbits));  // the pass's program
-  // per-tile phase coefficients (tile sweeps; sits right after the program staging area)
-  R* tcoef = reinterpret_cast<R*>(stage + (fixed ? kTileStageBytes : kStageBytes));
+  const uint32_t cap = TILE ? uint32_t(HI) << W : 1u << lbits;  // every pass has nlocal <= lbits
+  R* xi = xr + cap;
+  uint8_t* stage = reinterpret_cast<uint8_t*>(xi + cap);  // the pass's program
+  // per-tile phase sums (the factors of both sides) and slot tables (tile sweeps; after the staging area)
+  double* tphase = reinterpret_cast<double*>(stage + (TILE ? kTileStageBytes : kStageBytes));
+  R* ttab = reinterpret_cast<R*>(tphase + 4 * kTphSlots);
   __shared__ uint64_t s_gaddr[HI];
   __shared__ uint16_t s_swz[HI];
   __shared__ uint32_t s_item;
@@ -786,7 +846,7 @@ __global__ void __launch_bounds__(NT, MINB)
     // the pass's instructions, phases and coefficients into shared memory (kept while the next
     // item is a tile of the same pass), overlapped with the tile fill
     const uint32_t ph_bytes = P.prog_len * uint32_t(sizeof(Instr));
-    const uint32_t co_bytes = (ph_bytes + P.nphase * uint32_t(sizeof(PhaseDev)) + 7u) & ~7u;
+    const uint32_t co_bytes = (ph_bytes + P.nphase * uint32_t(sizeof(PhaseDev)) + 15u) & ~15u;  // (double2 reads)
     if (P.staged && staged_pass != item.pass &&
         QSVB_BC(co_bytes + P.ncoef * 2u * uint32_t(sizeof(R)) <= (fixed ? kTileStageBytes : kStageBytes), err)) {
       const uint32_t* src0 = reinterpret_cast<const uint32_t*>(prog + P.prog_off);
@@ -858,9 +918,9 @@ __global__ void __launch_bounds__(NT, MINB)
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    if (P.tph_n) {
-      // phase sums over the tile bits, one slot per operation: D1 blocks (the 0 and 1 sides of a
-      // register bit) or a single complex factor
+    if (TILE && P.tph_n) {
+      // phase sums over the tile bits: the factors of the 0 and 1 sides of a register bit, or one factor
+      // (type 2)
       const uint8_t* tb = reinterpret_cast<const uint8_t*>(&P) + P.tph_off;
       const uint32_t* offs = reinterpret_cast<const uint32_t*>(tb);
       const double* dd = reinterpret_cast<const double*>(tb + ((4 * P.tph_n + 7) & ~7u));
@@ -882,29 +942,36 @@ __global__ void __launch_bounds__(NT, MINB)
             z1r = r;
           }
         }
-        const double c0 = z0r, s0 = z0i, c1 = z1r, s1 = z1i;
-        R* o = tcoef + kTphSlotR * i;
-        if (type == 2) {
-          o[0] = R(c0);
-          o[1] = R(s0);
-        } else if constexpr (std::is_same<R, float>::value) {
-          const bool j0 = d[6 + 6 * m] != 0.0;  // register bit 0: lanes take the two sides
-          const float v[3][2] = {{float(c0), float(c1)}, {float(s0), float(s1)}, {float(-s0), float(-s1)}};
-          if (j0) {
-            for (int rep = 0; rep < 2; ++rep)
-              for (int e = 0; e < 3; ++e) {
-                o[6 * rep + 2 * e] = v[e][0];
-                o[6 * rep + 2 * e + 1] = v[e][1];
-              }
-          } else {
-            const float w[6] = {float(c0), float(s0), float(-s0), float(c1), float(s1), float(-s1)};
-            for (int e = 0; e < 6; ++e) o[2 * e] = o[2 * e + 1] = w[e];
-          }
+        tphase[4 * i] = z0r;
+        tphase[4 * i + 1] = z0i;
+        tphase[4 * i + 2] = z1r;
+        tphase[4 * i + 3] = z1i;
+      }
+      __syncthreads();
+      // the slot tables: constant factors times the sums on the register bits, in FP64, rounded once
+      const TileTab* tt = reinterpret_cast<const TileTab*>(reinterpret_cast<const uint8_t*>(&P) + P.ttab_off);
+      const double2* tbase = reinterpret_cast<const double2*>(reinterpret_cast<const uint8_t*>(&P) + P.ttab_base);
+      for (uint32_t i = tid; i < (P.ttab_n << RB); i += NT) {
+        const TileTab T1 = tt[i >> RB];
+        const uint32_t slot = i & ((1u << RB) - 1u);
+        double2 z = tbase[T1.base + slot];
+        auto times = [&](uint32_t op, uint32_t side) {
+          const double fr = tphase[4 * op + 2 * side], fi = tphase[4 * op + 2 * side + 1];
+          z = {z.x * fr - z.y * fi, z.x * fi + z.y * fr};
+        };
+#pragma unroll
+        for (int j = 0; j < RB; ++j)
+          if (T1.bit[j] != kTabNone) times(T1.bit[j], (slot >> j) & 1u);
+        if (T1.all != kTabNone) times(T1.all, 0);
+        R* o = ttab + (i >> RB) * tab_reals<R>(RB);
+        if constexpr (sizeof(R) == 4) {
+          o += 6 * (slot >> 1) + (slot & 1u);
+          o[0] = R(z.x);
+          o[2] = R(z.y);
+          o[4] = R(-z.y);
         } else {
-          o[0] = R(c0);
-          o[1] = R(s0);
-          o[2] = R(c1);
-          o[3] = R(s1);
+          o[2 * slot] = z.x;
+          o[2 * slot + 1] = z.y;
         }
       }
       __syncthreads();
@@ -919,12 +986,12 @@ __global__ void __launch_bounds__(NT, MINB)
       const uint32_t kbeg = k + 1, kend = kbeg + D.ninstr;
       uint32_t rp[RB];
 #pragma unroll
-      for (int j = 0; j < RB; ++j) rp[j] = D.rphys[j];
+      for (int j = 0; j < RB; ++j) rp[j] = D.rphys[j] * uint32_t(sizeof(R));
       // (checked builds) a group's offsets are XORs of these and of its two table entries, so each
       // below T keeps every offset in the tile
       bool rp_ok = true;
 #pragma unroll
-      for (int j = 0; j < RB; ++j) rp_ok = rp_ok && (uint32_t(j) >= D.r || QSVB_BC(rp[j] < T, err));  // bits in use
+      for (int j = 0; j < RB; ++j) rp_ok = rp_ok && (uint32_t(j) >= D.r || QSVB_BC(D.rphys[j] < T, err));  // bits in use
       auto grp_ok = [&](uint32_t gi) { return rp_ok && QSVB_BC((uint32_t(D.lo[gi & 31u]) ^ uint32_t(D.hi[gi >> 5])) < T, err); };
       // two groups at a time where the thread has two (independent updates interleave), then one
       const uint32_t ngrp = 1u << nt;
@@ -933,12 +1000,14 @@ __global__ void __launch_bounds__(NT, MINB)
         for (; grp + NT < ngrp; grp += 2 * NT) {
           const uint32_t gg[2] = {grp, grp + NT};
           if (grp_ok(gg[0]) && grp_ok(gg[1]))
-            phase_groups<R, RB, 2>(gg, D, rp, xr, xi, pprog, kbeg, kend, pcoef, item.tile, tcoef);
+            phase_groups<R, RB, 2>(gg, D, rp, reinterpret_cast<char*>(smem_raw), cap * uint32_t(sizeof(R)), pprog, kbeg, kend,
+                                   pcoef, item.tile, ttab);
         }
       }
       for (; grp < ngrp; grp += NT) {
         const uint32_t gg[1] = {grp};
-        if (grp_ok(gg[0])) phase_groups<R, RB, 1>(gg, D, rp, xr, xi, pprog, kbeg, kend, pcoef, item.tile, tcoef);
+        if (grp_ok(gg[0])) phase_groups<R, RB, 1>(gg, D, rp, reinterpret_cast<char*>(smem_raw), cap * uint32_t(sizeof(R)), pprog, kbeg, kend,
+                                 pcoef, item.tile, ttab);
       }
       k = kend;
       __syncthreads();
@@ -1024,7 +1093,7 @@ struct HostGate {
   std::vector<cd> a;
 };
 
-enum LKind : uint32_t {
+enum LKind : uint32_t {  // (D1P, DTP: a phase sum over the tile bits on one local qubit, on all amplitudes)
   LK_1Q = OP_1Q, LK_D1 = OP_D1, LK_CX = OP_CX, LK_2Q = OP_2Q, LK_D2 = OP_D2, LK_D1T = OP_D1T, LK_DT = OP_DT,
   LK_D1P = OP_D1P, LK_DTP = OP_DTP
 };
@@ -1035,7 +1104,12 @@ struct TphOp {
   int type = 1;
   double c0 = 0, c1 = 0;
   std::vector<std::array<double, 3>> terms;  // type 1: (bit, d0, d1); type 2: (bit k, bit l, angle)
-  bool j0 = false;                           // type 1: lives on register bit 0 of its phase
+  // type 1: the 0 side is 1 for every tile
+  bool half() const {
+    for (const auto& t : terms)
+      if (t[1] != 0.0) return false;
+    return type == 1 && c0 == 0.0;
+  }
 };
 
 struct LGate {  // a gate on local positions
@@ -1119,6 +1193,9 @@ struct BatchPlan {
   std::vector<PhaseDev> phases;
   std::vector<Instr> prog;
   std::vector<double> coef;  // complex entries as (re, im) pairs in FP64
+  std::vector<TileTab> ttabs;   // tile sweeps: slot tables computed per tile, and
+  std::vector<cd> ttab_base;    // their constant factors
+  double work = 0;              // tile sweeps: arithmetic per amplitude (see tile_prepare)
   std::vector<Item> items;
   std::vector<uint64_t> prob_off, zoff;
   std::vector<uint32_t> zcnt, nq;
@@ -1391,7 +1468,7 @@ void emit_phases(BatchPlan& bp, const std::vector<LGate>& G, uint32_t nlocal, st
       }
     }
     auto emit_table = [&](const std::vector<cd>& t) {
-      const size_t base = bp.coef.size() / 2;
+      bp.prog.push_back(Instr{OP_TAB, 0, 0, uint32_t(bp.coef.size() / 2 - coef_base)});
       if (bp.dtype == QSVB_C64) {
         for (uint32_t h = 0; h < nslot / 2; ++h) {
           const cd a0 = t[2 * h], a1 = t[2 * h + 1];
@@ -1402,16 +1479,35 @@ void emit_phases(BatchPlan& bp, const std::vector<LGate>& G, uint32_t nlocal, st
       } else {
         for (uint32_t s2 = 0; s2 < nslot; ++s2) push_coef(bp, t[s2]);
       }
-      bp.prog.push_back(Instr{OP_DTAB, 0, 0, uint32_t(base - coef_base)});
     };
     auto emit_group = [&](const Op& op) {
-      uint32_t mask = 0;
-      const uint32_t base = uint32_t(bp.coef.size() / 2 - coef_base);
-      for (const GFac& f : gfs[size_t(op.gidx)]) {
-        mask |= 1u << f.gbit;
-        for (int e = 0; e < 4; ++e) push_coef(bp, f.d[e]);
+      const std::vector<GFac>& fs = gfs[size_t(op.gidx)];
+      bool half = true;
+      for (const GFac& f : fs) half = half && f.d[0] == cd(1, 0) && f.d[2] == cd(1, 0);
+      // one table over the window of all the group bits, or two over a split of them: the fewest entries
+      std::vector<uint32_t> gb;
+      for (const GFac& f : fs) gb.push_back(f.gbit);  // ascending
+      uint32_t cut = uint32_t(gb.size()), best = 1u << (gb.back() - gb.front() + 1);
+      for (uint32_t k = 1; k < gb.size(); ++k) {
+        const uint32_t n2 = (1u << (gb[k - 1] - gb[0] + 1)) + (1u << (gb.back() - gb[k] + 1));
+        if (n2 + 4 < best) best = n2, cut = k;  // (the second table costs a complex product)
       }
-      bp.prog.push_back(Instr{OP_D1G, op.rbit, mask, base});
+      Instr in{half ? uint32_t(OP_D1GH) : uint32_t(OP_D1G), op.rbit, 0, uint32_t(bp.coef.size() / 2 - coef_base)};
+      auto table = [&](uint32_t k0, uint32_t k1, uint32_t shift) {
+        if (k0 == k1) return;
+        const uint32_t b0 = gb[k0], w = gb[k1 - 1] - b0 + 1;
+        in.b |= (b0 | (w << 4)) << shift;
+        for (uint32_t x = 0; x < (1u << w); ++x) {
+          cd z[2] = {1.0, 1.0};
+          for (uint32_t k = k0; k < k1; ++k)
+            for (uint32_t side = 0; side < 2; ++side) z[side] *= fs[k].d[side | (((x >> (gb[k] - b0)) & 1u) << 1)];
+          if (!half) push_coef(bp, z[0]);
+          push_coef(bp, z[1]);
+        }
+      };
+      table(0, cut, 0);
+      table(cut, uint32_t(gb.size()), 8);
+      bp.prog.push_back(in);
     };
     auto emit_split = [&](const Op& op) {
       Instr in{op.form == 2 ? uint32_t(OP_1QX) : uint32_t(OP_1QR), op.rbit, 0,
@@ -1444,27 +1540,6 @@ void emit_phases(BatchPlan& bp, const std::vector<LGate>& G, uint32_t nlocal, st
               for (int k = 0; k < 4; ++k) push_coef(bp, a[size_t(k)]);
             }
             break;
-          case LK_D1:
-            if (bp.dtype == QSVB_C64) {
-              const cd p0 = a[0], p1 = a[3];
-              if (in.a == 0) {  // lanes of a float2 pair are the two sides of the gate's bit
-                for (int rep = 0; rep < 2; ++rep) {
-                  push_coef(bp, cd(p0.real(), p1.real()));
-                  push_coef(bp, cd(p0.imag(), p1.imag()));
-                  push_coef(bp, cd(-p0.imag(), -p1.imag()));
-                }
-              } else {
-                for (const cd& e : {p0, p1}) {
-                  push_coef(bp, cd(e.real(), e.real()));
-                  push_coef(bp, cd(e.imag(), e.imag()));
-                  push_coef(bp, cd(-e.imag(), -e.imag()));
-                }
-              }
-            } else {
-              push_coef(bp, a[0]);
-              push_coef(bp, a[3]);
-            }
-            break;
           case LK_CX:
             in.b = uint32_t(regbit[g.p[1]]);
             break;
@@ -1494,14 +1569,6 @@ void emit_phases(BatchPlan& bp, const std::vector<LGate>& G, uint32_t nlocal, st
             }
             break;
           }
-          case LK_D1P:
-            in.coef = g.t[0];
-            (*tph)[g.t[0]].j0 = in.a == 0;
-            break;
-          case LK_DTP:
-            in.a = 0;
-            in.coef = g.t[0];
-            break;
           case LK_DT: {
             in.a = 0;
             in.b = g.t[0] | (g.t[1] << 8) | (g.nt << 16);
@@ -1509,18 +1576,14 @@ void emit_phases(BatchPlan& bp, const std::vector<LGate>& G, uint32_t nlocal, st
             for (size_t e = 0; e < d; ++e) push_coef(bp, a[e * d + e]);
             break;
           }
-          default: {  // LK_2Q / LK_D2: the kernel wants matrix bit 0 on the lower register bit
+          default: {  // LK_2Q: the kernel wants matrix bit 0 on the lower register bit
             const uint32_t ra = uint32_t(regbit[g.p[0]]), rbit = uint32_t(regbit[g.p[1]]);
             const bool swap = ra > rbit;
             in.a = std::min(ra, rbit);
             in.b = std::max(ra, rbit);
             auto perm = [&](int s) { return swap ? (((s & 1) << 1) | ((s >> 1) & 1)) : s; };
-            if (g.kind == LK_2Q) {
-              for (int r = 0; r < 4; ++r)
-                for (int c = 0; c < 4; ++c) push_coef(bp, a[size_t(perm(r) * 4 + perm(c))]);
-            } else {
-              for (int r = 0; r < 4; ++r) push_coef(bp, a[size_t(perm(r) * 4 + perm(r))]);
-            }
+            for (int r = 0; r < 4; ++r)
+              for (int c = 0; c < 4; ++c) push_coef(bp, a[size_t(perm(r) * 4 + perm(c))]);
             break;
           }
         }
@@ -1531,12 +1594,131 @@ void emit_phases(BatchPlan& bp, const std::vector<LGate>& G, uint32_t nlocal, st
         if (z != cd(1, 0)) return false;
       return true;
     };
+    // The rounds. Diagonals gather (they commute) until a gate needs its place: the next free register bit
+    // of the round, or a new round. A gate on register bit b takes its round's place b, the diagonals in
+    // front of it with it.
+    struct Diag {
+      std::vector<cd> t;                                  // constant factors (empty: all 1)
+      std::vector<const LGate*> sums;                     // phase sums over the tile bits
+      const Op* g[8] = {nullptr};                         // group-dependent diagonals by register bit
+      bool any = false;
+    };
+    struct Round {
+      Diag d[kRoundBits];
+      const Op* u[kRoundBits] = {nullptr};
+      uint32_t cx = 0;
+      const LGate* other = nullptr;
+    };
+    std::vector<Round> rounds(1);
+    Diag pend;
+    uint32_t place = 0;       // first register bit still free in the last round
+    uint32_t cx_place = 0;    // the same of its CX gates (place is RB once there is one)
+    auto new_round = [&] {
+      rounds.emplace_back();
+      place = cx_place = 0;
+    };
+    auto settle = [&](uint32_t at) {  // the gathered diagonals in front of place `at` of the last round
+      if (pend.any) rounds.back().d[at] = std::move(pend);
+      pend = Diag{};
+    };
+    auto close_diag = [&] {  // ... in front of whatever comes next
+      if (!pend.any) return;
+      if (place >= bp.rb) new_round();
+      settle(place);
+      ++place;  // (no gate there)
+    };
     for (size_t j = 0; j <= ops.size(); ++j) {
-      if (!tables[j].empty() && !identity(tables[j])) emit_table(tables[j]);
+      if (!tables[j].empty() && !identity(tables[j])) {
+        bp.work += 6.0;
+        if (pend.t.empty()) pend.t.assign(nslot, cd(1, 0));
+        for (uint32_t s2 = 0; s2 < nslot; ++s2) pend.t[s2] *= tables[j][s2];
+        pend.any = true;
+      }
       if (j == ops.size()) break;
-      if (ops[j].g) emit_one(*ops[j].g);
-      else if (ops[j].form == 3) emit_group(ops[j]);
-      else emit_split(ops[j]);
+      const Op& op = ops[j];
+      if (op.form == 3) {
+        bp.work += 6.0;
+        if (pend.g[op.rbit]) close_diag();
+        pend.g[op.rbit] = &op;
+        pend.any = true;
+      } else if (op.g && (op.g->kind == LK_D1P || op.g->kind == LK_DTP)) {
+        bp.work += 6.0;
+        pend.sums.push_back(op.g);
+        pend.any = true;
+      } else if (op.form == 1 || op.form == 2 || op.g->kind == LK_1Q) {
+        bp.work += op.form ? 8.0 : 16.0;
+        const uint32_t b = op.form ? op.rbit : uint32_t(regbit[op.g->p[0]]);
+        if (b < place) new_round();
+        settle(b);
+        rounds.back().u[b] = &op;
+        place = b + 1;
+      } else if (op.g->kind == LK_CX && regbit[op.g->p[1]] == regbit[op.g->p[0]] + 1) {
+        const uint32_t b = uint32_t(regbit[op.g->p[0]]);
+        close_diag();
+        if (b < cx_place) new_round();
+        rounds.back().cx |= 1u << b;
+        cx_place = b + 1;
+        place = bp.rb;
+      } else {
+        bp.work += op.g->kind == LK_2Q ? 32.0 : op.g->kind == LK_CX ? 0.0 : 6.0;
+        close_diag();
+        new_round();
+        rounds.back().other = op.g;
+        new_round();
+      }
+    }
+    close_diag();
+    for (const Round& r : rounds) {
+      const size_t at = bp.prog.size();
+      Instr hd{OP_ROUND, r.cx << kRoundCx, 0, 0};
+      bp.prog.push_back(hd);
+      if (r.other) {
+        hd.a = 1u << kRoundOther;
+        emit_one(*r.other);
+        bp.prog[at] = hd;
+        continue;
+      }
+      bool any = r.cx != 0;
+      for (uint32_t j = 0; j < bp.rb; ++j) {
+        const Diag& d = r.d[j];
+        if (!d.t.empty() || !d.sums.empty()) {
+          // factors other than 1 only where register bit j - 1 is 1 (complex64 keeps bit 0 inside its pairs)
+          bool half = j >= (bp.dtype == QSVB_C64 ? 2u : 1u);
+          for (uint32_t s2 = 0; s2 < nslot && half && !d.t.empty(); ++s2)
+            half = ((s2 >> (j - 1)) & 1u) || d.t[s2] == cd(1, 0);
+          for (const LGate* g : d.sums)
+            half = half && g->kind == LK_D1P && uint32_t(regbit[g->p[0]]) == j - 1 && (*tph)[g->t[0]].half();
+          hd.a |= (half ? 2u : 1u) << (kRoundTab + 2 * j);
+          if (d.sums.empty()) {
+            emit_table(d.t);
+          } else {
+            TileTab tt{uint32_t(bp.ttab_base.size()), {kTabNone, kTabNone, kTabNone, kTabNone, kTabNone}, kTabNone};
+            for (uint32_t s2 = 0; s2 < nslot; ++s2) bp.ttab_base.push_back(d.t.empty() ? cd(1, 0) : d.t[s2]);
+            for (const LGate* g : d.sums) {
+              uint8_t& e = g->kind == LK_DTP ? tt.all : tt.bit[regbit[g->p[0]]];
+              QSVB_REQUIRE(e == kTabNone, "two phase sums on one register bit of a diagonal");
+              e = uint8_t(g->t[0]);
+            }
+            bp.prog.push_back(Instr{OP_TAB, 1, 0, uint32_t(bp.ttabs.size())});
+            bp.ttabs.push_back(tt);
+          }
+          any = true;
+        }
+        for (uint32_t b = 0; b < bp.rb; ++b)
+          if (d.g[b]) {
+            hd.b |= 1u << (5 * j + b);
+            emit_group(*d.g[b]);
+            any = true;
+          }
+        if (const Op* u = r.u[j]) {
+          hd.a |= (u->form ? uint32_t(u->form) : 3u) << (2 * j);
+          if (u->form) emit_split(*u);
+          else emit_one(*u->g);
+          any = true;
+        }
+      }
+      if (any) bp.prog[at] = hd;
+      else bp.prog.pop_back();
     }
     bp.phases[phase_idx].ninstr = uint32_t(bp.prog.size() - phase_pc - 1);
   }
@@ -1648,7 +1830,7 @@ void plan_batch_part(BatchPart& part, const qsvb_circuit* circuits, size_t ncirc
       P.ncoef = uint32_t(bp->coef.size() / 2) - P.coef_off;
       {
         const size_t rsz = dtype == QSVB_C128 ? 8 : 4;
-        const size_t co = (P.prog_len * sizeof(Instr) + P.nphase * sizeof(PhaseDev) + 7) & ~size_t(7);
+        const size_t co = (P.prog_len * sizeof(Instr) + P.nphase * sizeof(PhaseDev) + 15) & ~size_t(15);
         P.staged = co + size_t(P.ncoef) * 2 * rsz <= kStageBytes ? 1u : 0u;
       }
       P.first = circuit_passes[ci].empty() ? 1u : 0u;
@@ -2057,21 +2239,25 @@ uint32_t tile_local_bits(int dtype, uint32_t n) {
 namespace {
 uint32_t tile_reg_bits(int dtype) { return dtype == QSVB_C128 ? 3u : 4u; }
 size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
-constexpr size_t kTileSmemMax = (size_t(2) * 4 << 12) + kTileStageBytes + kTphSlots * kTphSlotR * 8;
+// a 32 KB tile, the program, the phase sums and the slot tables they make
+template <class R> constexpr size_t tile_smem(uint32_t rb) {
+  return (size_t(32) << 10) + kTileStageBytes + kTphSlots * (4 * sizeof(double) + tab_reals<R>(rb) * sizeof(R));
+}
 
 template <class R, int RB, int NT, int MINB, int GP>
 void launch_tile_variant(const LaunchEnv& e, R* re, R* im, const Sweep& s, const uint8_t* base) {
   constexpr int W = sizeof(R) == 8 ? 4 : 5;
-  auto fn = k_batch<R, RB, W, NT, MINB, GP, kTileHi>;
+  auto fn = k_batch<R, RB, W, NT, MINB, GP, kTileHi, true>;
   QSVB_REQUIRE(s.tile_lbits <= 12 && (1u << (s.tile_lbits - uint32_t(W))) <= uint32_t(kTileHi),
                "tile sweep wider than its address tables");
   static std::once_flag once;
   std::call_once(once, [&] {
-    QSVB_CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTileSmemMax)));
+    QSVB_CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tile_smem<R>(RB))));
     QSVB_CK(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  int(cudaSharedmemCarveoutMaxShared)));
   });
-  const size_t smem = ((size_t(2) * sizeof(R)) << s.tile_lbits) + kTileStageBytes + kTphSlots * kTphSlotR * sizeof(R);
+  static_assert(2 * sizeof(R) * (size_t(kTileHi) << W) == size_t(32) << 10, "tile size");
+  const size_t smem = tile_smem<R>(RB);
   int occ = 0;
   QSVB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, NT, smem));
   QSVB_REQUIRE(occ >= 1, "tile kernel does not fit on an SM");
@@ -2243,29 +2429,18 @@ void tile_prepare(Sweep& s, uint32_t n, int dtype) {
     G.swap(out);
   }
   emit_phases(bp, G, P.nlocal, &tph);
-  // arithmetic per amplitude of the emitted program, in FP32/FP64 operations: general 1-qubit gates
-  // 16, split-form ones 8, 2-qubit dense 32, diagonal kinds 6 (one complex multiply), and each
-  // register phase kTilePhaseWork for its shared-memory round trip
+  // arithmetic per amplitude of the pass, in FP32/FP64 operations: general 1-qubit gates 16, split-form
+  // ones 8, 2-qubit dense 32, each kind of diagonal at each of its points 6 (one complex multiply), and
+  // each register phase kTilePhaseWork for its shared-memory round trip
   constexpr double kTilePhaseWork = 8.0;
-  double work = 0;
-  for (const Instr& in : bp.prog) {
-    switch (in.op) {
-      case OP_PHASE: work += kTilePhaseWork; break;
-      case OP_1Q: work += 16.0; break;
-      case OP_1QR:
-      case OP_1QX: work += 8.0; break;
-      case OP_2Q: work += 32.0; break;
-      case OP_CX: break;
-      default: work += 6.0; break;
-    }
-  }
+  const double work = bp.work + kTilePhaseWork * double(bp.phases.size());
   flops = dim * work;
   P.prog_len = uint32_t(bp.prog.size());
   P.nphase = uint32_t(bp.phases.size());
   P.ncoef = uint32_t(bp.coef.size() / 2);
   const size_t rsz = dtype == QSVB_C128 ? 8 : 4;
   {
-    const size_t co = (P.prog_len * sizeof(Instr) + P.nphase * sizeof(PhaseDev) + 7) & ~size_t(7);
+    const size_t co = (P.prog_len * sizeof(Instr) + P.nphase * sizeof(PhaseDev) + 15) & ~size_t(15);
     P.staged = co + size_t(P.ncoef) * 2 * rsz <= kTileStageBytes ? 1u : 0u;
   }
   const size_t off_phase = align16(sizeof(PassDev));
@@ -2295,17 +2470,25 @@ void tile_prepare(Sweep& s, uint32_t n, int dtype) {
       tdat.push_back(std::cos(a1));
       tdat.push_back(std::sin(a1));
     }
-    tdat.push_back(op.j0 ? 1.0 : 0.0);
   }
   const size_t tph_bytes = tph.empty() ? 0 : ((4 * toffs.size() + 7) & ~size_t(7)) + 8 * tdat.size();
   P.tph_n = uint32_t(tph.size());
   P.tph_off = uint32_t(off_tph);
-  const size_t total = off_tph + tph_bytes;
+  const size_t off_ttab = align16(off_tph + tph_bytes), off_tbase = align16(off_ttab + bp.ttabs.size() * sizeof(TileTab));
+  P.ttab_n = uint32_t(bp.ttabs.size());
+  P.ttab_off = uint32_t(off_ttab);
+  P.ttab_base = uint32_t(off_tbase);
+  QSVB_REQUIRE(P.ttab_n <= kTphSlots, "too many slot tables in a tile pass");
+  const size_t total = off_tbase + bp.ttab_base.size() * sizeof(cd);
   s.tile_blob.assign(total, 0);
   std::memcpy(s.tile_blob.data(), &P, sizeof(P));
   if (!tph.empty()) {
     std::memcpy(s.tile_blob.data() + off_tph, toffs.data(), 4 * toffs.size());
     std::memcpy(s.tile_blob.data() + off_tph + ((4 * toffs.size() + 7) & ~size_t(7)), tdat.data(), 8 * tdat.size());
+  }
+  if (!bp.ttabs.empty()) {
+    std::memcpy(s.tile_blob.data() + off_ttab, bp.ttabs.data(), bp.ttabs.size() * sizeof(TileTab));
+    std::memcpy(s.tile_blob.data() + off_tbase, bp.ttab_base.data(), bp.ttab_base.size() * sizeof(cd));
   }
   if (!bp.phases.empty()) std::memcpy(s.tile_blob.data() + off_phase, bp.phases.data(), bp.phases.size() * sizeof(PhaseDev));
   if (!bp.prog.empty()) std::memcpy(s.tile_blob.data() + off_prog, bp.prog.data(), bp.prog.size() * sizeof(Instr));
