@@ -63,16 +63,27 @@ void check_ctx(const qsvb_ctx* c) { QSVB_REQUIRE(c != nullptr, "null context"); 
 
 // Synchronize the context stream and surface a device-side bounded-wait timeout (the flag is
 // cleared so the context stays usable).
-void sync_and_check(qsvb_ctx* c) {
-  QSVB_CK(cudaStreamSynchronize(c->stream));
-  int flag = 0;
-  QSVB_CK(cudaMemcpy(&flag, c->d_err, sizeof(int), cudaMemcpyDeviceToHost));
+void check_flag(qsvb_ctx* c, int flag) {
   if (flag) {
     QSVB_CK(cudaMemset(c->d_err, 0, sizeof(int)));
     if (flag & kErrBounds)
       throw Error(QSVB_E_CUDA, "a device bounds check failed (an index out of its buffer); results are invalid");
     throw Error(QSVB_E_TIMEOUT, "a device-side wait ran out of its iteration budget; results are invalid");
   }
+}
+void sync_and_check(qsvb_ctx* c) {
+  QSVB_CK(cudaStreamSynchronize(c->stream));
+  int flag = 0;
+  QSVB_CK(cudaMemcpy(&flag, c->d_err, sizeof(int), cudaMemcpyDeviceToHost));
+  check_flag(c, flag);
+}
+// The results of a reduction queued into c->h_result; the flag came with them.
+void wait_result(qsvb_ctx* c, double h[2]) {
+  QSVB_CK(cudaStreamSynchronize(c->stream));
+  const volatile double* r = c->h_result;
+  h[0] = r[0];
+  h[1] = r[1];
+  check_flag(c, int(r[2]));
 }
 void check_state(const qsvb_ctx* c, const qsvb_state* s) {
   check_ctx(c);
@@ -227,11 +238,10 @@ double reduce(qsvb_ctx* c, int op, const qsvb_state* a, const qsvb_state* b, uin
     using R = decltype(r);
     launch_reduce<R>(c->env(), op, static_cast<const R*>(a->re), static_cast<const R*>(a->im),
                      b ? static_cast<const R*>(b->re) : nullptr, b ? static_cast<const R*>(b->im) : nullptr,
-                     a->n_qubits, mask, c->d_partials, c->d_result);
+                     a->n_qubits, mask, c->d_partials, c->h_result);
   });
   double h[2];
-  QSVB_CK(cudaMemcpyAsync(h, c->d_result, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
-  sync_and_check(c);
+  wait_result(c, h);
   if (second) *second = h[1];
   return h[0];
 }
@@ -263,7 +273,9 @@ int qsvb_create(int device_ordinal, qsvb_ctx** out) {
     c->num_sms = prop.multiProcessorCount;
     QSVB_CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     QSVB_CK(cudaMalloc(&c->d_partials, reduce_partials_needed(c->num_sms) * sizeof(double)));
-    QSVB_CK(cudaMalloc(&c->d_result, 2 * sizeof(double)));
+    QSVB_CK(cudaMemset(c->d_partials, 0, reduce_partials_needed(c->num_sms) * sizeof(double)));
+    QSVB_CK(cudaMalloc(&c->d_result, 3 * sizeof(double)));
+    QSVB_CK(cudaHostAlloc(reinterpret_cast<void**>(&c->h_result), 3 * sizeof(double), cudaHostAllocMapped));
     QSVB_CK(cudaMalloc(&c->d_err, sizeof(int)));
     QSVB_CK(cudaMemset(c->d_err, 0, sizeof(int)));
     *out = c.release();
@@ -277,6 +289,7 @@ int qsvb_destroy(qsvb_ctx* c) {
     cudaStreamSynchronize(c->stream);
     if (c->d_partials) cudaFree(c->d_partials);
     if (c->d_result) cudaFree(c->d_result);
+    if (c->h_result) cudaFreeHost(c->h_result);
     if (c->d_mat_ring) cudaFree(c->d_mat_ring);
     if (c->d_exec_mats) cudaFree(c->d_exec_mats);
     if (c->d_prob) cudaFree(c->d_prob);
@@ -747,13 +760,12 @@ int qsvb_inner_product(qsvb_ctx* c, const qsvb_state* a, const qsvb_state* b, do
     if (a->dtype == QSVB_C64)
       launch_inner_mixed<float, double>(c->env(), static_cast<const float*>(a->re), static_cast<const float*>(a->im),
                                         static_cast<const double*>(b->re), static_cast<const double*>(b->im),
-                                        a->n_qubits, c->d_partials, c->d_result);
+                                        a->n_qubits, c->d_partials, c->h_result);
     else
       launch_inner_mixed<double, float>(c->env(), static_cast<const double*>(a->re), static_cast<const double*>(a->im),
                                         static_cast<const float*>(b->re), static_cast<const float*>(b->im),
-                                        a->n_qubits, c->d_partials, c->d_result);
-    QSVB_CK(cudaMemcpyAsync(out, c->d_result, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    sync_and_check(c);  // also reports a failure flagged by earlier device work
+                                        a->n_qubits, c->d_partials, c->h_result);
+    wait_result(c, out);  // also reports a failure flagged by earlier device work
   });
 }
 

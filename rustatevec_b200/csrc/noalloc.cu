@@ -121,6 +121,9 @@ extern "C" int qsvb_expectation_z_noalloc(const void* d_re, const void* d_im, ui
     double* scratch = scratch_for(dev);
     double* result = scratch + 2 * kNoAllocMaxCtas;
     const LaunchEnv env{static_cast<cudaStream_t>(stream), sms, nullptr};
+    // the counter of finished CTAs starts from zero even if an earlier call broke the rule against
+    // overlapping calls and left it elsewhere
+    QSVB_CK(cudaMemsetAsync(scratch + reduce_partials_needed(sms) - 1, 0, sizeof(double), env.stream));
     if (dtype == QSVB_C128)
       launch_reduce<double>(env, RED_EXPZ, static_cast<const double*>(d_re), static_cast<const double*>(d_im),
                             nullptr, nullptr, n_qubits, mask, scratch, result);

@@ -206,8 +206,8 @@ void launch_sweep(const LaunchEnv& e, R* re, R* im, uint32_t n, const Sweep& s, 
 size_t sweep_matrix_bytes(const Sweep& s, int dtype);
 void pack_sweep_matrix(const Sweep& s, int dtype, void* host_dst);
 
-// Reductions (FP64). `partials` holds >= reduce_partials_needed() doubles; results land in
-// d_out (2 doubles).
+// Reductions (FP64). `partials` holds >= reduce_partials_needed() doubles, zeroed once; results land in
+// d_out: 2 doubles, then the error flag's value when the environment has one.
 size_t reduce_partials_needed(int num_sms);
 template <class R>
 void launch_reduce(const LaunchEnv& e, int op, const R* re, const R* im, const R* re2, const R* im2,
@@ -261,7 +261,8 @@ struct qsvb_ctx {
   int num_sms = 148;
   cudaStream_t stream = nullptr;
   double* d_partials = nullptr;   // reduction partials
-  double* d_result = nullptr;     // 2 doubles
+  double* d_result = nullptr;     // 3 doubles (results that stay on the device)
+  double* h_result = nullptr;     // the same in pinned host memory (results the host waits for)
   char* d_mat_ring = nullptr;     // per-apply matrix uploads
   size_t mat_ring_cap = 0;
   size_t mat_ring_pos = 0;
