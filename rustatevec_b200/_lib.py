@@ -164,36 +164,42 @@ def check(rc: int):
         raise QsvbError(rc, lib().qsvb_last_error().decode(errors="replace"))
 
 
+_GATE_DT = np.dtype({"names": ["n", "q", "mat"], "formats": ["<u4", ("<u4", MAX_GATE_QUBITS), "<u8"],
+                     "offsets": [0, 4, 32], "itemsize": 40})
+_CIRC_DT = np.dtype({"names": ["n", "ngates", "gates"], "formats": ["<u4", "<u8", "<u8"],
+                     "offsets": [0, 8, 16], "itemsize": 24})
+
+
+def _pack_gates(arity, qubits, mats):
+    """The ``qsvb_gate`` array of flattened ops (numpy-built, no per-gate ctypes work); it points into
+    ``mats``, which the caller keeps alive."""
+    n = len(arity)
+    gates = np.zeros(max(n, 1), dtype=_GATE_DT)
+    a64 = arity.astype(np.int64)
+    gates["n"][:n] = arity
+    qoff = np.concatenate([[0], np.cumsum(a64)])
+    for j in range(int(a64.max()) if n else 0):
+        sel = a64 > j
+        gates["q"][:n][sel, j] = qubits[qoff[:-1][sel] + j]
+    moff = np.concatenate([[0], np.cumsum(2 * (1 << (2 * a64)))])[:-1]
+    gates["mat"][:n] = mats.ctypes.data + 8 * moff
+    return gates
+
+
 class PackedCircuit:
     """A circuit packed into the C structs; keeps the matrix buffer alive."""
 
     def __init__(self, circuit):
         arity, qubits, mats = circuit.flatten()
         self.mats = np.ascontiguousarray(mats, dtype=np.float64)
-        n = len(arity)
-        self.gates = (Gate * max(n, 1))()
-        base = self.mats.ctypes.data
-        qo = mo = 0
-        for i, m in enumerate(arity.tolist()):
-            g = self.gates[i]
-            g.n_qubits = m
-            for j in range(m):
-                g.qubits[j] = int(qubits[qo + j])
-            g.matrix = C.cast(base + 8 * mo, _dp)
-            qo += m
-            mo += 2 * (1 << (2 * m))
-        self.struct = CircuitS(circuit.n_qubits(), n, C.cast(self.gates, C.POINTER(Gate)))
+        gates = _pack_gates(arity, qubits, self.mats)
+        self.gates = (Gate * len(gates)).from_buffer(gates)
+        self.struct = CircuitS(circuit.n_qubits(), len(arity), C.cast(self.gates, C.POINTER(Gate)))
 
     def ref(self):
         """By-reference argument for the C calls. The struct points into this object's gate array
         and matrix buffer: keep the PackedCircuit alive until the call returns."""
         return C.byref(self.struct)
-
-
-_GATE_DT = np.dtype({"names": ["n", "q", "mat"], "formats": ["<u4", ("<u4", MAX_GATE_QUBITS), "<u8"],
-                     "offsets": [0, 4, 32], "itemsize": 40})
-_CIRC_DT = np.dtype({"names": ["n", "ngates", "gates"], "formats": ["<u4", "<u8", "<u8"],
-                     "offsets": [0, 8, 16], "itemsize": 24})
 
 
 class PackedBatch:
@@ -207,16 +213,7 @@ class PackedBatch:
         counts = np.array([len(c) for c in circuits], dtype=np.int64)
         arity, allq, mats = flatten_ops(list(chain.from_iterable(c.ops() for c in circuits)))
         self.mats = mats if len(mats) else np.zeros(1)
-        ng = len(arity)
-        self.gates = np.zeros(max(ng, 1), dtype=_GATE_DT)
-        self.gates["n"][:ng] = arity
-        a64 = arity.astype(np.int64)
-        qoff = np.concatenate([[0], np.cumsum(a64)])
-        for j in range(int(a64.max()) if ng else 0):
-            sel = a64 > j
-            self.gates["q"][:ng][sel, j] = allq[qoff[:-1][sel] + j]
-        moff = np.concatenate([[0], np.cumsum(2 * (1 << (2 * a64)))])[:-1]
-        self.gates["mat"][:ng] = self.mats.ctypes.data + 8 * moff
+        self.gates = _pack_gates(arity, allq, self.mats)
         nc = len(circuits)
         goff = np.concatenate([[0], np.cumsum(counts)])[:-1]
         self.circs = np.zeros(max(nc, 1), dtype=_CIRC_DT)

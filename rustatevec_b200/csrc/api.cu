@@ -72,10 +72,10 @@ void check_flag(qsvb_ctx* c, int flag) {
   }
 }
 void sync_and_check(qsvb_ctx* c) {
+  int* flag = reinterpret_cast<int*>(c->h_result + 3);
+  QSVB_CK(cudaMemcpyAsync(flag, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   QSVB_CK(cudaStreamSynchronize(c->stream));
-  int flag = 0;
-  QSVB_CK(cudaMemcpy(&flag, c->d_err, sizeof(int), cudaMemcpyDeviceToHost));
-  check_flag(c, flag);
+  check_flag(c, *flag);
 }
 // The results of a reduction queued into c->h_result; the flag came with them.
 void wait_result(qsvb_ctx* c, double h[2]) {
@@ -89,6 +89,31 @@ void check_state(const qsvb_ctx* c, const qsvb_state* s) {
   check_ctx(c);
   QSVB_REQUIRE(s != nullptr, "null state");
   QSVB_REQUIRE(s->device == c->device, "state belongs to another device");
+}
+
+// A component buffer of exactly `bytes` from the context's spare ones (nullptr: none).
+void* take_spare(qsvb_ctx* c, size_t bytes) {
+  for (size_t i = c->spare.size(); i-- > 0;)
+    if (c->spare[i].first == bytes) {
+      void* p = c->spare[i].second;
+      c->spare.erase(c->spare.begin() + ptrdiff_t(i));
+      c->spare_bytes -= bytes;
+      return p;
+    }
+  return nullptr;
+}
+void give_spare(qsvb_ctx* c, void* p, size_t bytes) {
+  if (c->spare_bytes + bytes > kStateKeep) {
+    cudaFree(p);
+    return;
+  }
+  c->spare.emplace_back(bytes, p);
+  c->spare_bytes += bytes;
+}
+void drop_spares(qsvb_ctx* c) {
+  for (auto& s : c->spare) cudaFree(s.second);
+  c->spare.clear();
+  c->spare_bytes = 0;
 }
 
 size_t state_bytes(const qsvb_state* s) { return (s->dtype == QSVB_C128 ? 8u : 4u) * (size_t(1) << s->n_qubits); }
@@ -176,9 +201,9 @@ qsvb_plan* build_plan(qsvb_ctx* c, const qsvb_circuit* circ, int dtype, const qs
       }
       p->d_mats = c->d_exec_mats;
       p->owns_mats = false;
-      // stream-ordered after every earlier use of the block on this context's stream
+      // stream-ordered after every earlier use of the block on this context's stream; `host` is pageable,
+      // so the call returns once its contents are staged
       QSVB_CK(cudaMemcpyAsync(p->d_mats, host.data(), total, cudaMemcpyHostToDevice, c->stream));
-      QSVB_CK(cudaStreamSynchronize(c->stream));  // `host` is pageable and about to go away
     } else {
       QSVB_CK(cudaMalloc(&p->d_mats, total));
       QSVB_CK(cudaMemcpy(p->d_mats, host.data(), total, cudaMemcpyHostToDevice));
@@ -275,7 +300,7 @@ int qsvb_create(int device_ordinal, qsvb_ctx** out) {
     QSVB_CK(cudaMalloc(&c->d_partials, reduce_partials_needed(c->num_sms) * sizeof(double)));
     QSVB_CK(cudaMemset(c->d_partials, 0, reduce_partials_needed(c->num_sms) * sizeof(double)));
     QSVB_CK(cudaMalloc(&c->d_result, 3 * sizeof(double)));
-    QSVB_CK(cudaHostAlloc(reinterpret_cast<void**>(&c->h_result), 3 * sizeof(double), cudaHostAllocMapped));
+    QSVB_CK(cudaHostAlloc(reinterpret_cast<void**>(&c->h_result), 4 * sizeof(double), cudaHostAllocMapped));
     QSVB_CK(cudaMalloc(&c->d_err, sizeof(int)));
     QSVB_CK(cudaMemset(c->d_err, 0, sizeof(int)));
     *out = c.release();
@@ -292,6 +317,7 @@ int qsvb_destroy(qsvb_ctx* c) {
     if (c->h_result) cudaFreeHost(c->h_result);
     if (c->d_mat_ring) cudaFree(c->d_mat_ring);
     if (c->d_exec_mats) cudaFree(c->d_exec_mats);
+    drop_spares(c);
     if (c->d_prob) cudaFree(c->d_prob);
     if (c->d_sample) cudaFree(c->d_sample);
     if (c->d_err) cudaFree(c->d_err);
@@ -329,17 +355,27 @@ int qsvb_state_alloc(qsvb_ctx* c, uint32_t n, int dtype, qsvb_state** out) {
     DeviceGuard dg(c->device);
     std::unique_ptr<qsvb_state> s(new qsvb_state{n, dtype, c->device, nullptr, nullptr});
     const size_t bytes = state_bytes(s.get());
-    size_t free_b = 0, total_b = 0;
-    QSVB_CK(cudaMemGetInfo(&free_b, &total_b));
-    if (2 * bytes > free_b)
-      throw Error(QSVB_E_OOM, "state of " + std::to_string(n) + " qubits needs " + std::to_string(2 * bytes) +
-                                  " bytes; " + std::to_string(free_b) + " free");
-    cudaError_t e = cudaMalloc(&s->re, bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&s->im, bytes);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      if (s->re) cudaFree(s->re);
-      throw Error(QSVB_E_OOM, std::string("state allocation failed: ") + cudaGetErrorString(e));
+    s->re = take_spare(c, bytes);
+    s->im = s->re ? take_spare(c, bytes) : nullptr;
+    if (!s->im) {
+      if (s->re) give_spare(c, s->re, bytes);
+      s->re = nullptr;
+      size_t free_b = 0, total_b = 0;
+      QSVB_CK(cudaMemGetInfo(&free_b, &total_b));
+      if (2 * bytes > free_b && !c->spare.empty()) {
+        drop_spares(c);
+        QSVB_CK(cudaMemGetInfo(&free_b, &total_b));
+      }
+      if (2 * bytes > free_b)
+        throw Error(QSVB_E_OOM, "state of " + std::to_string(n) + " qubits needs " + std::to_string(2 * bytes) +
+                                    " bytes; " + std::to_string(free_b) + " free");
+      cudaError_t e = cudaMalloc(&s->re, bytes);
+      if (e == cudaSuccess) e = cudaMalloc(&s->im, bytes);
+      if (e != cudaSuccess) {
+        cudaGetLastError();
+        if (s->re) cudaFree(s->re);
+        throw Error(QSVB_E_OOM, std::string("state allocation failed: ") + cudaGetErrorString(e));
+      }
     }
     *out = s.release();
   });
@@ -350,9 +386,12 @@ int qsvb_state_free(qsvb_ctx* c, qsvb_state* s) {
     if (!s) return;
     check_state(c, s);
     DeviceGuard dg(c->device);
-    QSVB_CK(cudaStreamSynchronize(c->stream));
-    cudaFree(s->re);
-    cudaFree(s->im);
+    // a buffer kept for reuse must be as free of pending work as cudaFree leaves one: work that the caller
+    // queued on it on other streams is waited for, too
+    QSVB_CK(cudaDeviceSynchronize());
+    const size_t bytes = state_bytes(s);
+    give_spare(c, s->re, bytes);
+    give_spare(c, s->im, bytes);
     delete s;
   });
 }

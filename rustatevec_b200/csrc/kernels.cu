@@ -1187,7 +1187,8 @@ void launch_dense_mma_shape(const LaunchEnv& env, R* re, R* im, uint64_t ngroups
                             const TailIf<R, TAIL>& t) {
   constexpr size_t smem = size_t(32) << (2 * K);
   auto kern = k_dense_mma<R, K, G, TH, MINB, TAIL>;
-  QSVB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  if constexpr (smem > 48 * 1024)
+    QSVB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   const uint64_t items = ngroups / G;
   launch_pdl(kern, grid_for(items, TH / 32, env.num_sms, MINB), TH, smem, env.stream, re, im, items, u, p, t);
   check_launch();

@@ -234,14 +234,22 @@ Gate make_group(const std::vector<const Gate*>& grp, bool cost_only) {
   return compose(q, grp);
 }
 
-// The fused gates of a grouping, in order. Full compositions of many groups run on host threads
-// (each group is independent; the result does not depend on the split).
+// The fused gates of a grouping, in order. Full compositions run on host threads once there is enough
+// to do (each group is independent; the result does not depend on the split): a product with a gate costs
+// about 4^k steps on k qubits, and starting the threads takes longer than 2^20 of them. 180 gates in 50
+// groups of 4 qubits (47,000 steps): 0.43 -> 0.18 ms for the whole plan without threads.
 std::vector<Gate> emit_groups(const std::vector<std::vector<const Gate*>>& groups, bool cost_only) {
   std::vector<Gate> out(groups.size());
   auto range = [&](size_t lo, size_t hi) {
     for (size_t i = lo; i < hi; ++i) out[i] = make_group(groups[i], cost_only);
   };
-  parallel_ranges(groups.size(), cost_only ? SIZE_MAX : 32, range);
+  size_t steps = 0;
+  for (const auto& grp : groups) {
+    uint64_t mask = 0;
+    for (const Gate* g : grp) mask |= qmask(*g);
+    if (grp.size() > 1) steps += grp.size() << (2 * __builtin_popcountll(mask));
+  }
+  parallel_ranges(groups.size(), cost_only || steps < (size_t(1) << 20) ? SIZE_MAX : 32, range);
   return out;
 }
 

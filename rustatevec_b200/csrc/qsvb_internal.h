@@ -10,6 +10,7 @@
 #include <stdexcept>
 #include <string>
 #include <thread>
+#include <utility>
 #include <vector>
 
 #include "../../include/qsvb.h"
@@ -262,7 +263,8 @@ struct qsvb_ctx {
   cudaStream_t stream = nullptr;
   double* d_partials = nullptr;   // reduction partials
   double* d_result = nullptr;     // 3 doubles (results that stay on the device)
-  double* h_result = nullptr;     // the same in pinned host memory (results the host waits for)
+  double* h_result = nullptr;     // the same in pinned host memory (results the host waits for), then the
+                                  // error flag as sync_and_check copies it
   char* d_mat_ring = nullptr;     // per-apply matrix uploads
   size_t mat_ring_cap = 0;
   size_t mat_ring_pos = 0;
@@ -272,6 +274,11 @@ struct qsvb_ctx {
   size_t prob_cap = 0;
   char* d_sample = nullptr;       // sampling scratch (sample.cu)
   size_t sample_cap = 0;
+  // Memory of freed states, kept for the next states of the same size (at most kStateKeep bytes in all, so
+  // small states only; returned on destroy and when a larger state needs it): cudaMalloc takes 0.1 to 100 ms
+  // on a busy host, as long as a one-shot circuit on such a state.
+  std::vector<std::pair<size_t, void*>> spare;
+  size_t spare_bytes = 0;
   int* d_err = nullptr;           // device error flag (bounded waits)
   void* h_pin[2] = {nullptr, nullptr};      // pinned host ring for large device -> host copies
   cudaEvent_t pin_ev[2] = {nullptr, nullptr};
@@ -284,6 +291,7 @@ namespace qsvb {
 // fills a device chunk first (it returns the device pointer to copy from); pass nullptr to copy
 // straight from `src`.
 constexpr size_t kPinChunk = size_t(64) << 20;
+constexpr size_t kStateKeep = size_t(64) << 20;
 void d2h_staged(qsvb_ctx* c, void* dst, const void* src, size_t bytes);
 void sample_shots(qsvb_ctx* c, const qsvb_state* st, uint64_t shots, uint64_t seed, uint64_t* out);
 }  // namespace qsvb
