@@ -99,15 +99,6 @@ __device__ __forceinline__ void apply2(const M2<R>& g, R& r0, R& i0, R& r1, R& i
   r0 = y0r; i0 = y0i; r1 = y1r; i1 = y1i;
 }
 
-// Programmatic launch: a kernel launched with launch_pdl may start while the one before it on the stream
-// is still running (as soon as every block of that one has called early_next), so that its launch, its
-// block scheduling and the staging of its matrix overlap it. It must not touch the state, nor anything else
-// an earlier kernel writes, before wait_prior, which returns when everything before it has finished and
-// is visible. Every thread calls both, whatever launched the kernel (they do nothing after an ordinary
-// launch). 28 dependent sweeps of a 12-qubit state, complex128: 97 -> 58 us.
-__device__ __forceinline__ void early_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void wait_prior() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 __device__ __forceinline__ uint64_t gtid() { return blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; }
 __device__ __forceinline__ uint64_t gstride() { return (uint64_t)gridDim.x * blockDim.x; }
 
@@ -1050,22 +1041,6 @@ inline unsigned grid_for(uint64_t items, int per_block, int num_sms, int blocks_
 }
 
 inline void check_launch() { QSVB_CK(cudaGetLastError()); }
-
-// Launches a kernel that calls early_next and wait_prior (see there).
-template <class... P, class... A>
-void launch_pdl(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, A&&... args) {
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  QSVB_CK(cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...));
-}
 
 template <class R> M2<R> to_m2(const std::vector<cd>& u) {
   M2<R> g;

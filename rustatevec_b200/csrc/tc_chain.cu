@@ -341,6 +341,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_chain(float* __restrict__ re
   constexpr int NIO = 3;                       // input slots
   constexpr uint32_t A0 = 64u * DEPTH;         // tensor-memory column of matrix 0's Whi
   static_assert(A0 + 128u * (DEPTH == 2 ? 3u : 2u) <= uint32_t(kTmemCols), "chain pass: tensor memory");
+  early_next();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* bbuf = smem;                                               // buffer b: hi, then lo
@@ -432,6 +433,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_chain(float* __restrict__ re
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  // barriers, tensor memory and matrices are set up; every thread waits here for the sweep before (not in
+  // its role, where the waits are bounded)
+  wait_prior();
 
   auto tile_base = [&](uint64_t tile) {
     uint64_t base = tile << 6;
@@ -705,6 +709,7 @@ __global__ void __launch_bounds__(kPermThreads) k_permute_tiles(R* __restrict__ 
                                                                 const __grid_constant__ PermParams p) {
   using V = typename std::conditional<sizeof(R) == 4, float4, double2>::type;
   constexpr int VN = 16 / sizeof(R);  // amplitudes per 16-byte vector
+  early_next();
   extern __shared__ __align__(16) uint8_t smem_raw[];
   R* sre = reinterpret_cast<R*>(smem_raw);
   R* sim = sre + kTileAmps;
@@ -716,6 +721,7 @@ __global__ void __launch_bounds__(kPermThreads) k_permute_tiles(R* __restrict__ 
     s_phi[i] = p.phi[i];
   }
   __syncthreads();
+  wait_prior();
   for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     uint64_t base = tile << 6;
 #pragma unroll
@@ -1224,9 +1230,8 @@ void launch_tc_chain(const LaunchEnv& env, float* re, float* im, uint32_t n, con
                                int(cudaSharedmemCarveoutMaxShared)));
   // one persistent CTA per SM (the tensor-memory allocation of 512 columns assumes it)
   const unsigned grid = unsigned(std::max<uint64_t>(1, std::min<uint64_t>(ntiles, uint64_t(env.num_sms))));
-  kern<<<grid, kThreads, kChainSmem, env.stream>>>(re, im, ntiles, static_cast<const uint4*>(dev_mat), p,
-                                                     env.err_flag, lay.maps[0], lay.maps[1]);
-  QSVB_CK(cudaGetLastError());
+  launch_pdl(kern, grid, kThreads, kChainSmem, env.stream, re, im, ntiles, static_cast<const uint4*>(dev_mat), p,
+             env.err_flag, lay.maps[0], lay.maps[1]);
 }
 
 template <class R>
@@ -1249,8 +1254,7 @@ void launch_permute(const LaunchEnv& env, R* re, R* im, uint32_t n, const Sweep&
   QSVB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_permute_tiles<R>, kPermThreads, smem));
   QSVB_REQUIRE(occ >= 1, "permutation kernel does not fit on an SM");
   const unsigned grid = unsigned(std::max<uint64_t>(1, std::min<uint64_t>(ntiles, uint64_t(env.num_sms) * occ)));
-  k_permute_tiles<R><<<grid, kPermThreads, smem, env.stream>>>(re, im, ntiles, p);
-  QSVB_CK(cudaGetLastError());
+  launch_pdl(k_permute_tiles<R>, grid, kPermThreads, smem, env.stream, re, im, ntiles, p);
 }
 template void launch_permute<float>(const LaunchEnv&, float*, float*, uint32_t, const Sweep&);
 template void launch_permute<double>(const LaunchEnv&, double*, double*, uint32_t, const Sweep&);

@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_dense(float* __restrict__ 
                                                             TcParams p, int* err, long long* prof,
                                                             const __grid_constant__ CUtensorMap tm_re,
                                                             const __grid_constant__ CUtensorMap tm_im) {
+  early_next();
   constexpr int M2 = 1 << KQ;      // complex gate rows
   constexpr int KR = 2 * M2;       // real rows of one block
   constexpr int NCB = kTileBits - KQ;
@@ -196,6 +197,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_dense(float* __restrict__ 
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+
+  // everything that does not touch the state is set up; every thread waits here for the sweep before (not
+  // in its role, where the waits are bounded)
+  wait_prior();
 
   auto tile_base = [&](uint64_t tile) {
     uint64_t base = tile << 6;
@@ -766,9 +771,8 @@ static void launch_tc_k(const LaunchEnv& env, float* re, float* im, uint32_t n, 
   long long* prof = nullptr;
   if (profile) QSVB_CK(cudaMalloc(&prof, sizeof(long long) * 12 * grid));
   if (prof) QSVB_CK(cudaMemsetAsync(prof, 0, sizeof(long long) * 12 * grid, env.stream));
-  kern<<<grid, kTcThreads, kTcSmem, env.stream>>>(re, im, ntiles, static_cast<const uint4*>(dev_mat), p, env.err_flag,
-                                                  prof, lay.maps[0], lay.maps[1]);
-  QSVB_CK(cudaGetLastError());
+  launch_pdl(kern, grid, kTcThreads, kTcSmem, env.stream, re, im, ntiles, static_cast<const uint4*>(dev_mat), p,
+             env.err_flag, prof, lay.maps[0], lay.maps[1]);
   if (prof) {
     std::vector<long long> h(12 * size_t(grid));
     QSVB_CK(cudaMemcpyAsync(h.data(), prof, h.size() * sizeof(long long), cudaMemcpyDeviceToHost, env.stream));
