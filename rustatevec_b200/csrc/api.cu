@@ -146,6 +146,7 @@ void run_sweep(qsvb_ctx* c, qsvb_state* st, const Sweep& s, const void* dev_mat,
     using R = decltype(r);
     launch_sweep<R>(c->env(), static_cast<R*>(st->re), static_cast<R*>(st->im), st->n_qubits, s, dev_mat, tail);
   });
+  c->reverse = !c->reverse;
 }
 
 // exec_block: the plan is run once and freed by the caller before the context's next call (one-shot

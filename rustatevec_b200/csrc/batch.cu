@@ -796,14 +796,15 @@ __global__ void __launch_bounds__(NT, MINB)
   wait_prior();
   long long t_wait = 0, t_fill = 0, t_gates = 0, t_out = 0, n_items = 0, t_mark = prof ? clock64() : 0;
   uint32_t staged_pass = ~0u;
-  // fixed != 0: one pass (passes[0]) over one state, tile i handled by block i mod grid, no queue
+  // fixed != 0: one pass (passes[0]) over one state, tile i (2: from the last one) handled by block i mod
+  // grid, no queue
   uint32_t iter = 0;
   while (true) {
     if (!fixed && tid == 0) s_item = atomicAdd(queue, 1u);
     __syncthreads();
     const uint32_t it = fixed ? blockIdx.x + (iter++) * gridDim.x : s_item;
     if (it >= nitems) break;
-    const Item item = fixed ? Item{0u, it} : items[it];
+    const Item item = fixed ? Item{0u, fixed == 2u ? nitems - 1u - it : it} : items[it];
     const PassDev& P = passes[item.pass];
     const uint32_t L = P.nlocal, T = 1u << L;
     [[maybe_unused]] const uint64_t gsize = 1ull << (L + P.nnon);  // the circuit's amplitudes (checked builds)
@@ -2268,7 +2269,7 @@ void launch_tile_variant(const LaunchEnv& e, R* re, R* im, const Sweep& s, const
              reinterpret_cast<const PassDev*>(base), reinterpret_cast<const PhaseDev*>(base + s.tile_off_phase),
              reinterpret_cast<const Instr*>(base + s.tile_off_prog), reinterpret_cast<const R*>(base + s.tile_off_coef),
              re, im, static_cast<double*>(nullptr), static_cast<double*>(nullptr), static_cast<uint32_t*>(nullptr),
-             static_cast<uint32_t*>(nullptr), e.err_flag, s.tile_lbits, static_cast<long long*>(nullptr), 1u,
+             static_cast<uint32_t*>(nullptr), e.err_flag, s.tile_lbits, static_cast<long long*>(nullptr), e.reverse ? 2u : 1u,
              static_cast<const long long*>(nullptr));
 }
 }  // namespace

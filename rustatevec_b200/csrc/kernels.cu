@@ -62,10 +62,11 @@ struct Enum {
   uint32_t nfixed;
   uint32_t fixed[7];
   uint64_t set_mask;
+  uint64_t flip;  // XORed to the work item (LaunchEnv::flip)
 };
 
 __device__ __forceinline__ uint64_t enum_base(uint64_t w, uint32_t cb, const Enum& e) {
-  uint64_t x = w << cb;
+  uint64_t x = (w ^ e.flip) << cb;
 #pragma unroll
   for (uint32_t j = 0; j < 7; ++j) {
     if (j < e.nfixed) {
@@ -485,6 +486,7 @@ template <class R, bool TAIL> using TailIf = std::conditional_t<TAIL, Tail<R>, N
 struct DenseMmaP {
   uint64_t bit[6];  // address of the gate bits, ascending
   uint64_t grp[3];  // address of the column bits that number a warp's groups
+  uint64_t flip;    // XORed to the item (LaunchEnv::flip)
 };
 
 template <class R, int K, int G, int TH, int MINB, bool TAIL>
@@ -526,7 +528,7 @@ __global__ void __launch_bounds__(TH, MINB) k_dense_mma(R* __restrict__ re, R* _
   const uint64_t nwarps = uint64_t(gridDim.x) * (TH / 32);
 #pragma unroll 1
   for (uint64_t w = blockIdx.x * uint64_t(TH / 32) + (threadIdx.x >> 5); w < nitems; w += nwarps) {
-    uint64_t base = w * (G * 8) + (lane >> 2);
+    uint64_t base = (w ^ p.flip) * (G * 8) + (lane >> 2);
 #pragma unroll
     for (int j = 0; j < K; ++j) {
       const uint64_t lo = base & (p.bit[j] - 1ull);
@@ -596,6 +598,7 @@ struct DenseColP {
   uint32_t zero;          // 0: see `fresh`
   uint64_t hi[4];         // address of the gate bits that are not in the vector
   uint64_t ext[2];        // address of the extra column bits
+  uint64_t flip;          // XORed to the item (LaunchEnv::flip)
 };
 
 using f32x2 = unsigned long long;
@@ -659,7 +662,7 @@ __global__ void __launch_bounds__(TH, 1) k_dense_cols(float* __restrict__ re, fl
   const uint64_t nwarps = uint64_t(gridDim.x) * (TH / 32);
 #pragma unroll 1
   for (uint64_t w = blockIdx.x * uint64_t(TH / 32) + (threadIdx.x >> 5); w < nitems; w += nwarps) {
-    const uint64_t base = insert(w << (5 + NL)) + lane_off;
+    const uint64_t base = insert((w ^ p.flip) << (5 + NL)) + lane_off;
     asm volatile("" ::: "memory");  // the matrix stays in shared memory (hoisted, it would spill)
     uint32_t tsub = 0;  // tail sub-index of the thread's first amplitude
     if constexpr (TAIL) tsub = tail_index(t, base);
@@ -1051,8 +1054,9 @@ template <class R> M2<R> to_m2(const std::vector<cd>& u) {
   return g;
 }
 
-Enum make_enum(std::vector<uint32_t> fixed, uint64_t set_mask) {
+Enum make_enum(std::vector<uint32_t> fixed, uint64_t set_mask, uint64_t flip = 0) {
   Enum e{};
+  e.flip = flip;
   std::sort(fixed.begin(), fixed.end());
   QSVB_REQUIRE(fixed.size() <= 7, "too many fixed bits");
   e.nfixed = uint32_t(fixed.size());
@@ -1090,25 +1094,25 @@ void launch_pair(const LaunchEnv& env, R* re, R* im, uint32_t n, uint32_t t, con
       const uint64_t nwork = 1ull << (n - LOG - fixed.size());
       auto kern = t == 0 ? k_pair_invec<R, 0> : k_pair_invec<R, LOG - 1>;  // LOG is 1 or 2
       launch_pdl(kern, grid_for(nwork, kThreads, env.num_sms), kThreads, 0, env.stream, re, im, nwork,
-                 make_enum(fixed, set), low, g);
+                 make_enum(fixed, set, env.flip(nwork)), low, g);
     } else if (t < LOG + 5) {
       const uint64_t set = split(LOG + 5, fixed, low);
       const uint64_t nwork = 1ull << (n - LOG - 5 - fixed.size());
       launch_pdl(k_pair_shfl<R>, grid_for(nwork * 32, kThreads, env.num_sms), kThreads, 0, env.stream,
-          re, im, nwork, make_enum(fixed, set), t, low, g);
+          re, im, nwork, make_enum(fixed, set, env.flip(nwork)), t, low, g);
     } else {
       const uint64_t set = split(LOG, fixed, low);
       fixed.push_back(t);
       const uint64_t nwork = 1ull << (n - LOG - fixed.size());
       launch_pdl(k_pair_strided<R>, grid_for(nwork, kThreads, env.num_sms), kThreads, 0, env.stream,
-          re, im, nwork, make_enum(fixed, set), t, low, g);
+          re, im, nwork, make_enum(fixed, set, env.flip(nwork)), t, low, g);
     }
   } else {
     std::vector<uint32_t> fixed(ctrl, ctrl + nctrl);
     fixed.push_back(t);
     const uint64_t nwork = 1ull << (n - fixed.size());
     launch_pdl(k_pair_scalar<R>, grid_for(nwork, kThreads, env.num_sms), kThreads, 0, env.stream,
-        re, im, nwork, make_enum(fixed, cmask), t, g);
+        re, im, nwork, make_enum(fixed, cmask, env.flip(nwork)), t, g);
   }
   check_launch();
 }
@@ -1134,7 +1138,7 @@ void launch_diag(const LaunchEnv& env, R* re, R* im, uint32_t n, const Sweep& s)
       }
     const uint64_t nwork = 1ull << (n - LOG - fixed.size());
     launch_pdl(k_diag<R>, grid_for(nwork, kThreads, env.num_sms), kThreads, 0, env.stream,
-        re, im, nwork, make_enum(fixed, set), p);
+        re, im, nwork, make_enum(fixed, set, env.flip(nwork)), p);
   } else {
     const uint64_t dim = 1ull << n;
     launch_pdl(k_diag_scalar<R>, grid_for(dim, kThreads, env.num_sms), kThreads, 0, env.stream, re, im, dim, p);
@@ -1158,13 +1162,14 @@ constexpr DenseMmaShape dense_mma_shape(int K) {
 }
 
 template <class R, int K, int G, int TH, int MINB, bool TAIL>
-void launch_dense_mma_shape(const LaunchEnv& env, R* re, R* im, uint64_t ngroups, const R* u, const DenseMmaP& p,
+void launch_dense_mma_shape(const LaunchEnv& env, R* re, R* im, uint64_t ngroups, const R* u, DenseMmaP p,
                             const TailIf<R, TAIL>& t) {
   constexpr size_t smem = size_t(32) << (2 * K);
   auto kern = k_dense_mma<R, K, G, TH, MINB, TAIL>;
   if constexpr (smem > 48 * 1024)
     QSVB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   const uint64_t items = ngroups / G;
+  p.flip = env.flip(items);
   launch_pdl(kern, grid_for(items, TH / 32, env.num_sms, MINB), TH, smem, env.stream, re, im, items, u, p, t);
   check_launch();
 }
@@ -1214,10 +1219,11 @@ constexpr int dense_cols_threads(int K, int nlow, int l2) {
 }
 
 template <int K, int L0, int L1, int L2, bool TAIL>
-void launch_dense_cols_at(const LaunchEnv& env, float* re, float* im, uint32_t n, const float* u, const DenseColP& p,
+void launch_dense_cols_at(const LaunchEnv& env, float* re, float* im, uint32_t n, const float* u, DenseColP p,
                           const TailIf<float, TAIL>& t) {
   constexpr int TH = dense_cols_threads(K, L0 + L1, L2);
   const uint64_t items = 1ull << (n - K - 7);
+  p.flip = env.flip(items);
   launch_pdl(k_dense_cols<K, L0, L1, L2, TH, TAIL>, grid_for(items, TH / 32, env.num_sms, 1), TH, 0, env.stream, re, im,
              items, reinterpret_cast<const float2*>(u), p, t);
   check_launch();

@@ -86,6 +86,7 @@ static_assert(kChainSmem <= 232448, "chain pass: shared memory above the 227 KB 
 static_assert(kChainMaxMats * 128 + 2 * 64 <= kTmemCols && 2 * 128 + 4 * 64 <= kTmemCols, "chain pass: tensor memory");
 
 struct ChainParams {
+  uint64_t flip;  // XORed to the tile's number (LaunchEnv::flip)
   // tile addressing (tile_layout)
   uint32_t hibits[6];
   uint64_t hioff[64];
@@ -438,7 +439,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_chain(float* __restrict__ re
   wait_prior();
 
   auto tile_base = [&](uint64_t tile) {
-    uint64_t base = tile << 6;
+    uint64_t base = (tile ^ p.flip) << 6;
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
       const uint32_t b = p.hibits[j];
@@ -699,6 +700,7 @@ struct PermParams {
   uint32_t hibits[6];
   uint64_t hioff[64];
   uint16_t plo[64], phi[64];  // destination tile position of each value of the low / high six bits
+  uint64_t flip;              // XORed to the tile's number (LaunchEnv::flip)
 };
 
 // Each block moves its tiles through shared memory: 16-byte loads of the tile in address order,
@@ -723,7 +725,7 @@ __global__ void __launch_bounds__(kPermThreads) k_permute_tiles(R* __restrict__ 
   __syncthreads();
   wait_prior();
   for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    uint64_t base = tile << 6;
+    uint64_t base = (tile ^ p.flip) << 6;
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
       const uint32_t b = p.hibits[j];
@@ -1220,6 +1222,7 @@ void launch_tc_chain(const LaunchEnv& env, float* re, float* im, uint32_t n, con
   TileLayout lay;
   const uint32_t bmode = build_chain_params(s, n, re, im, p, lay);
   const uint64_t ntiles = 1ull << (n - 12);
+  p.flip = env.flip(ntiles);
   // up to two matrices: four accumulators (tiles in flight); three matrices leave tensor memory for two
   using Kern = decltype(&k_tc_chain<0, 2>);
   static const Kern kerns[2][4] = {{k_tc_chain<0, 2>, k_tc_chain<1, 2>, k_tc_chain<2, 2>, k_tc_chain<3, 2>},
@@ -1248,6 +1251,7 @@ void launch_permute(const LaunchEnv& env, R* re, R* im, uint32_t n, const Sweep&
     p.phi[i] = uint16_t(permute12(i << 6, s.chain_perm));
   }
   const uint64_t ntiles = 1ull << (n - 12);
+  p.flip = env.flip(ntiles);
   const size_t smem = 2 * sizeof(R) * kTileAmps;
   QSVB_CK(cudaFuncSetAttribute(k_permute_tiles<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   int occ = 0;

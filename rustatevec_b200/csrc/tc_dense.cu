@@ -78,6 +78,7 @@ constexpr size_t kTcSmem = 1024 + kBSlots * 2 * size_t(kBBytes) + kIoBufs * size
 static_assert(kTcSmem <= 232448, "tensor-core sweep: shared memory above the 227 KB per-block limit");
 
 struct TcParams {
+  uint64_t flip;  // XORed to the tile's number (LaunchEnv::flip)
   uint32_t hibits[6];      // tile bits above the 6 lowest state bits (ascending)
   uint32_t ncb;            // column bits (12 - k)
   uint32_t runbits;        // log2 of the contiguous run length of a tile (>= 6)
@@ -203,7 +204,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_dense(float* __restrict__ 
   wait_prior();
 
   auto tile_base = [&](uint64_t tile) {
-    uint64_t base = tile << 6;
+    uint64_t base = (tile ^ p.flip) << 6;
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
       const uint32_t b = p.hibits[j];
@@ -759,6 +760,7 @@ static void launch_tc_k(const LaunchEnv& env, float* re, float* im, uint32_t n, 
   }
 
   const uint64_t ntiles = 1ull << (n - kTileBits);
+  p.flip = env.flip(ntiles);
   auto kern = p.bmode == 0 ? k_tc_dense<KQ, 0> : p.bmode == 1 ? k_tc_dense<KQ, 1>
              : p.bmode == 2 ? k_tc_dense<KQ, 2> : k_tc_dense<KQ, 3>;
   QSVB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTcSmem)));
