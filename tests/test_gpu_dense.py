@@ -60,9 +60,12 @@ def test_dense_sweep_every_size_class(be64, be32, precision, k, n):
     st.free()
 
 
-def diagonal(m, rng, controls=0):
-    """A random diagonal on m qubits that acts only where the lowest `controls` bits are 1."""
-    d = np.exp(1j * rng.uniform(0, 2 * np.pi, size=1 << m))
+def diagonal(m, rng, controls=0, signs=False):
+    """A random diagonal (of signs, or of phases) on m qubits that acts only where the lowest `controls`
+    bits are 1."""
+    d = rng.choice([-1.0, 1.0], size=1 << m) if signs else np.exp(1j * rng.uniform(0, 2 * np.pi, size=1 << m))
+    d = d.astype(np.complex128)
+    d[-1] = -1.0 if signs else d[-1]
     d[(np.arange(1 << m) & ((1 << controls) - 1)) != (1 << controls) - 1] = 1.0
     return np.diag(d)
 
@@ -80,7 +83,7 @@ def test_diagonal_carried_by_a_dense_sweep(be64, be32, precision, k, n):
     for i, qs in enumerate(qsets if n < 17 else qsets[::4]):
         if len(set(qs)) < k:
             continue
-        m = 1 + i % 4
+        m = 1 + (i + k) % 5
         psi = rng.normal(size=1 << n) + 1j * rng.normal(size=1 << n)
         psi = (psi / np.linalg.norm(psi)).astype(np.complex128 if precision == "f64" else np.complex64)
         c = Circuit(n)
@@ -89,7 +92,7 @@ def test_diagonal_carried_by_a_dense_sweep(be64, be32, precision, k, n):
         dq = rng.permutation(qs)[:m].tolist() if inside else rng.choice(n, size=m, replace=False).tolist()
         m = len(dq)
         inside = set(dq) <= set(qs)
-        c.push(G.DenseGate(m, diagonal(m, rng, controls=i % 2)), dq)
+        c.push(G.DenseGate(m, diagonal(m, rng, controls=i % 2, signs=i % 4 >= 2)), dq)
         got = []
         for planner in (PLAN_AS_GIVEN, PLAN_GREEDY):  # (a width cap of 1 leaves the gates apart)
             plan = Plan(be, c, L.make_opts(planner, 1, ENGINE_CUDA_CORE))
