@@ -26,6 +26,22 @@ void set_last_error(const std::string& msg) { g_last_error = msg; }
                         file + ":" + std::to_string(line));
 }
 
+static void drop_spares(qsvb_ctx* c) {
+  for (auto& s : c->spare) cudaFree(s.second);
+  c->spare.clear();
+  c->spare_bytes = 0;
+}
+
+void device_malloc(qsvb_ctx* c, void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && !c->spare.empty()) {
+    cudaGetLastError();
+    drop_spares(c);
+    e = cudaMalloc(p, bytes);
+  }
+  QSVB_CK(e);
+}
+
 namespace {
 
 template <class F> int guarded(F&& f) {
@@ -110,12 +126,6 @@ void give_spare(qsvb_ctx* c, void* p, size_t bytes) {
   c->spare.emplace_back(bytes, p);
   c->spare_bytes += bytes;
 }
-void drop_spares(qsvb_ctx* c) {
-  for (auto& s : c->spare) cudaFree(s.second);
-  c->spare.clear();
-  c->spare_bytes = 0;
-}
-
 size_t state_bytes(const qsvb_state* s) { return (s->dtype == QSVB_C128 ? 8u : 4u) * (size_t(1) << s->n_qubits); }
 
 template <class F> void by_dtype(int dtype, F&& f) {
@@ -131,7 +141,7 @@ void* ring_upload(qsvb_ctx* c, const void* src, size_t bytes) {
     QSVB_CK(cudaStreamSynchronize(c->stream));
     if (c->d_mat_ring) QSVB_CK(cudaFree(c->d_mat_ring));
     c->mat_ring_cap = std::max(need, size_t(1) << 20);
-    QSVB_CK(cudaMalloc(&c->d_mat_ring, c->mat_ring_cap));
+    device_malloc(c, reinterpret_cast<void**>(&c->d_mat_ring), c->mat_ring_cap);
     c->mat_ring_pos = 0;
   }
   if (c->mat_ring_pos + need > c->mat_ring_cap) c->mat_ring_pos = 0;
@@ -197,7 +207,7 @@ qsvb_plan* build_plan(qsvb_ctx* c, const qsvb_circuit* circ, int dtype, const qs
         if (c->d_exec_mats) QSVB_CK(cudaFree(c->d_exec_mats));
         c->d_exec_mats = nullptr;
         c->exec_mats_cap = 0;
-        QSVB_CK(cudaMalloc(&c->d_exec_mats, total));
+        device_malloc(c, reinterpret_cast<void**>(&c->d_exec_mats), total);
         c->exec_mats_cap = total;
       }
       p->d_mats = c->d_exec_mats;
@@ -206,7 +216,7 @@ qsvb_plan* build_plan(qsvb_ctx* c, const qsvb_circuit* circ, int dtype, const qs
       // so the call returns once its contents are staged
       QSVB_CK(cudaMemcpyAsync(p->d_mats, host.data(), total, cudaMemcpyHostToDevice, c->stream));
     } else {
-      QSVB_CK(cudaMalloc(&p->d_mats, total));
+      device_malloc(c, reinterpret_cast<void**>(&p->d_mats), total);
       QSVB_CK(cudaMemcpy(p->d_mats, host.data(), total, cudaMemcpyHostToDevice));
     }
   }
@@ -387,12 +397,19 @@ int qsvb_state_free(qsvb_ctx* c, qsvb_state* s) {
     if (!s) return;
     check_state(c, s);
     DeviceGuard dg(c->device);
+    QSVB_CK(cudaStreamSynchronize(c->stream));
     // a buffer kept for reuse must be as free of pending work as cudaFree leaves one: work that the caller
-    // queued on it on other streams is waited for, too
-    QSVB_CK(cudaDeviceSynchronize());
-    const size_t bytes = state_bytes(s);
-    give_spare(c, s->re, bytes);
-    give_spare(c, s->im, bytes);
+    // queued on it on other streams is waited for, too (where that cannot be done, as while some stream is
+    // being captured, the buffers are freed)
+    if (cudaDeviceSynchronize() == cudaSuccess) {
+      const size_t bytes = state_bytes(s);
+      give_spare(c, s->re, bytes);
+      give_spare(c, s->im, bytes);
+    } else {
+      cudaGetLastError();
+      cudaFree(s->re);
+      cudaFree(s->im);
+    }
     delete s;
   });
 }
@@ -733,7 +750,7 @@ int qsvb_probabilities(qsvb_ctx* c, const qsvb_state* s, void* out, int out_dtyp
       QSVB_CK(cudaStreamSynchronize(c->stream));
       if (c->d_prob) QSVB_CK(cudaFree(c->d_prob));
       c->d_prob = nullptr;
-      QSVB_CK(cudaMalloc(&c->d_prob, chunk * esz));
+      device_malloc(c, &c->d_prob, chunk * esz);
       c->prob_cap = chunk * esz;
     }
     ensure_pinned(c);

@@ -2085,9 +2085,9 @@ qsvb_batch* batch_create(qsvb_ctx* c, const qsvb_circuit* circuits, size_t n, in
   }
   upload_vec(&b->d_zcnt, bp.zcnt, s);
   upload_vec(&b->d_zoff, bp.zoff, s);
-  QSVB_CK(cudaMalloc(&b->d_sre, std::max<uint64_t>(bp.state_amps, 1) * rb));
-  QSVB_CK(cudaMalloc(&b->d_sim, std::max<uint64_t>(bp.state_amps, 1) * rb));
-  QSVB_CK(cudaMalloc(reinterpret_cast<void**>(&b->d_probs), bp.prob_total * 8));
+  device_malloc(c, &b->d_sre, std::max<uint64_t>(bp.state_amps, 1) * rb);
+  device_malloc(c, &b->d_sim, std::max<uint64_t>(bp.state_amps, 1) * rb);
+  device_malloc(c, reinterpret_cast<void**>(&b->d_probs), bp.prob_total * 8);
   QSVB_CK(cudaMalloc(reinterpret_cast<void**>(&b->d_zpart), bp.zslots * 8));
   QSVB_CK(cudaMalloc(reinterpret_cast<void**>(&b->d_z0), size_t(bp.ncirc) * 8));
   QSVB_CK(cudaMalloc(reinterpret_cast<void**>(&b->d_done), bp.passes.size() * 4));

@@ -327,6 +327,8 @@ namespace qsvb {
 // straight from `src`.
 constexpr size_t kPinChunk = size_t(64) << 20;
 constexpr size_t kStateKeep = size_t(64) << 20;
+// cudaMalloc that gives the context's spare state buffers back before it fails.
+void device_malloc(qsvb_ctx* c, void** p, size_t bytes);
 void d2h_staged(qsvb_ctx* c, void* dst, const void* src, size_t bytes);
 void sample_shots(qsvb_ctx* c, const qsvb_state* st, uint64_t shots, uint64_t seed, uint64_t* out);
 }  // namespace qsvb

@@ -40,7 +40,7 @@ struct Scratch {
   bool keep = false;
   Scratch(qsvb_ctx* ctx, size_t bytes) : c(ctx), keep(bytes <= kSampleKeep) {
     if (!keep) {
-      QSVB_CK(cudaMalloc(&p, bytes));
+      device_malloc(c, reinterpret_cast<void**>(&p), bytes);
       return;
     }
     if (c->sample_cap < bytes) {
@@ -48,7 +48,7 @@ struct Scratch {
       if (c->d_sample) QSVB_CK(cudaFree(c->d_sample));
       c->d_sample = nullptr;
       c->sample_cap = 0;
-      QSVB_CK(cudaMalloc(&c->d_sample, bytes));
+      device_malloc(c, reinterpret_cast<void**>(&c->d_sample), bytes);
       c->sample_cap = bytes;
     }
     p = c->d_sample;
