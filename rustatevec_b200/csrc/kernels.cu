@@ -1054,6 +1054,17 @@ __global__ void k_probs(const R* __restrict__ re, const R* __restrict__ im, uint
 // ---------------------------------------------------------------------------------------------
 // host helpers
 // ---------------------------------------------------------------------------------------------
+// Blocks of a kernel an SM holds at a time. A grid of persistent blocks launched programmatically has to fill
+// every SM: its blocks start wherever the kernel before it leaves room, so with fewer of them than fit, the SMs
+// that finish first take more than their share (26-qubit complex128 two-qubit sweeps, 3 blocks an SM where 4 or
+// fit, back to back: 413 us against 337 us alone).
+inline int resident_blocks(const void* kern, int threads, size_t smem) {
+  int blocks = 0;
+  QSVB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, threads, smem));
+  QSVB_REQUIRE(blocks >= 1, "kernel does not fit on an SM");
+  return blocks;
+}
+
 inline unsigned grid_for(uint64_t items, int per_block, int num_sms, int blocks_per_sm = 8) {
   const uint64_t need = (items + per_block - 1) / per_block;
   const uint64_t cap = uint64_t(num_sms) * blocks_per_sm;
@@ -1166,12 +1177,13 @@ void launch_diag(const LaunchEnv& env, R* re, R* im, uint32_t n, const Sweep& s)
 // Launch shape of k_dense_mma for K gate bits: column groups of 8 a warp works on at a time, threads a
 // block, blocks an SM. More groups keep more bytes in flight and use each matrix fragment more often,
 // as far as registers allow (27-qubit complex128 states, gate bits 10..17: K = 4 0.99 / 0.78 / 0.71 ms
-// with 1 / 2 / 4 groups, K = 3 0.81 / 0.74 ms with 2 / 4, K = 5 1.27 / 1.24 ms with 1 / 2).
+// with 1 / 2 / 4 groups, K = 3 0.81 / 0.74 ms with 2 / 4, K = 5 1.27 / 1.24 ms with 1 / 2. K = 2 is one
+// block of 12 warps: with four blocks of four warps, which also fit, 26 qubits take 0.38 instead of 0.33 ms).
 struct DenseMmaShape {
   int groups, threads, blocks;
 };
 constexpr DenseMmaShape dense_mma_shape(int K) {
-  return K == 2 ? DenseMmaShape{8, 128, 3}
+  return K == 2 ? DenseMmaShape{8, 384, 1}
          : K == 3 ? DenseMmaShape{4, 128, 4}
          : K == 4 ? DenseMmaShape{4, 128, 3}
          : K == 5 ? DenseMmaShape{2, 128, 3}
@@ -1187,7 +1199,8 @@ void launch_dense_mma_shape(const LaunchEnv& env, R* re, R* im, uint64_t ngroups
     QSVB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   const uint64_t items = ngroups / G;
   p.flip = env.flip(items);
-  launch_pdl(kern, grid_for(items, TH / 32, env.num_sms, MINB), TH, smem, env.stream, re, im, items, u, p, t);
+  static const int per_sm = resident_blocks(reinterpret_cast<const void*>(kern), TH, smem);
+  launch_pdl(kern, grid_for(items, TH / 32, env.num_sms, per_sm), TH, smem, env.stream, re, im, items, u, p, t);
   check_launch();
 }
 

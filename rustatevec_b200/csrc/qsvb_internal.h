@@ -260,13 +260,15 @@ namespace qsvb {
 // block scheduling and the staging of its matrix overlap it. It must not touch the state, nor anything else
 // an earlier kernel writes, before wait_prior, which returns when everything before it has finished and
 // is visible. Every thread calls both, whatever launched the kernel (they do nothing after an ordinary
-// launch). 28 dependent sweeps of a 12-qubit state, complex128: 97 -> 58 us.
+// launch). 28 dependent sweeps of a 12-qubit state and its <Z_0>, complex128, with reductions that end in one kernel:
+// 129 -> 62 us a replay.
 __device__ __forceinline__ void early_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_prior() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Launches a kernel that calls early_next and wait_prior (see there).
+// Launches a kernel that calls early_next and wait_prior (see there); programmatic = false: an ordinary launch.
 template <class... P, class... A>
-void launch_pdl(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, A&&... args) {
+void launch_pdl_if(bool programmatic, void (*kern)(P...), unsigned grid, unsigned block, size_t smem,
+                   cudaStream_t stream, A&&... args) {
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
@@ -276,8 +278,12 @@ void launch_pdl(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, 
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = programmatic ? 1 : 0;
   QSVB_CK(cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...));
+}
+template <class... P, class... A>
+void launch_pdl(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, A&&... args) {
+  launch_pdl_if(true, kern, grid, block, smem, stream, std::forward<A>(args)...);
 }
 #endif
 }  // namespace qsvb
