@@ -175,7 +175,10 @@ qsvb_plan* build_plan(qsvb_ctx* c, const qsvb_circuit* circ, int dtype, const qs
   p->stats.n_gates_in = circ->n_gates;
   sweep_costs(p->sweeps, circ->n_qubits, dtype, &p->stats);
   // (as given: one sweep per gate, in order)
-  if (p->opts.planner != QSVB_PLAN_AS_GIVEN) attach_diagonals(p->sweeps, circ->n_qubits);
+  if (p->opts.planner != QSVB_PLAN_AS_GIVEN) {
+    p->stats.predicted_seconds = predict_plan_seconds(p->sweeps, circ->n_qubits, dtype, true);
+    attach_diagonals(p->sweeps, circ->n_qubits);
+  }
   // one device block holding every sweep's matrix, uploaded once
   size_t total = 0;
   for (const Sweep& s : p->sweeps) {

@@ -30,10 +30,21 @@ constexpr double kTileFp32Flops = 29.5e12;
 constexpr double kTileFp64Flops = 15.5e12;
 constexpr double kTileMemFactor32 = 1.95;
 constexpr double kTileMemFactor64 = 1.80;
+// the same form with a trained model installed, fitted to the kernels the model's records were taken on (411
+// passes of QFT, brickwork, QAOA, GHZ and random circuits at 22-30 qubits: mean |log2 error| 0.16 / 0.15, where
+// the constants above, which the planner without a model keeps, are off by 0.18 / 0.43)
+constexpr double kTrainedTileFp32Flops = 31.0e12;
+constexpr double kTrainedTileFp64Flops = 19.7e12;
+constexpr double kTrainedTileMemFactor32 = 1.72;
+constexpr double kTrainedTileMemFactor64 = 1.24;
 // chain and permutation passes (not in the cost model's training records: roofline times an
 // overhead factor)
 constexpr double kChainOverhead = 1.25;
 constexpr double kPermuteOverhead = 1.15;
+
+double tile_seconds(double mem, double flops, double mem_factor, double rate) {
+  return mem_factor * mem + flops / rate + kLaunchSeconds;
+}
 
 int lowest_bit(const Sweep& s) {
   uint32_t lo = 64;
@@ -106,9 +117,8 @@ double analytic_sweep_seconds(const Sweep& s, uint32_t n, int dtype) {
   if (s.kind == SK_PERMUTE) return mem * kPermuteOverhead + kLaunchSeconds;
   if (s.kind == SK_TILE) {
     // each block loads, updates and stores its tile in turn: memory and arithmetic add up
-    const double rate = dtype == QSVB_C128 ? kTileFp64Flops : kTileFp32Flops;
-    const double mf = dtype == QSVB_C128 ? kTileMemFactor64 : kTileMemFactor32;
-    return mf * mem + s.tile_flops / rate + kLaunchSeconds;
+    return tile_seconds(mem, s.tile_flops, dtype == QSVB_C128 ? kTileMemFactor64 : kTileMemFactor32,
+                        dtype == QSVB_C128 ? kTileFp64Flops : kTileFp32Flops);
   }
   return std::max(mem, comp) + kLaunchSeconds;
 }
@@ -235,12 +245,20 @@ double predict_sweep_seconds(const Sweep& s, uint32_t n, int dtype) {
     sweep_features(s, n, dtype, f);
     return std::exp2(double(mlp_forward_host_memo(m, f)));
   }
+  if (m.hidden > 0 && s.kind == SK_TILE) {
+    const double mem = std::ldexp(dtype == QSVB_C128 ? 32.0 : 16.0, int(n)) / kHbmBytesPerSec;
+    return tile_seconds(mem, s.tile_flops, dtype == QSVB_C128 ? kTrainedTileMemFactor64 : kTrainedTileMemFactor32,
+                        dtype == QSVB_C128 ? kTrainedTileFp64Flops : kTrainedTileFp32Flops);
+  }
   return analytic_sweep_seconds(s, n, dtype);
 }
 
-double predict_plan_seconds(const std::vector<Sweep>& sw, uint32_t n, int dtype) {
+double predict_plan_seconds(const std::vector<Sweep>& sw, uint32_t n, int dtype, bool carry) {
+  std::vector<char> carried;
+  if (carry) carried = carried_diagonals(sw, n);
   double t = 0;
-  for (const Sweep& s : sw) t += predict_sweep_seconds(s, n, dtype);
+  for (size_t i = 0; i < sw.size(); ++i)
+    if (!carry || !carried[i]) t += predict_sweep_seconds(sw[i], n, dtype);
   return t;
 }
 
@@ -284,7 +302,7 @@ std::vector<Gate> learned_fuse(const std::vector<Gate>& seg, uint32_t n, const q
       if (s.kind != SK_NONE) sw.push_back(std::move(s));
     }
     select_engines(sw, n, o, dtype);
-    return predict_plan_seconds(sw, n, dtype);
+    return predict_plan_seconds(sw, n, dtype, true);
   };
   const size_t ncand = 2 * size_t(cap);
   std::vector<double> secs(ncand, 1e300);

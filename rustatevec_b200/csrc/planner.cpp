@@ -459,7 +459,7 @@ std::vector<Sweep> plan_sweeps(const std::vector<Gate>& in, uint32_t n, const qs
     double best_t = 1e300;
     for (uint32_t m = 1; m <= uint32_t(kChainMaxMats); ++m) {
       std::vector<Sweep> cand = plan_chain(in, n, m);
-      const double t = predict_plan_seconds(cand, n, dtype);
+      const double t = predict_plan_seconds(cand, n, dtype, true);
       if (t < best_t) {
         best_t = t;
         best = std::move(cand);
@@ -492,7 +492,7 @@ std::vector<Sweep> plan_sweeps(const std::vector<Gate>& in, uint32_t n, const qs
   double best_t = 1e300;
   for (size_t c = 0; c < fut.size(); ++c) {
     std::vector<Sweep> cand = fut[c].get();
-    const double t = predict_plan_seconds(cand, n, dtype);
+    const double t = predict_plan_seconds(cand, n, dtype, true);
     if (t < best_t) {
       best_t = t;
       best = std::move(cand);
@@ -585,7 +585,7 @@ void tile_segment(const std::vector<Gate>& seg, uint32_t n, const qsvb_plan_opts
           std::vector<Sweep> alt = fused_sweeps(t.tile_gates, n, o, dtype);
           select_engines(alt, n, o, dtype);
           tile_prepare(t, n, dtype);
-          if (predict_plan_seconds(alt, n, dtype) <= predict_sweep_seconds(t, n, dtype)) {
+          if (predict_plan_seconds(alt, n, dtype, true) <= predict_sweep_seconds(t, n, dtype)) {
             res[i] = std::move(alt);
             continue;
           }
@@ -681,6 +681,61 @@ std::vector<Sweep> plan_with(const std::vector<Gate>& in, uint32_t n, const qsvb
 }
 }  // namespace
 
+namespace {
+uint64_t sweep_qubits(const Sweep& s) {
+  uint64_t m = 0;
+  switch (s.kind) {
+    case SK_1Q: return uint64_t(1) << s.target;
+    case SK_CTRL:
+      for (uint32_t j = 0; j < s.nctrl; ++j) m |= uint64_t(1) << s.ctrl[j];
+      return m | uint64_t(1) << s.target;
+    case SK_DENSE:
+    case SK_DENSE_TC:
+    case SK_DIAG:
+      for (uint32_t j = 0; j < s.m; ++j) m |= uint64_t(1) << s.q[j];
+      return m;
+    default: return ~uint64_t(0);
+  }
+}
+
+enum CarryHow { CARRY_NO, CARRY_INSIDE, CARRY_OPEN, CARRY_JOINT };
+
+// The sweep that carries the diagonal sweep i, and how; tails[j]: the qubits of sweep j's tail so far.
+std::pair<size_t, CarryHow> find_carrier(const std::vector<Sweep>& sw, size_t i, uint32_t n,
+                                         const std::vector<uint64_t>& tails) {
+  constexpr size_t kReach = 64;  // sweeps looked back over, to bound the planning time
+  const uint64_t dm = sweep_qubits(sw[i]);
+  std::pair<size_t, CarryHow> open{0, CARRY_NO}, joint{0, CARRY_NO};
+  for (size_t j = i; j-- > 0 && i - j <= kReach;) {
+    const Sweep& s = sw[j];
+    if (s.kind == SK_DIAG || s.kind == SK_PHASE) continue;
+    const uint64_t sm = sweep_qubits(s);
+    if (s.kind == SK_DENSE && (sm & dm) == dm) return {j, CARRY_INSIDE};
+    if (s.kind == SK_DENSE && n >= s.m + 3) {  // smaller states run one thread a block of amplitudes
+      if (tails[j] == 0)
+        open = {j, CARRY_OPEN};
+      else if (__builtin_popcountll(dm | tails[j]) <= 6)
+        joint = {j, CARRY_JOINT};
+    }
+    if (sm & dm) break;
+  }
+  return open.second != CARRY_NO ? open : joint;
+}
+}  // namespace
+
+std::vector<char> carried_diagonals(const std::vector<Sweep>& sw, uint32_t n) {
+  std::vector<char> out(sw.size(), 0);
+  std::vector<uint64_t> tails(sw.size(), 0);
+  for (size_t i = 0; i < sw.size(); ++i) {
+    if (sw[i].kind != SK_DIAG) continue;
+    const auto [j, how] = find_carrier(sw, i, n, tails);
+    if (how == CARRY_NO) continue;
+    out[i] = 1;
+    if (how != CARRY_INSIDE) tails[j] |= sweep_qubits(sw[i]);
+  }
+  return out;
+}
+
 // A diagonal sweep moves the whole state (or the part it acts on) for six flops an amplitude, so a dense
 // sweep takes it along: its kernel multiplies the product by the diagonal before the write-back. The
 // diagonal may be carried by any dense sweep it can be moved back to, past sweeps on other qubits and
@@ -689,45 +744,16 @@ std::vector<Sweep> plan_with(const std::vector<Gate>& in, uint32_t n, const qsvb
 // the diagonal joins a tail when the two together act on at most 6 qubits. On greedy 28-qubit brickwork
 // (complex64, k = 4, depth 6) 39 of 83 sweeps are carried: 63.5 -> 37.6 ms.
 void attach_diagonals(std::vector<Sweep>& sw, uint32_t n) {
-  constexpr size_t kReach = 64;  // sweeps looked back over, to bound the planning time
-  auto mask = [](const Sweep& s) {
-    uint64_t m = 0;
-    switch (s.kind) {
-      case SK_1Q: return uint64_t(1) << s.target;
-      case SK_CTRL:
-        for (uint32_t j = 0; j < s.nctrl; ++j) m |= uint64_t(1) << s.ctrl[j];
-        return m | uint64_t(1) << s.target;
-      case SK_DENSE:
-      case SK_DENSE_TC:
-      case SK_DIAG:
-        for (uint32_t j = 0; j < s.m; ++j) m |= uint64_t(1) << s.q[j];
-        return m;
-      default: return ~uint64_t(0);
-    }
-  };
+  std::vector<uint64_t> tails(sw.size(), 0);
   for (size_t i = 0; i < sw.size(); ++i) {
     Sweep& d = sw[i];
     if (d.kind != SK_DIAG) continue;
-    const uint64_t dm = mask(d);
-    Sweep *inside = nullptr, *open = nullptr, *joint = nullptr;
-    for (size_t j = i; j-- > 0 && i - j <= kReach;) {
-      Sweep& s = sw[j];
-      if (s.kind == SK_DIAG || s.kind == SK_PHASE) continue;
-      if (s.kind == SK_DENSE && (mask(s) & dm) == dm) {
-        inside = &s;
-        break;
-      }
-      if (s.kind == SK_DENSE && n >= s.m + 3) {  // smaller states run one thread a block of amplitudes
-        if (s.tail_m == 0) {
-          open = &s;
-        } else {
-          uint64_t both = dm;
-          for (uint32_t k = 0; k < s.tail_m; ++k) both |= uint64_t(1) << s.tail_q[k];
-          if (__builtin_popcountll(both) <= 6) joint = &s;
-        }
-      }
-      if (mask(s) & dm) break;
-    }
+    const auto [j, how] = find_carrier(sw, i, n, tails);
+    if (how == CARRY_NO) continue;
+    if (how != CARRY_INSIDE) tails[j] |= sweep_qubits(d);
+    Sweep* const inside = how == CARRY_INSIDE ? &sw[j] : nullptr;
+    Sweep* const open = how == CARRY_OPEN ? &sw[j] : nullptr;
+    Sweep* const joint = how == CARRY_JOINT ? &sw[j] : nullptr;
     if (inside) {
       const size_t M = size_t(1) << inside->m;
       for (size_t r = 0; r < M; ++r) {

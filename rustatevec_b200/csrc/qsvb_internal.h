@@ -183,6 +183,8 @@ std::vector<Sweep> plan_chain(const std::vector<Gate>& in, uint32_t n, uint32_t 
 // Lets dense sweeps carry diagonal sweeps in their write-back (Sweep::tail); the list of sweeps and
 // their costs stay as planned.
 void attach_diagonals(std::vector<Sweep>& sw, uint32_t n);
+// Which sweeps attach_diagonals would have carried (sweeps without matrices will do).
+std::vector<char> carried_diagonals(const std::vector<Sweep>& sw, uint32_t n);
 void sweep_costs(const std::vector<Sweep>& sw, uint32_t n, int dtype, qsvb_plan_stats* st);
 qsvb_plan_opts default_opts();
 
