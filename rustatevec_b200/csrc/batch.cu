@@ -2525,7 +2525,7 @@ void launch_tile(const LaunchEnv& e, R* re, R* im, uint32_t n, const Sweep& s, c
   const uint8_t* base = static_cast<const uint8_t*>(dev_blob);
   // five blocks per SM (some stream their tiles while others compute; the gates' register phases
   // and shared-memory round trips are latency-bound, so warps per SM set the pace): <= 102
-  // registers a thread, the 8 KB program stage and 128-entry address tables
+  // registers a thread, the 7.5 KB program stage and 128-entry address tables
   if constexpr (sizeof(R) == 8) launch_tile_variant<double, 3, 128, 5, 1>(e, re, im, s, base);
   else launch_tile_variant<float, 4, 128, 5, 1>(e, re, im, s, base);
 }
