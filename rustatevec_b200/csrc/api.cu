@@ -105,6 +105,10 @@ void check_state(const qsvb_ctx* c, const qsvb_state* s) {
   check_ctx(c);
   QSVB_REQUIRE(s != nullptr, "null state");
   QSVB_REQUIRE(s->device == c->device, "state belongs to another device");
+  if (s->shared) return;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (c->stream_shared) QSVB_CK(cudaStreamIsCapturing(c->stream, &capture));
+  if (s->owner != c || capture != cudaStreamCaptureStatusNone) s->shared = true;
 }
 
 // A component buffer of exactly `bytes` from the context's spare ones (nullptr: none).
@@ -348,6 +352,7 @@ int qsvb_stream(qsvb_ctx* c, void** out) {
   return guarded([&] {
     check_ctx(c);
     QSVB_REQUIRE(out != nullptr, "null output pointer");
+    c->stream_shared = true;
     *out = reinterpret_cast<void*>(c->stream);
   });
 }
@@ -367,7 +372,7 @@ int qsvb_state_alloc(qsvb_ctx* c, uint32_t n, int dtype, qsvb_state** out) {
     QSVB_REQUIRE(n >= 1 && n <= QSVB_MAX_QUBITS, "qubit count must be 1..34");
     QSVB_REQUIRE(dtype == QSVB_C64 || dtype == QSVB_C128, "dtype must be QSVB_C64 or QSVB_C128");
     DeviceGuard dg(c->device);
-    std::unique_ptr<qsvb_state> s(new qsvb_state{n, dtype, c->device, nullptr, nullptr});
+    std::unique_ptr<qsvb_state> s(new qsvb_state{n, dtype, c->device, nullptr, nullptr, c});
     const size_t bytes = state_bytes(s.get());
     s->re = take_spare(c, bytes);
     s->im = s->re ? take_spare(c, bytes) : nullptr;
@@ -401,17 +406,16 @@ int qsvb_state_free(qsvb_ctx* c, qsvb_state* s) {
     check_state(c, s);
     DeviceGuard dg(c->device);
     QSVB_CK(cudaStreamSynchronize(c->stream));
-    // a buffer kept for reuse must be as free of pending work as cudaFree leaves one: work that the caller
-    // queued on it on other streams is waited for, too (where that cannot be done, as while some stream is
-    // being captured, the buffers are freed)
-    if (cudaDeviceSynchronize() == cudaSuccess) {
+    // A buffer kept for reuse must be as free of pending work as cudaFree leaves one. Only this stream can hold
+    // any on a state that nothing else has seen; a shared one is freed (a wait for the whole device instead
+    // would end any capture in progress on it, other threads' included).
+    if (s->shared) {
+      cudaFree(s->re);
+      cudaFree(s->im);
+    } else {
       const size_t bytes = state_bytes(s);
       give_spare(c, s->re, bytes);
       give_spare(c, s->im, bytes);
-    } else {
-      cudaGetLastError();
-      cudaFree(s->re);
-      cudaFree(s->im);
     }
     delete s;
   });
@@ -422,6 +426,7 @@ int qsvb_state_info(const qsvb_state* s, uint32_t* n, int* dtype, void** re, voi
     QSVB_REQUIRE(s != nullptr, "null state");
     if (n) *n = s->n_qubits;
     if (dtype) *dtype = s->dtype;
+    if (re || im) s->shared = true;
     if (re) *re = s->re;
     if (im) *im = s->im;
   });

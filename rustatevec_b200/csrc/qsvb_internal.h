@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <complex>
 #include <cstdint>
 #include <future>
@@ -297,6 +298,10 @@ struct qsvb_state {
   int device;
   void* re;
   void* im;
+  const qsvb_ctx* owner = nullptr;  // the context that allocated it
+  // Work may be queued on it elsewhere than on the owner's stream: another context has used it, its pointers
+  // were handed out, or a caller's capture of the owner's stream recorded them.
+  mutable std::atomic<bool> shared{false};
 };
 
 struct qsvb_ctx {
@@ -318,13 +323,14 @@ struct qsvb_ctx {
   size_t sample_cap = 0;
   // Memory of freed states, kept for the next states of the same size (at most kStateKeep bytes in all, so
   // small states only; returned on destroy and when a larger state needs it): cudaMalloc takes 0.1 to 100 ms
-  // on a busy host, as long as a one-shot circuit on such a state.
+  // on a busy host, as long as a one-shot circuit on such a state. Shared states (qsvb_state::shared) are not kept.
   std::vector<std::pair<size_t, void*>> spare;
   size_t spare_bytes = 0;
   int* d_err = nullptr;           // device error flag (bounded waits)
   void* h_pin[2] = {nullptr, nullptr};      // pinned host ring for large device -> host copies
   cudaEvent_t pin_ev[2] = {nullptr, nullptr};
   bool reverse = false;           // direction of the next sweep (LaunchEnv::reverse)
+  bool stream_shared = false;     // qsvb_stream handed the stream out, so a caller may capture it
   qsvb::LaunchEnv env() const { return {stream, num_sms, d_err, reverse}; }
 };
 

@@ -1,0 +1,88 @@
+"""Memory of freed states: what freeing leaves alone, and what the next state finds in it."""
+import ctypes as C
+import threading
+
+import numpy as np
+import pytest
+
+from rustatevec_b200 import B200Backend
+from rustatevec_b200 import _lib as L
+from rustatevec_b200.circuits import random_circuit
+
+import oracle
+from helpers import max_abs_diff
+
+pytestmark = pytest.mark.gpu
+
+
+def pointers(state):
+    re, im = C.c_void_p(), C.c_void_p()
+    L.check(L.lib().qsvb_state_info(state.handle, None, None, C.byref(re), C.byref(im)))
+    return re.value, im.value
+
+
+@pytest.mark.parametrize("exposed", [False, True])
+def test_free_leaves_another_threads_capture_alone(be32, exposed):
+    """One thread records a graph on its own stream (thread-local capture, which allows other threads any
+    call) while another frees a state. A device-wide wait would invalidate the capture."""
+    import torch
+    state = be32.alloc(12)
+    be32.init_basis(state, 0)
+    if exposed:
+        pointers(state)
+    x = torch.zeros(1000, device="cuda")
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        graph.capture_begin(capture_error_mode="thread_local")
+        x.add_(1)
+        worker = threading.Thread(target=state.free)
+        worker.start()
+        worker.join()
+        x.add_(1)
+        graph.capture_end()
+    assert state.handle is None
+    graph.replay()
+    torch.cuda.synchronize()
+    assert bool((x == 2).all())
+
+
+def test_reused_memory_shows_nothing_of_its_last_state(built):
+    """One-shot circuits on states of changing sizes, whose memory held random amplitudes before."""
+    for precision, tol in (("f64", 1e-12), ("f32", 1e-5)):
+        be = B200Backend(0, precision=precision)
+        for i, n in enumerate((13, 9, 13, 13, 14, 9)):
+            for _ in range(2):
+                junk = be.alloc(n)
+                be.init_gaussian(junk, i)
+                junk.free()
+            c = random_circuit(n, 60, i)
+            state = be.execute(c)
+            re, im = oracle.run(c, oracle.REF, oracle.F64)
+            assert max_abs_diff(re + 1j * im, be.download(state).as_complex()) <= tol
+            state.free()
+        be.close()
+
+
+def test_two_states_never_share_memory(built):
+    """Freed through another context, or with their pointers handed out, buffers are not handed on; live states
+    of one size always differ."""
+    a, b = B200Backend(0, precision="f32"), B200Backend(0, precision="f32")
+    live = []
+    for i in range(12):
+        s = a.alloc(11)
+        a.init_basis(s, i)
+        if i % 3 == 0:
+            b.norm_sqr(s)
+        live.append(s)
+        if i % 4 == 3:
+            live.pop(0).free()
+    spans = sorted(p for s in live for p in pointers(s))
+    assert all(q - p >= 4 << 11 for p, q in zip(spans, spans[1:]))
+    kept = [i for i in range(12) if i not in (0, 1, 2)]
+    for i, s in zip(kept, live):
+        psi = a.download(s).as_complex()
+        assert psi[i] == 1 and np.count_nonzero(psi) == 1
+        s.free()
+    a.close()
+    b.close()
