@@ -27,7 +27,10 @@ void set_last_error(const std::string& msg) { g_last_error = msg; }
 }
 
 static void drop_spares(qsvb_ctx* c) {
-  for (auto& s : c->spare) cudaFree(s.second);
+  for (const SpareState& s : c->spare) {
+    cudaFree(s.re);
+    cudaFree(s.im);
+  }
   c->spare.clear();
   c->spare_bytes = 0;
 }
@@ -111,24 +114,35 @@ void check_state(const qsvb_ctx* c, const qsvb_state* s) {
   if (s->owner != c || capture != cudaStreamCaptureStatusNone) s->shared = true;
 }
 
-// A component buffer of exactly `bytes` from the context's spare ones (nullptr: none).
-void* take_spare(qsvb_ctx* c, size_t bytes) {
+// The two component buffers of a kept state of `bytes` a component, newest first.
+bool take_spare(qsvb_ctx* c, size_t bytes, void** re, void** im) {
   for (size_t i = c->spare.size(); i-- > 0;)
-    if (c->spare[i].first == bytes) {
-      void* p = c->spare[i].second;
+    if (c->spare[i].bytes == bytes) {
+      *re = c->spare[i].re;
+      *im = c->spare[i].im;
       c->spare.erase(c->spare.begin() + ptrdiff_t(i));
-      c->spare_bytes -= bytes;
-      return p;
+      c->spare_bytes -= 2 * bytes;
+      return true;
     }
-  return nullptr;
+  return false;
 }
-void give_spare(qsvb_ctx* c, void* p, size_t bytes) {
-  if (c->spare_bytes + bytes > kStateKeep) {
-    cudaFree(p);
+// Keeps a freed state's buffers; the oldest kept ones make room (sizes no longer in use do not hold the
+// cap), and a state that would not fit alone is freed, both halves.
+void give_spare(qsvb_ctx* c, void* re, void* im, size_t bytes) {
+  if (2 * bytes > kStateKeep) {
+    cudaFree(re);
+    cudaFree(im);
     return;
   }
-  c->spare.emplace_back(bytes, p);
-  c->spare_bytes += bytes;
+  while (c->spare_bytes + 2 * bytes > kStateKeep) {
+    const SpareState& old = c->spare.front();
+    cudaFree(old.re);
+    cudaFree(old.im);
+    c->spare_bytes -= 2 * old.bytes;
+    c->spare.erase(c->spare.begin());
+  }
+  c->spare.push_back({bytes, re, im});
+  c->spare_bytes += 2 * bytes;
 }
 size_t state_bytes(const qsvb_state* s) { return (s->dtype == QSVB_C128 ? 8u : 4u) * (size_t(1) << s->n_qubits); }
 
@@ -374,11 +388,7 @@ int qsvb_state_alloc(qsvb_ctx* c, uint32_t n, int dtype, qsvb_state** out) {
     DeviceGuard dg(c->device);
     std::unique_ptr<qsvb_state> s(new qsvb_state{n, dtype, c->device, nullptr, nullptr, c});
     const size_t bytes = state_bytes(s.get());
-    s->re = take_spare(c, bytes);
-    s->im = s->re ? take_spare(c, bytes) : nullptr;
-    if (!s->im) {
-      if (s->re) give_spare(c, s->re, bytes);
-      s->re = nullptr;
+    if (!take_spare(c, bytes, &s->re, &s->im)) {
       size_t free_b = 0, total_b = 0;
       QSVB_CK(cudaMemGetInfo(&free_b, &total_b));
       if (2 * bytes > free_b && !c->spare.empty()) {
@@ -413,9 +423,7 @@ int qsvb_state_free(qsvb_ctx* c, qsvb_state* s) {
       cudaFree(s->re);
       cudaFree(s->im);
     } else {
-      const size_t bytes = state_bytes(s);
-      give_spare(c, s->re, bytes);
-      give_spare(c, s->im, bytes);
+      give_spare(c, s->re, s->im, state_bytes(s));
     }
     delete s;
   });

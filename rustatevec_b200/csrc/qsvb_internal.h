@@ -304,6 +304,13 @@ struct qsvb_state {
   mutable std::atomic<bool> shared{false};
 };
 
+namespace qsvb {
+struct SpareState {
+  size_t bytes;  // of either component
+  void *re, *im;
+};
+}  // namespace qsvb
+
 struct qsvb_ctx {
   int device = 0;
   int num_sms = 148;
@@ -321,10 +328,10 @@ struct qsvb_ctx {
   size_t prob_cap = 0;
   char* d_sample = nullptr;       // sampling scratch (sample.cu)
   size_t sample_cap = 0;
-  // Memory of freed states, kept for the next states of the same size (at most kStateKeep bytes in all, so
-  // small states only; returned on destroy and when a larger state needs it): cudaMalloc takes 0.1 to 100 ms
+  // Memory of freed states, oldest first, kept for the next states of the same size (at most kStateKeep bytes
+  // in all, so small states only; returned on destroy and when a larger state needs it): cudaMalloc takes 0.1 to 100 ms
   // on a busy host, as long as a one-shot circuit on such a state. Shared states (qsvb_state::shared) are not kept.
-  std::vector<std::pair<size_t, void*>> spare;
+  std::vector<qsvb::SpareState> spare;
   size_t spare_bytes = 0;
   int* d_err = nullptr;           // device error flag (bounded waits)
   void* h_pin[2] = {nullptr, nullptr};      // pinned host ring for large device -> host copies

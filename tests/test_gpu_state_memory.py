@@ -86,3 +86,33 @@ def test_two_states_never_share_memory(built):
         s.free()
     a.close()
     b.close()
+
+
+def device_free():
+    import torch
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+def test_kept_memory_counts_whole_states(built):
+    """At most 64 MB of freed states are kept, both components of a state or neither, and the most recent sizes."""
+    mb = 1 << 20
+    be = B200Backend(0, precision="f32")
+    before = device_free()
+    be.alloc(24).free()  # two components of 64 MB
+    assert device_free() == before
+    held = [be.alloc(22) for _ in range(2)]  # 32 MB each
+    for s in held:
+        s.free()
+    assert before - device_free() == 64 * mb
+    be.alloc(21).free()  # 16 MB: the older of the two makes room
+    assert before - device_free() == 48 * mb
+    again = be.alloc(21)
+    assert before - device_free() == 48 * mb  # found again
+    again.free()
+    be.alloc(23).free()  # 64 MB: everything else makes room
+    assert before - device_free() == 64 * mb
+    again = be.alloc(23)
+    assert before - device_free() == 64 * mb
+    again.free()
+    be.close()
