@@ -35,12 +35,27 @@ static void drop_spares(qsvb_ctx* c) {
   c->spare_bytes = 0;
 }
 
+bool give_back(qsvb_ctx* c) {
+  if (c->spare.empty() && !c->d_sample) return false;
+  drop_spares(c);
+  if (c->d_sample) cudaFree(c->d_sample);  // (only in use within a call that allocates nothing after it)
+  c->d_sample = nullptr;
+  c->sample_cap = 0;
+  return true;
+}
+
+size_t device_free_bytes(qsvb_ctx* c, double need) {
+  size_t free_b = 0, total_b = 0;
+  QSVB_CK(cudaMemGetInfo(&free_b, &total_b));
+  if (need > double(free_b) && give_back(c)) QSVB_CK(cudaMemGetInfo(&free_b, &total_b));
+  return free_b;
+}
+
 void device_malloc(qsvb_ctx* c, void** p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, bytes);
-  if (e == cudaErrorMemoryAllocation && !c->spare.empty()) {
+  if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
-    drop_spares(c);
-    e = cudaMalloc(p, bytes);
+    if (give_back(c)) e = cudaMalloc(p, bytes);
   }
   QSVB_CK(e);
 }
@@ -389,21 +404,17 @@ int qsvb_state_alloc(qsvb_ctx* c, uint32_t n, int dtype, qsvb_state** out) {
     std::unique_ptr<qsvb_state> s(new qsvb_state{n, dtype, c->device, nullptr, nullptr, c});
     const size_t bytes = state_bytes(s.get());
     if (!take_spare(c, bytes, &s->re, &s->im)) {
-      size_t free_b = 0, total_b = 0;
-      QSVB_CK(cudaMemGetInfo(&free_b, &total_b));
-      if (2 * bytes > free_b && !c->spare.empty()) {
-        drop_spares(c);
-        QSVB_CK(cudaMemGetInfo(&free_b, &total_b));
-      }
+      const size_t free_b = device_free_bytes(c, 2.0 * double(bytes));
       if (2 * bytes > free_b)
         throw Error(QSVB_E_OOM, "state of " + std::to_string(n) + " qubits needs " + std::to_string(2 * bytes) +
                                     " bytes; " + std::to_string(free_b) + " free");
-      cudaError_t e = cudaMalloc(&s->re, bytes);
-      if (e == cudaSuccess) e = cudaMalloc(&s->im, bytes);
-      if (e != cudaSuccess) {
+      try {
+        device_malloc(c, &s->re, bytes);
+        device_malloc(c, &s->im, bytes);
+      } catch (const Error& e) {
         cudaGetLastError();
         if (s->re) cudaFree(s->re);
-        throw Error(QSVB_E_OOM, std::string("state allocation failed: ") + cudaGetErrorString(e));
+        throw Error(QSVB_E_OOM, std::string("state allocation failed: ") + e.what());
       }
     }
     *out = s.release();

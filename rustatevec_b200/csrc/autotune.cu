@@ -178,7 +178,7 @@ extern "C" int qsvb_autotune(qsvb_ctx* c, uint32_t n, int dtype, int reps, uint6
       const size_t mb = sweep_matrix_bytes(s, dtype);
       if (mb > dcap) {
         if (dmat) QSVB_CK(cudaFree(dmat));
-        QSVB_CK(cudaMalloc(&dmat, mb));
+        device_malloc(c, &dmat, mb);
         dcap = mb;
       }
       if (mb) {

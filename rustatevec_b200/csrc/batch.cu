@@ -1994,9 +1994,9 @@ struct qsvb_batch {
 namespace qsvb {
 namespace {
 
-template <class T> void upload_vec(void** dst, const std::vector<T>& v, cudaStream_t s) {
-  QSVB_CK(cudaMalloc(dst, std::max<size_t>(v.size(), 1) * sizeof(T)));
-  if (!v.empty()) QSVB_CK(cudaMemcpyAsync(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s));
+template <class T> void upload_vec(qsvb_ctx* c, void** dst, const std::vector<T>& v) {
+  device_malloc(c, dst, std::max<size_t>(v.size(), 1) * sizeof(T));
+  if (!v.empty()) QSVB_CK(cudaMemcpyAsync(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, c->stream));
 }
 
 template <class R, int RB, int W, int NT> void configure(qsvb_batch* b, qsvb_ctx* c) {
@@ -2062,37 +2062,36 @@ qsvb_batch* batch_create(qsvb_ctx* c, const qsvb_circuit* circuits, size_t n, in
   const bool f64 = dtype == QSVB_C128;
   const size_t rb = f64 ? 8 : 4;
   {
-    size_t free_b = 0, total_b = 0;
-    QSVB_CK(cudaMemGetInfo(&free_b, &total_b));
     const double need = double(bp.state_amps) * 2.0 * double(rb) + double(bp.prob_total) * 8.0 +
                         double(bp.items.size()) * sizeof(Item) + double(bp.passes.size()) * (sizeof(PassDev) + 4) +
                         double(bp.prog.size()) * sizeof(Instr) + double(bp.coef.size()) * 8.0;
+    const size_t free_b = device_free_bytes(c, need);
     if (need > double(free_b))
       throw Error(QSVB_E_OOM, "batch needs " + std::to_string(need / 1e9) + " GB of device memory, " +
                                   std::to_string(double(free_b) / 1e9) + " GB free");
   }
   cudaStream_t s = c->stream;
-  upload_vec(&b->d_items, bp.items, s);
-  upload_vec(&b->d_passes, bp.passes, s);
-  upload_vec(&b->d_phases, bp.phases, s);
-  upload_vec(&b->d_prog, bp.prog, s);
+  upload_vec(c, &b->d_items, bp.items);
+  upload_vec(c, &b->d_passes, bp.passes);
+  upload_vec(c, &b->d_phases, bp.phases);
+  upload_vec(c, &b->d_prog, bp.prog);
   if (f64) {
-    upload_vec(&b->d_coef, bp.coef, s);
+    upload_vec(c, &b->d_coef, bp.coef);
   } else {
     const std::vector<float> cf(bp.coef.begin(), bp.coef.end());
-    upload_vec(&b->d_coef, cf, s);
+    upload_vec(c, &b->d_coef, cf);
     QSVB_CK(cudaStreamSynchronize(s));
   }
-  upload_vec(&b->d_zcnt, bp.zcnt, s);
-  upload_vec(&b->d_zoff, bp.zoff, s);
+  upload_vec(c, &b->d_zcnt, bp.zcnt);
+  upload_vec(c, &b->d_zoff, bp.zoff);
   device_malloc(c, &b->d_sre, std::max<uint64_t>(bp.state_amps, 1) * rb);
   device_malloc(c, &b->d_sim, std::max<uint64_t>(bp.state_amps, 1) * rb);
   device_malloc(c, reinterpret_cast<void**>(&b->d_probs), bp.prob_total * 8);
-  QSVB_CK(cudaMalloc(reinterpret_cast<void**>(&b->d_zpart), bp.zslots * 8));
-  QSVB_CK(cudaMalloc(reinterpret_cast<void**>(&b->d_z0), size_t(bp.ncirc) * 8));
-  QSVB_CK(cudaMalloc(reinterpret_cast<void**>(&b->d_done), bp.passes.size() * 4));
-  QSVB_CK(cudaMalloc(reinterpret_cast<void**>(&b->d_queue), 4));
-  QSVB_CK(cudaMalloc(reinterpret_cast<void**>(&b->d_wait), sizeof(long long)));
+  device_malloc(c, reinterpret_cast<void**>(&b->d_zpart), bp.zslots * 8);
+  device_malloc(c, reinterpret_cast<void**>(&b->d_z0), size_t(bp.ncirc) * 8);
+  device_malloc(c, reinterpret_cast<void**>(&b->d_done), bp.passes.size() * 4);
+  device_malloc(c, reinterpret_cast<void**>(&b->d_queue), 4);
+  device_malloc(c, reinterpret_cast<void**>(&b->d_wait), sizeof(long long));
   {
     const long long budget = kSpinBudget;
     QSVB_CK(cudaMemcpyAsync(b->d_wait, &budget, sizeof(budget), cudaMemcpyHostToDevice, s));
@@ -2103,7 +2102,7 @@ qsvb_batch* batch_create(qsvb_ctx* c, const qsvb_circuit* circuits, size_t n, in
   // QSVB_BATCH_PROFILE=1: per-block cycles spent waiting, filling, in gates and writing out,
   // averaged over blocks and printed to stderr after each run
   if (std::getenv("QSVB_BATCH_PROFILE"))
-    QSVB_CK(cudaMalloc(reinterpret_cast<void**>(&b->d_prof), 5 * 8 * size_t(b->grid)));
+    device_malloc(c, reinterpret_cast<void**>(&b->d_prof), 5 * 8 * size_t(b->grid));
   QSVB_CK(cudaEventCreate(&b->e0));
   QSVB_CK(cudaEventCreate(&b->e1));
   // the per-run device work as one graph: counter resets, the persistent kernel, the <Z_0> sums

@@ -108,7 +108,7 @@ __global__ void k_adam(float* __restrict__ P, const float* __restrict__ g, float
 
 template <class T> struct DevBuf {
   T* p = nullptr;
-  explicit DevBuf(size_t n) { QSVB_CK(cudaMalloc(&p, sizeof(T) * std::max<size_t>(n, 1))); }
+  DevBuf(qsvb_ctx* c, size_t n) { device_malloc(c, reinterpret_cast<void**>(&p), sizeof(T) * std::max<size_t>(n, 1)); }
   ~DevBuf() {
     if (p) cudaFree(p);
   }
@@ -153,7 +153,7 @@ int qsvb_costmodel_forward_backward(qsvb_ctx* c, const float* params, uint32_t h
     QSVB_CK(cudaSetDevice(c->device));
     const int H = int(hidden);
     const size_t np = n_params(H);
-    DevBuf<float> dP(np), dX(n * F), dT(n), dG(n * np), dL(n), dg(np), dl(1);
+    DevBuf<float> dP(c, np), dX(c, n * F), dT(c, n), dG(c, n * np), dL(c, n), dg(c, np), dl(c, 1);
     QSVB_CK(cudaMemcpyAsync(dP.p, params, np * 4, cudaMemcpyHostToDevice, c->stream));
     QSVB_CK(cudaMemcpyAsync(dX.p, X, n * F * 4, cudaMemcpyHostToDevice, c->stream));
     QSVB_CK(cudaMemcpyAsync(dT.p, t, n * 4, cudaMemcpyHostToDevice, c->stream));
@@ -209,7 +209,7 @@ int qsvb_costmodel_train(qsvb_ctx* c, const float* features, const float* log2_s
       T[i] = (log2_seconds[i] - m.y_mean) / m.y_scale;
     }
     std::vector<float> P = init_params(H, seed);
-    DevBuf<float> dP(np), dX(n * F), dT(n), dG(n * np), dL(n), dg(np), dm(np), dv(np), dl(1);
+    DevBuf<float> dP(c, np), dX(c, n * F), dT(c, n), dG(c, n * np), dL(c, n), dg(c, np), dm(c, np), dv(c, np), dl(c, 1);
     QSVB_CK(cudaMemcpyAsync(dP.p, P.data(), np * 4, cudaMemcpyHostToDevice, c->stream));
     QSVB_CK(cudaMemcpyAsync(dX.p, X.data(), n * F * 4, cudaMemcpyHostToDevice, c->stream));
     QSVB_CK(cudaMemcpyAsync(dT.p, T.data(), n * 4, cudaMemcpyHostToDevice, c->stream));

@@ -326,10 +326,10 @@ struct qsvb_ctx {
   size_t exec_mats_cap = 0;
   void* d_prob = nullptr;         // probability staging chunk
   size_t prob_cap = 0;
-  char* d_sample = nullptr;       // sampling scratch (sample.cu)
+  char* d_sample = nullptr;       // sampling scratch (sample.cu), given back likewise
   size_t sample_cap = 0;
   // Memory of freed states, oldest first, kept for the next states of the same size (at most kStateKeep bytes
-  // in all, so small states only; returned on destroy and when a larger state needs it): cudaMalloc takes 0.1 to 100 ms
+  // in all, so small states only; given back on destroy and before any allocation of the context fails): cudaMalloc takes 0.1 to 100 ms
   // on a busy host, as long as a one-shot circuit on such a state. Shared states (qsvb_state::shared) are not kept.
   std::vector<qsvb::SpareState> spare;
   size_t spare_bytes = 0;
@@ -348,7 +348,11 @@ namespace qsvb {
 // straight from `src`.
 constexpr size_t kPinChunk = size_t(64) << 20;
 constexpr size_t kStateKeep = size_t(64) << 20;
-// cudaMalloc that gives the context's spare state buffers back before it fails.
+// Frees what the context keeps for later calls only: states' memory and the sampler's scratch (false: nothing).
+bool give_back(qsvb_ctx* c);
+// Free device memory, counting what the context keeps if `need` bytes are not there without it.
+size_t device_free_bytes(qsvb_ctx* c, double need);
+// cudaMalloc that gives the kept memory back before it fails: every allocation a context makes once it exists.
 void device_malloc(qsvb_ctx* c, void** p, size_t bytes);
 void d2h_staged(qsvb_ctx* c, void* dst, const void* src, size_t bytes);
 void sample_shots(qsvb_ctx* c, const qsvb_state* st, uint64_t shots, uint64_t seed, uint64_t* out);

@@ -116,3 +116,40 @@ def test_kept_memory_counts_whole_states(built):
     assert before - device_free() == 64 * mb
     again.free()
     be.close()
+
+
+def test_kept_memory_is_given_back_before_an_allocation_fails(built):
+    """With the device nearly full, a batch and a state that fit only without the kept states and the sampler's
+    kept scratch. (The kernels run once before, so that loading them needs no memory then.)"""
+    import torch
+    mb = 1 << 20
+    be = B200Backend(0, precision="f32")
+    small = be.alloc(20)
+    be.init_basis(small, 0)
+    be.execute_batch([random_circuit(20, 40, 1)], probabilities=False)
+    be.download(be.execute(random_circuit(24, 1, 1)))
+    circuits = [random_circuit(20, 40, i) for i in range(15)]  # 16 MB each
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+
+    def fill(leave):
+        return torch.empty(device_free() - leave, dtype=torch.uint8, device="cuda")
+
+    be.sample_device(small, 1000000, 1)
+    be.alloc(23).free()
+    full = fill(200 * mb)
+    assert device_free() < 204 * mb
+    z0, _, _ = be.execute_batch(circuits, probabilities=False)
+    del full
+    torch.cuda.empty_cache()
+    assert max_abs_diff(z0, be.execute_batch(circuits, probabilities=False)[0]) == 0
+
+    be.sample_device(small, 1000000, 1)  # keeps between 40 and 64 MB
+    full = fill(100 * mb)
+    state = be.alloc(24)  # 128 MB
+    be.init_basis(state, 3)
+    assert be.amplitude(state, 3) == 1
+    state.free()
+    del full
+    torch.cuda.empty_cache()
+    be.close()
