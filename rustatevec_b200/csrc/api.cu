@@ -60,6 +60,11 @@ void device_malloc(qsvb_ctx* c, void** p, size_t bytes) {
   QSVB_CK(e);
 }
 
+void upload_now(void* dst, const void* src, size_t bytes) {
+  QSVB_CK(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
+  QSVB_CK(cudaStreamSynchronize(cudaStreamLegacy));
+}
+
 namespace {
 
 template <class F> int guarded(F&& f) {
@@ -99,7 +104,7 @@ void check_ctx(const qsvb_ctx* c) { QSVB_REQUIRE(c != nullptr, "null context"); 
 // cleared so the context stays usable).
 void check_flag(qsvb_ctx* c, int flag) {
   if (flag) {
-    QSVB_CK(cudaMemset(c->d_err, 0, sizeof(int)));
+    QSVB_CK(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
     if (flag & kErrBounds)
       throw Error(QSVB_E_CUDA, "a device bounds check failed (an index out of its buffer); results are invalid");
     throw Error(QSVB_E_TIMEOUT, "a device-side wait ran out of its iteration budget; results are invalid");
@@ -253,7 +258,7 @@ qsvb_plan* build_plan(qsvb_ctx* c, const qsvb_circuit* circ, int dtype, const qs
       QSVB_CK(cudaMemcpyAsync(p->d_mats, host.data(), total, cudaMemcpyHostToDevice, c->stream));
     } else {
       device_malloc(c, reinterpret_cast<void**>(&p->d_mats), total);
-      QSVB_CK(cudaMemcpy(p->d_mats, host.data(), total, cudaMemcpyHostToDevice));
+      upload_now(p->d_mats, host.data(), total);
     }
   }
   return p.release();
@@ -343,13 +348,15 @@ int qsvb_create(int device_ordinal, qsvb_ctx** out) {
     std::unique_ptr<qsvb_ctx> c(new qsvb_ctx);
     c->device = device_ordinal;
     c->num_sms = prop.multiProcessorCount;
+    // The stream does not wait for the default one, so whatever its kernels find in device memory is written
+    // on it (a cudaMemset or a pageable cudaMemcpy may return before the device has done it).
     QSVB_CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     QSVB_CK(cudaMalloc(&c->d_partials, reduce_partials_needed(c->num_sms) * sizeof(double)));
-    QSVB_CK(cudaMemset(c->d_partials, 0, reduce_partials_needed(c->num_sms) * sizeof(double)));
+    QSVB_CK(cudaMemsetAsync(c->d_partials, 0, reduce_partials_needed(c->num_sms) * sizeof(double), c->stream));
     QSVB_CK(cudaMalloc(&c->d_result, 3 * sizeof(double)));
     QSVB_CK(cudaHostAlloc(reinterpret_cast<void**>(&c->h_result), 4 * sizeof(double), cudaHostAllocMapped));
     QSVB_CK(cudaMalloc(&c->d_err, sizeof(int)));
-    QSVB_CK(cudaMemset(c->d_err, 0, sizeof(int)));
+    QSVB_CK(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
     *out = c.release();
   });
 }

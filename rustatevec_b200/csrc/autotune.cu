@@ -184,7 +184,7 @@ extern "C" int qsvb_autotune(qsvb_ctx* c, uint32_t n, int dtype, int reps, uint6
       if (mb) {
         host.assign(mb, 0);
         pack_sweep_matrix(s, dtype, host.data());
-        QSVB_CK(cudaMemcpy(dmat, host.data(), mb, cudaMemcpyHostToDevice));
+        upload_now(dmat, host.data(), mb);
       }
       auto run = [&] {
         if (dtype == QSVB_C128)
@@ -209,7 +209,7 @@ extern "C" int qsvb_autotune(qsvb_ctx* c, uint32_t n, int dtype, int reps, uint6
     int flag = 0;
     QSVB_CK(cudaMemcpy(&flag, c->d_err, sizeof(int), cudaMemcpyDeviceToHost));
     if (flag) {
-      QSVB_CK(cudaMemset(c->d_err, 0, sizeof(int)));
+      QSVB_CK(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
       throw Error(QSVB_E_TIMEOUT, "a device-side wait ran out during autotuning");
     }
     return QSVB_OK;

@@ -2154,7 +2154,7 @@ void batch_run(qsvb_ctx* c, qsvb_batch* b, double* z0_out, double* probs_out, co
   int flag = 0;
   QSVB_CK(cudaMemcpy(&flag, c->d_err, sizeof(int), cudaMemcpyDeviceToHost));
   if (flag) {
-    QSVB_CK(cudaMemset(c->d_err, 0, sizeof(int)));
+    QSVB_CK(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
     if (flag & kErrBounds)
       throw Error(QSVB_E_CUDA, "a device bounds check failed (an index out of its buffer); results are invalid");
     throw Error(QSVB_E_TIMEOUT, "a batched-runner dependency wait ran out of its budget; results are invalid");

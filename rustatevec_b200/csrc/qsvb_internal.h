@@ -354,6 +354,9 @@ bool give_back(qsvb_ctx* c);
 size_t device_free_bytes(qsvb_ctx* c, double need);
 // cudaMalloc that gives the kept memory back before it fails: every allocation a context makes once it exists.
 void device_malloc(qsvb_ctx* c, void** p, size_t bytes);
+// Host -> device copy that is on the device when it returns (cudaMemcpy from pageable memory returns once its
+// last part is staged), for memory that kernels on another stream than the default one read next.
+void upload_now(void* dst, const void* src, size_t bytes);
 void d2h_staged(qsvb_ctx* c, void* dst, const void* src, size_t bytes);
 void sample_shots(qsvb_ctx* c, const qsvb_state* st, uint64_t shots, uint64_t seed, uint64_t* out);
 }  // namespace qsvb

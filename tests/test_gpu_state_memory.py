@@ -5,12 +5,12 @@ import threading
 import numpy as np
 import pytest
 
-from rustatevec_b200 import B200Backend
+from rustatevec_b200 import B200Backend, Circuit, DenseGate, Plan
 from rustatevec_b200 import _lib as L
 from rustatevec_b200.circuits import random_circuit
 
 import oracle
-from helpers import max_abs_diff
+from helpers import max_abs_diff, numpy_run
 
 pytestmark = pytest.mark.gpu
 
@@ -153,3 +153,29 @@ def test_kept_memory_is_given_back_before_an_allocation_fails(built):
     del full
     torch.cuda.empty_cache()
     be.close()
+
+
+def test_first_calls_of_a_context_find_their_memory_written(built):
+    """Counters, flags and plan matrices are in place before the context's stream reads them, on memory that held
+    other bits before."""
+    import torch
+    rng = np.random.default_rng(3)
+    for i in range(20):
+        junk = torch.full((64 << 20,), 255, dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        del junk
+        torch.cuda.empty_cache()
+        be = B200Backend(0, precision="f64")
+        s = be.alloc(9)
+        be.init_basis(s, i)
+        assert be.norm_sqr(s) == 1.0 and be.expectation_z(s, 1) == (-1.0 if i & 1 else 1.0)
+        c = Circuit(9)
+        for q in range(4):
+            u = np.linalg.qr(rng.normal(size=(64, 64)) + 1j * rng.normal(size=(64, 64)))[0]
+            c.push(DenseGate(6, u), list(range(q, q + 6)))
+        psi = np.zeros(512, dtype=complex)
+        psi[i] = 1
+        Plan(be, c, L.make_opts(L.PLAN_AS_GIVEN, 6)).run(s)
+        assert max_abs_diff(numpy_run(c, psi), be.download(s).as_complex()) <= 1e-12
+        s.free()
+        be.close()
