@@ -98,12 +98,12 @@ typedef struct qsvb_plan_stats {
   uint64_t n_gates_in;        /* gates in the input circuit */
   uint64_t n_sweeps;          /* sweeps of the plan; a run launches one kernel for each, except for diagonal
                                  sweeps that a dense sweep's kernel carries along */
-  uint64_t n_sweeps_by_kind[10]; /* 1q, ctrl1q, diag, phase, dense CUDA-core, dense TC, tile pass,
+  uint64_t n_sweeps_by_kind[10]; /* of n_sweeps: 1q, ctrl1q, diag, phase, dense CUDA-core, dense TC, tile pass,
                                    other, tensor-core chain pass, tile permutation */
-  double algorithmic_bytes;   /* sum over sweeps of 2 * (amplitudes the sweep may change) * bytes/amp */
-  double full_sweep_bytes;    /* sum over sweeps of 2 * 2^n * bytes/amp */
+  double algorithmic_bytes;   /* sum over launched sweeps of 2 * (amplitudes the sweep may change) * bytes/amp */
+  double full_sweep_bytes;    /* sum over launched sweeps of 2 * 2^n * bytes/amp */
   double flops;               /* complex-MAC flops of the dense sweeps (8 * 2^k per amplitude) */
-  double predicted_seconds;   /* planner's cost-model estimate (0 where nothing is predicted) */
+  double predicted_seconds;   /* cost-model estimate of the launched sweeps (0 where nothing is predicted) */
   double measured_seconds;    /* device seconds measured by the call itself (qsvb_execute_batch*,
                                  qsvb_batch_run); 0 where the call measures nothing */
 } qsvb_plan_stats;

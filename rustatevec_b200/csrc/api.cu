@@ -197,6 +197,14 @@ void run_sweep(qsvb_ctx* c, qsvb_state* st, const Sweep& s, const void* dev_mat,
   c->reverse = !c->reverse;
 }
 
+// The sweeps of a plan as they will run.
+std::vector<Sweep> final_sweeps(const qsvb_circuit* circ, const qsvb_plan_opts& o, int dtype) {
+  std::vector<Sweep> sw = plan_sweeps(gates_from_circuit(circ), circ->n_qubits, o, dtype);
+  // (as given: one sweep per gate, in order)
+  if (o.planner != QSVB_PLAN_AS_GIVEN) attach_diagonals(sw, circ->n_qubits);
+  return sw;
+}
+
 // exec_block: the plan is run once and freed by the caller before the context's next call (one-shot
 // execute); its matrices then go into the context's reusable block instead of an allocation of
 // their own, so a one-shot call allocates and frees nothing on the device once the block is large
@@ -209,14 +217,9 @@ qsvb_plan* build_plan(qsvb_ctx* c, const qsvb_circuit* circ, int dtype, const qs
   p->n_qubits = circ->n_qubits;
   p->dtype = dtype;
   p->opts = opts ? *opts : default_opts();
-  p->sweeps = plan_sweeps(gates_from_circuit(circ), circ->n_qubits, p->opts, dtype);
+  p->sweeps = final_sweeps(circ, p->opts, dtype);
   p->stats.n_gates_in = circ->n_gates;
   sweep_costs(p->sweeps, circ->n_qubits, dtype, &p->stats);
-  // (as given: one sweep per gate, in order)
-  if (p->opts.planner != QSVB_PLAN_AS_GIVEN) {
-    p->stats.predicted_seconds = predict_plan_seconds(p->sweeps, circ->n_qubits, dtype, true);
-    attach_diagonals(p->sweeps, circ->n_qubits);
-  }
   // one device block holding every sweep's matrix, uploaded once
   size_t total = 0;
   for (const Sweep& s : p->sweeps) {
@@ -640,7 +643,7 @@ int qsvb_plan_dry_run(const qsvb_circuit* circ, int dtype, const qsvb_plan_opts*
     QSVB_REQUIRE(dtype == QSVB_C64 || dtype == QSVB_C128, "dtype must be QSVB_C64 or QSVB_C128");
     QSVB_REQUIRE(stats != nullptr, "null output");
     const qsvb_plan_opts o = opts ? *opts : default_opts();
-    const std::vector<Sweep> sw = plan_sweeps(gates_from_circuit(circ), circ->n_qubits, o, dtype);
+    const std::vector<Sweep> sw = final_sweeps(circ, o, dtype);
     *stats = qsvb_plan_stats{};
     stats->n_gates_in = circ->n_gates;
     sweep_costs(sw, circ->n_qubits, dtype, stats);

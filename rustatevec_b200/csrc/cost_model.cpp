@@ -258,7 +258,7 @@ double predict_plan_seconds(const std::vector<Sweep>& sw, uint32_t n, int dtype,
   if (carry) carried = carried_diagonals(sw, n);
   double t = 0;
   for (size_t i = 0; i < sw.size(); ++i)
-    if (!carry || !carried[i]) t += predict_sweep_seconds(sw[i], n, dtype);
+    if (!sw[i].carried && !(carry && carried[i])) t += predict_sweep_seconds(sw[i], n, dtype);
   return t;
 }
 

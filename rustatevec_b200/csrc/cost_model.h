@@ -16,7 +16,7 @@ void sweep_features(const Sweep& s, uint32_t n, int dtype, float* out);
 double analytic_sweep_seconds(const Sweep& s, uint32_t n, int dtype);
 // MLP estimate when a trained model is installed, else the analytic estimate.
 double predict_sweep_seconds(const Sweep& s, uint32_t n, int dtype);
-// carry: the diagonals that dense sweeps will carry (attach_diagonals) cost nothing
+// Diagonals that dense sweeps carry cost nothing; carry: so do those that attach_diagonals will let them carry
 double predict_plan_seconds(const std::vector<Sweep>& sw, uint32_t n, int dtype, bool carry = false);
 
 // Kernel choice for dense sweeps (CUDA cores vs tensor cores), shared by the planner and the

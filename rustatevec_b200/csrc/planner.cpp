@@ -804,6 +804,7 @@ void sweep_costs(const std::vector<Sweep>& sw, uint32_t n, int dtype, qsvb_plan_
   for (const Sweep& s : sw) {
     int kind = s.kind;
     st->n_sweeps_by_kind[kind < kNumSweepKinds ? kind : 7]++;
+    if (s.carried) continue;  // (not run by itself)
     double amps = dim;
     if (s.kind == SK_CTRL) amps = std::ldexp(dim, -int(s.nctrl));
     if (s.kind == SK_DIAG) amps = std::ldexp(dim, -int(s.nctrl));

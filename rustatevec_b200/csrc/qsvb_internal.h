@@ -181,8 +181,8 @@ template <class F> void parallel_ranges(size_t n, size_t min_items, F&& fn) {
 // Tensor-core chain passes with qubit relabelling, then the permutation passes that restore every
 // qubit to its own state bit (chain_planner.cpp). max_mats: matrices per pass (1..3).
 std::vector<Sweep> plan_chain(const std::vector<Gate>& in, uint32_t n, uint32_t max_mats);
-// Lets dense sweeps carry diagonal sweeps in their write-back (Sweep::tail); the list of sweeps and
-// their costs stay as planned.
+// Lets dense sweeps carry diagonal sweeps in their write-back (Sweep::tail); the list of sweeps stays as
+// planned, but the carried ones no longer count in sweep_costs' bytes and seconds.
 void attach_diagonals(std::vector<Sweep>& sw, uint32_t n);
 // Which sweeps attach_diagonals would have carried (sweeps without matrices will do).
 std::vector<char> carried_diagonals(const std::vector<Sweep>& sw, uint32_t n);

@@ -112,3 +112,13 @@ def test_diagonal_carried_by_a_dense_sweep(be64, be32, precision, k, n):
         err = max_abs_diff(numpy_run(c, psi), be.download(st).as_complex())
         assert err <= (2 ** (k + 1) + 2 ** 3 + 20) * UNIT[precision], (qs, m, err)
     st.free()
+
+
+@pytest.mark.parametrize("planner", [L.PLAN_GREEDY, L.PLAN_WINDOW, L.PLAN_LEARNED, PLAN_AS_GIVEN])
+def test_dry_run_reports_what_the_plan_reports(be32, planner):
+    import ctypes as C
+    from rustatevec_b200.circuits import brickwork
+    c, opts = brickwork(22, 4, 1), L.make_opts(planner, 4, ENGINE_CUDA_CORE)
+    pc, st = L.PackedCircuit(c), L.PlanStats()
+    L.check(L.lib().qsvb_plan_dry_run(pc.ref(), be32.dtype, C.byref(opts), C.byref(st)))
+    assert Plan(be32, c, opts).stats() == st.to_dict()

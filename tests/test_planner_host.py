@@ -98,3 +98,26 @@ def test_chain_planner_passes(built):
     assert "tc_chain" not in dry(c, L.PLAN_CHAIN, 6, dtype=L.C128)["by_kind"]
     assert "tc_chain" not in dry(random_circuit(11, 60, 1), L.PLAN_CHAIN, 6)["by_kind"]
     assert "tc_chain" not in dry(c, L.PLAN_CHAIN, 6, engine=L.ENGINE_CUDA_CORE)["by_kind"]
+
+
+@pytest.mark.parametrize("dtype", [L.C64, L.C128])
+def test_carried_diagonals_cost_nothing(built, dtype):
+    """A diagonal that a dense sweep carries along (on its own qubits, or on others) is a sweep of the plan but
+    adds no bytes and no seconds; as given, it runs by itself."""
+    import numpy as np
+    from rustatevec_b200 import Circuit, DenseGate
+    z = np.linalg.qr(np.random.default_rng(0).normal(size=(8, 8)))[0]
+    dense = Circuit(20)
+    dense.push(DenseGate(3, z), [1, 4, 9])
+    alone = dry(dense, L.PLAN_GREEDY, 1, dtype)
+    for qs in ([1, 4], [2, 15], [4, 19]):
+        both = Circuit(20)
+        both.push(DenseGate(3, z), [1, 4, 9])
+        both.push(DenseGate(2, np.diag(np.exp(1j * np.arange(4)))), qs)
+        st = dry(both, L.PLAN_GREEDY, 1, dtype)
+        assert st["by_kind"] == {"dense": 1, "diag": 1} and st["n_sweeps"] == 2
+        for key in ("algorithmic_bytes", "full_sweep_bytes", "flops", "predicted_seconds"):
+            assert st[key] == alone[key], key
+        given = dry(both, L.PLAN_AS_GIVEN, 1, dtype)
+        assert given["algorithmic_bytes"] == 2 * alone["algorithmic_bytes"]
+        assert given["predicted_seconds"] > alone["predicted_seconds"]
