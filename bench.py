@@ -333,6 +333,8 @@ def run_gpu(args):
         per = hp.profile(state, reps=2)
         by_kind = {}
         for s, t in zip(sweeps, per):
+            if s["carried"]:
+                continue
             d = by_kind.setdefault(s["kind"], {"time": 0.0, "bytes": 0.0, "flops": 0.0, "launches": 0})
             d["time"] += t
             d["bytes"] += s["algorithmic_bytes"]
@@ -374,7 +376,7 @@ def run_gpu(args):
             cpu["lscpu"] = lscpu_summary()
             if not args.no_cpu_scaling:
                 cpu["full_circuit_seconds"] = cpu_full_circuits()
-        n_launch = args.steps * (hst["n_sweeps"] + 1)
+        n_launch = args.steps * (hp.launches() + 1)
         out = {
             "metric": METRIC, "value": round(t_step, 6), "unit": "s", "n_gpus": world,
             "circuits_per_second": round(world / t_step, 3),
@@ -465,6 +467,8 @@ def plan_roofline(plan, state, reps=1):
     per = plan.profile(state, reps=reps)
     by_kind = {}
     for s, t in zip(sweeps, per):
+        if s["carried"]:
+            continue
         d = by_kind.setdefault(s["kind"], {"time": 0.0, "bytes": 0.0, "launches": 0})
         d["time"] += t
         d["bytes"] += s["algorithmic_bytes"]
@@ -533,7 +537,7 @@ def run_config_ghz24(args):
           {"workload": "GHZ chain H(0), CX(i,i+1), 24 qubits, complex128", "plan_sweeps":
            plans["learned"].stats()["n_sweeps"], "l2": "256 MiB state (> L2)"},
           methods_seconds={k: round(v, 7) for k, v in secs.items()}, known_answer_ok=bool(ok),
-          roofline=rl, cpu_baseline=cpu, clocks=clk, gpu_launches=args.steps * (plans["learned"].stats()["n_sweeps"] + 1),
+          roofline=rl, cpu_baseline=cpu, clocks=clk, gpu_launches=args.steps * (plans["learned"].launches() + 1),
           e2e={"value": round(e2e, 6), "unit": "s", "h2d_bytes_per_step": sum(32 * (1 << (2 * len(o.qubits))) // 2 for o in circ.ops()),
                "d2h_bytes_per_step": 8 << n, "path": "run(host circuit) + probabilities(fp64) download"})
     st.free()
@@ -602,7 +606,7 @@ def run_config_qft32(args):
           methods_seconds={k: round(v, 5) for k, v in secs.items()}, infidelity_vs_fp64=fids,
           speedup_learned_vs_greedy_k5=round(secs["greedy_k5"] / t, 3),
           speedup_learned_vs_unfused=round(secs["unfused"] / t, 3),
-          roofline=rl, cpu_baseline=cpu, clocks=clk, gpu_launches=args.steps * (plans["learned"].stats()["n_sweeps"] + 3),
+          roofline=rl, cpu_baseline=cpu, clocks=clk, gpu_launches=args.steps * (plans["learned"].launches() + 3),
           e2e={"value": round(e2e, 6), "unit": "s", "h2d_bytes_per_step": sum(16 << (2 * len(o.qubits)) for o in circ.ops()),
                "d2h_bytes_per_step": 8, "path": "init_gaussian + run(host circuit) + expectation_z(mask=1)",
                "z0": z})
@@ -651,7 +655,7 @@ def run_config_qaoa33(args):
                            "max_abs_diff_learned_vs_greedy": diff, "z_masks": masks, "z_learned": l["z"]},
           roofline=rl, cpu_baseline={"value": None, "unit": "s", "cores": None, "kind": "port",
                                      "sample": "not run (RAM): the 137 GB state does not fit the host"},
-          clocks=clk, gpu_launches=max(1, args.steps // 2) * (plans["learned"].stats()["n_sweeps"] + 1),
+          clocks=clk, gpu_launches=max(1, args.steps // 2) * (plans["learned"].launches() + 1),
           e2e={"value": None, "unit": "s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0,
                "note": "device-resident workload; see value"})
     st.free()
@@ -863,7 +867,7 @@ def run_kernel_case(args):
     nbytes = sum(s["algorithmic_bytes"] for s in info)
     peak, kind = peaks()
     print(json.dumps({"kernel_case": args.kernel_case, "qubits": n, "precision": prec, "input": args.input,
-                      "sweeps": [s["kind"] for s in info], "us_per_launch": round(t * 1e6, 2),
+                      "sweeps": [s["kind"] for s in info if not s["carried"]], "us_per_launch": round(t * 1e6, 2),
                       "algorithmic_bytes": nbytes, "GB/s": round(nbytes / t / 1e9, 1),
                       "frac_of_peak": round(nbytes / t / 1e9 / peak, 4), "peak": f"{peak} ({kind})"}))
 

@@ -90,7 +90,8 @@ typedef struct qsvb_plan_opts {
   uint32_t engine;           /* qsvb_engine */
   uint32_t use_graph;        /* reusable plans: capture the sweep sequence in a CUDA graph */
   uint32_t chain_max_matrices; /* QSVB_PLAN_CHAIN: matrices per pass, 1..3 (0: chosen by cost) */
-  uint32_t reserved[3];
+  uint32_t diagonals_apart;  /* not 0: every diagonal sweep runs by itself (0: dense sweeps carry those they can) */
+  uint32_t reserved[2];
 } qsvb_plan_opts;
 
 /* What a plan does, for reports and rooflines. */
@@ -163,6 +164,8 @@ typedef struct qsvb_sweep_info {
   uint32_t n_ctrl;                /* controls (ctrl1q) or skipped identity halves (diag) */
   uint32_t ctrl[QSVB_MAX_GATE_QUBITS];
   uint32_t n_terms;               /* phase polynomial terms */
+  uint32_t carried;               /* 1: a diagonal that a dense sweep's kernel applies, not launched by itself (its
+                                     bytes, flops and profiled time are 0) */
   uint64_t n_gates;               /* input gates this sweep covers */
   double algorithmic_bytes;       /* 2 * (amplitudes it may change) * bytes per amplitude */
   double flops;                   /* 8 * 2^k per amplitude for dense sweeps */
@@ -170,7 +173,8 @@ typedef struct qsvb_sweep_info {
 } qsvb_sweep_info;
 int qsvb_plan_sweep_info(const qsvb_plan* plan, size_t index, qsvb_sweep_info* out);
 /* Device time of each sweep of `plan` on `st`: CUDA events around `reps` back-to-back launches of
- * each sweep; out_seconds[i] = mean seconds per launch of sweep i. The state is overwritten. */
+ * each sweep as a run launches it, carried diagonals included; out_seconds[i] = mean seconds per launch of
+ * sweep i (0: carried by another). The state is overwritten. */
 int qsvb_plan_profile(qsvb_ctx* ctx, qsvb_plan* plan, qsvb_state* st, int reps, double* out_seconds);
 /* Fused gate list a planner produces (crates/qsv-core/src/fusion.rs:39 fuse). Call with
  * out_gates == NULL to get the count in *n_out; matrices are written to out_mats (FP64

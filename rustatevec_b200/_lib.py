@@ -48,7 +48,8 @@ class CircuitS(C.Structure):
 
 class PlanOpts(C.Structure):
     _fields_ = [("planner", C.c_uint32), ("max_fused_qubits", C.c_uint32), ("engine", C.c_uint32),
-                ("use_graph", C.c_uint32), ("chain_max_matrices", C.c_uint32), ("reserved", C.c_uint32 * 3)]
+                ("use_graph", C.c_uint32), ("chain_max_matrices", C.c_uint32),
+                ("diagonals_apart", C.c_uint32), ("reserved", C.c_uint32 * 2)]
 
 
 class PlanStats(C.Structure):
@@ -71,14 +72,14 @@ class PlanStats(C.Structure):
 class SweepInfo(C.Structure):
     _fields_ = [("kind", C.c_uint32), ("n_qubits", C.c_uint32), ("qubits", C.c_uint32 * MAX_GATE_QUBITS),
                 ("target", C.c_uint32), ("n_ctrl", C.c_uint32), ("ctrl", C.c_uint32 * MAX_GATE_QUBITS),
-                ("n_terms", C.c_uint32), ("n_gates", C.c_uint64), ("algorithmic_bytes", C.c_double),
+                ("n_terms", C.c_uint32), ("carried", C.c_uint32), ("n_gates", C.c_uint64), ("algorithmic_bytes", C.c_double),
                 ("flops", C.c_double), ("features", C.c_float * 16)]
 
     def to_dict(self) -> dict:
         return {"kind": SWEEP_KINDS[self.kind], "k": int(self.n_qubits),
                 "qubits": [int(self.qubits[j]) for j in range(self.n_qubits)],
                 "target": int(self.target), "ctrl": [int(self.ctrl[j]) for j in range(self.n_ctrl)],
-                "n_terms": int(self.n_terms), "n_gates": int(self.n_gates),
+                "n_terms": int(self.n_terms), "carried": bool(self.carried), "n_gates": int(self.n_gates),
                 "algorithmic_bytes": float(self.algorithmic_bytes), "flops": float(self.flops),
                 "features": [float(x) for x in self.features]}
 

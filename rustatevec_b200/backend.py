@@ -265,6 +265,10 @@ class Plan:
         L.check(L.lib().qsvb_plan_stats_get(self.handle, C.byref(st)))
         return st.to_dict()
 
+    def launches(self) -> int:
+        """Kernels a run launches: the sweeps that no other sweep carries."""
+        return sum(not s["carried"] for s in self.sweeps())
+
     def sweeps(self) -> list:
         out = []
         for i in range(self.stats()["n_sweeps"]):
@@ -274,7 +278,7 @@ class Plan:
         return out
 
     def profile(self, state: DeviceState, reps: int = 3) -> np.ndarray:
-        """Mean device seconds per launch of each sweep (CUDA events, native)."""
+        """Mean device seconds per launch of each sweep (CUDA events, native); 0 for carried ones."""
         n = self.stats()["n_sweeps"]
         out = np.zeros(max(n, 1), dtype=np.float64)
         L.check(L.lib().qsvb_plan_profile(self.backend.ctx, self.handle, state.handle, reps,

@@ -201,7 +201,7 @@ void run_sweep(qsvb_ctx* c, qsvb_state* st, const Sweep& s, const void* dev_mat,
 std::vector<Sweep> final_sweeps(const qsvb_circuit* circ, const qsvb_plan_opts& o, int dtype) {
   std::vector<Sweep> sw = plan_sweeps(gates_from_circuit(circ), circ->n_qubits, o, dtype);
   // (as given: one sweep per gate, in order)
-  if (o.planner != QSVB_PLAN_AS_GIVEN) attach_diagonals(sw, circ->n_qubits);
+  if (o.planner != QSVB_PLAN_AS_GIVEN && !o.diagonals_apart) attach_diagonals(sw, circ->n_qubits);
   return sw;
 }
 
@@ -565,6 +565,7 @@ int qsvb_plan_sweep_info(const qsvb_plan* p, size_t i, qsvb_sweep_info* out) {
     out->target = s.target;
     out->n_ctrl = s.nctrl;
     out->n_terms = uint32_t(s.terms.size());
+    out->carried = s.carried;
     out->n_gates = s.n_gates;
     if (s.kind == SK_TC_CHAIN || s.kind == SK_PERMUTE) {
       out->n_qubits = s.chain_nmat;
@@ -591,9 +592,11 @@ int qsvb_plan_profile(qsvb_ctx* c, qsvb_plan* p, qsvb_state* s, int reps, double
     try {
       for (size_t i = 0; i < p->sweeps.size(); ++i) {
         const void* m = sweep_matrix_bytes(p->sweeps[i], p->dtype) ? p->d_mats + p->mat_offset[i] : nullptr;
-        run_sweep(c, s, p->sweeps[i], m);  // warm-up launch
+        out[i] = 0.0;
+        if (p->sweeps[i].carried) continue;
+        run_sweep(c, s, p->sweeps[i], m, true);  // warm-up launch
         QSVB_CK(cudaEventRecord(e0, c->stream));
-        for (int r = 0; r < reps; ++r) run_sweep(c, s, p->sweeps[i], m);
+        for (int r = 0; r < reps; ++r) run_sweep(c, s, p->sweeps[i], m, true);
         QSVB_CK(cudaEventRecord(e1, c->stream));
         QSVB_CK(cudaEventSynchronize(e1));
         float ms = 0;

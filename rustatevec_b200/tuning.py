@@ -56,7 +56,9 @@ def plan_records(backend, n_qubits: int, reps: int = 2, seed: int = 0) -> dict:
             for planner in (L.PLAN_GREEDY, L.PLAN_WINDOW):
                 for k in (2, 4, 6):
                     for eng in engines:
-                        p = Plan(backend, circ, L.make_opts(planner, k, eng, use_graph=False))
+                        opts = L.make_opts(planner, k, eng, use_graph=False)
+                        opts.diagonals_apart = 1  # the model predicts each sweep by itself
+                        p = Plan(backend, circ, opts)
                         info = p.sweeps()
                         t = p.profile(st, reps)
                         for s, sec in zip(info, t):

@@ -122,3 +122,30 @@ def test_dry_run_reports_what_the_plan_reports(be32, planner):
     pc, st = L.PackedCircuit(c), L.PlanStats()
     L.check(L.lib().qsvb_plan_dry_run(pc.ref(), be32.dtype, C.byref(opts), C.byref(st)))
     assert Plan(be32, c, opts).stats() == st.to_dict()
+
+
+def test_profile_runs_what_the_plan_runs(be64):
+    """A carried diagonal is marked, takes no time of its own and is part of its dense sweep's: profiling launches
+    every sweep twice (reps = 1 and a warm-up), which for one launched sweep is two runs of the plan."""
+    rng = np.random.default_rng(2)
+    n = 11
+    c = Circuit(n)
+    c.push(G.DenseGate(3, unitary(3, rng)), [2, 5, 6])
+    c.push(G.DenseGate(2, diagonal(2, rng)), [5, 9])
+    psi = rng.normal(size=1 << n) + 1j * rng.normal(size=1 << n)
+    apart = L.make_opts(PLAN_GREEDY, 1)
+    apart.diagonals_apart = 1
+    st = be64.alloc(n)
+    got = []
+    for opts in (L.make_opts(PLAN_GREEDY, 1), apart):
+        plan = Plan(be64, c, opts)
+        for step in (lambda: plan.profile(st, 1), lambda: (plan.run(st), plan.run(st))):
+            be64.upload(st, psi.real, psi.imag)
+            secs = step()
+            got.append((be64.download(st).as_complex(), secs, [s["carried"] for s in plan.sweeps()], plan.launches()))
+    (prof, secs, carried, launches), (runs, *_), (prof_apart, secs_apart, carried_apart, two), (runs_apart, *_) = got
+    assert carried == [False, True] and launches == 1 and secs[0] > 0 and secs[1] == 0
+    assert carried_apart == [False, False] and two == 2 and (secs_apart > 0).all()
+    assert np.array_equal(prof, runs) and np.array_equal(runs, runs_apart)
+    assert not np.array_equal(prof_apart, runs_apart)  # (there the dense sweep ran twice, then the diagonal)
+    st.free()

@@ -121,3 +121,8 @@ def test_carried_diagonals_cost_nothing(built, dtype):
         given = dry(both, L.PLAN_AS_GIVEN, 1, dtype)
         assert given["algorithmic_bytes"] == 2 * alone["algorithmic_bytes"]
         assert given["predicted_seconds"] > alone["predicted_seconds"]
+    apart, st = L.make_opts(L.PLAN_GREEDY, 1), L.PlanStats()
+    apart.diagonals_apart = 1
+    pc = L.PackedCircuit(both)
+    L.check(L.lib().qsvb_plan_dry_run(pc.ref(), dtype, C.byref(apart), C.byref(st)))
+    assert st.to_dict() == given
