@@ -768,7 +768,6 @@ __global__ void __launch_bounds__(NT, MINB)
             R* __restrict__ sre, R* __restrict__ sim, double* __restrict__ probs, double* __restrict__ zpart,
             uint32_t* __restrict__ done, uint32_t* __restrict__ queue, int* __restrict__ err, uint32_t lbits,
             long long* __restrict__ prof, uint32_t fixed, const long long* __restrict__ wait_budget) {
-  if (!TILE || (fixed & 4u)) early_next();
   extern __shared__ __align__(16) uint8_t smem_raw[];
   R* xr = reinterpret_cast<R*>(smem_raw);
   const uint32_t cap = TILE ? uint32_t(HI) << W : 1u << lbits;  // every pass has nlocal <= lbits
@@ -793,11 +792,10 @@ __global__ void __launch_bounds__(NT, MINB)
       if ((h >> i) & 1u) v ^= swz_col(W + i, W);
     if (QSVB_BC(h < uint32_t(HI), err)) s_swz[h] = uint16_t(v);
   }
-  wait_prior();
   long long t_wait = 0, t_fill = 0, t_gates = 0, t_out = 0, n_items = 0, t_mark = prof ? clock64() : 0;
   uint32_t staged_pass = ~0u;
   // fixed != 0: one pass (passes[0]) over one state, tile i (bit 1: from the last one) handled by block i mod
-  // grid, no queue (bit 2: launched programmatically)
+  // grid, no queue
   uint32_t iter = 0;
   while (true) {
     if (!fixed && tid == 0) s_item = atomicAdd(queue, 1u);
@@ -2264,17 +2262,16 @@ void launch_tile_variant(const LaunchEnv& e, R* re, R* im, const Sweep& s, const
   QSVB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, NT, smem));
   QSVB_REQUIRE(occ >= 1, "tile kernel does not fit on an SM");
   const uint32_t grid = uint32_t(std::min<uint64_t>(s.tile_ntiles, uint64_t(e.num_sms) * uint64_t(occ)));
-  // Programmatic on both sides only while every SM gets one block. These blocks need all of an SM's memory as
-  // shared memory, and an SM changes its split only when it is idle: started among the last blocks of a sweep
-  // with another split, fewer of them fit and the rest run as a second wave (26 qubits, complex128: a GHZ
-  // tile pass 1.04 against 0.75 ms, that pass and a five-qubit dense sweep in turn 2.17 against 1.36 ms).
-  const bool early = s.tile_ntiles <= uint32_t(e.num_sms);
-  launch_pdl_if(early, fn, grid, NT, smem, e.stream, static_cast<const Item*>(nullptr), s.tile_ntiles,
-             reinterpret_cast<const PassDev*>(base), reinterpret_cast<const PhaseDev*>(base + s.tile_off_phase),
-             reinterpret_cast<const Instr*>(base + s.tile_off_prog), reinterpret_cast<const R*>(base + s.tile_off_coef),
-             re, im, static_cast<double*>(nullptr), static_cast<double*>(nullptr), static_cast<uint32_t*>(nullptr),
-             static_cast<uint32_t*>(nullptr), e.err_flag, s.tile_lbits, static_cast<long long*>(nullptr), (e.reverse ? 2u : 1u) | (early ? 4u : 0u),
-             static_cast<const long long*>(nullptr));
+  // Launched ordinarily on both sides: these blocks need all of an SM's memory as shared memory, and an SM
+  // changes its split only when it is idle. Started among the last blocks of a sweep with another split, fewer
+  // of them fit and the rest run as a second wave (26 qubits, complex128: a GHZ tile pass 1.04 against 0.75 ms,
+  // that pass and a five-qubit dense sweep in turn 2.17 against 1.36 ms).
+  fn<<<grid, NT, smem, e.stream>>>(nullptr, s.tile_ntiles, reinterpret_cast<const PassDev*>(base),
+                                   reinterpret_cast<const PhaseDev*>(base + s.tile_off_phase),
+                                   reinterpret_cast<const Instr*>(base + s.tile_off_prog),
+                                   reinterpret_cast<const R*>(base + s.tile_off_coef), re, im, nullptr, nullptr,
+                                   nullptr, nullptr, e.err_flag, s.tile_lbits, nullptr, e.reverse ? 2u : 1u, nullptr);
+  QSVB_CK(cudaGetLastError());
 }
 }  // namespace
 

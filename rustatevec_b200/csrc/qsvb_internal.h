@@ -268,10 +268,9 @@ namespace qsvb {
 __device__ __forceinline__ void early_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_prior() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Launches a kernel that calls early_next and wait_prior (see there); programmatic = false: an ordinary launch.
+// Launches a kernel that calls early_next and wait_prior (see there).
 template <class... P, class... A>
-void launch_pdl_if(bool programmatic, void (*kern)(P...), unsigned grid, unsigned block, size_t smem,
-                   cudaStream_t stream, A&&... args) {
+void launch_pdl(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, A&&... args) {
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
@@ -281,12 +280,8 @@ void launch_pdl_if(bool programmatic, void (*kern)(P...), unsigned grid, unsigne
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cfg.attrs = &attr;
-  cfg.numAttrs = programmatic ? 1 : 0;
+  cfg.numAttrs = 1;
   QSVB_CK(cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...));
-}
-template <class... P, class... A>
-void launch_pdl(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, A&&... args) {
-  launch_pdl_if(true, kern, grid, block, smem, stream, std::forward<A>(args)...);
 }
 #endif
 }  // namespace qsvb
