@@ -190,9 +190,10 @@ void* ring_upload(qsvb_ctx* c, const void* src, size_t bytes) {
 }
 
 void run_sweep(qsvb_ctx* c, qsvb_state* st, const Sweep& s, const void* dev_mat, bool tail = false) {
+  const LaunchEnv env = c->next_env(st->n_qubits - s.nctrl, s.kind == SK_DENSE_TC || s.kind == SK_TC_CHAIN);
   by_dtype(st->dtype, [&](auto r) {
     using R = decltype(r);
-    launch_sweep<R>(c->env(), static_cast<R*>(st->re), static_cast<R*>(st->im), st->n_qubits, s, dev_mat, tail);
+    launch_sweep<R>(env, static_cast<R*>(st->re), static_cast<R*>(st->im), st->n_qubits, s, dev_mat, tail);
   });
   c->reverse = !c->reverse;
 }
@@ -316,7 +317,7 @@ void free_plan(qsvb_plan* p) {
 double reduce(qsvb_ctx* c, int op, const qsvb_state* a, const qsvb_state* b, uint64_t mask, double* second) {
   by_dtype(a->dtype, [&](auto r) {
     using R = decltype(r);
-    launch_reduce<R>(c->env(), op, static_cast<const R*>(a->re), static_cast<const R*>(a->im),
+    launch_reduce<R>(c->next_env(a->n_qubits), op, static_cast<const R*>(a->re), static_cast<const R*>(a->im),
                      b ? static_cast<const R*>(b->re) : nullptr, b ? static_cast<const R*>(b->im) : nullptr,
                      a->n_qubits, mask, c->d_partials, c->h_result);
   });
@@ -468,7 +469,7 @@ int qsvb_init_basis(qsvb_ctx* c, qsvb_state* s, uint64_t basis) {
     DeviceGuard dg(c->device);
     by_dtype(s->dtype, [&](auto r) {
       using R = decltype(r);
-      launch_init_basis<R>(c->env(), static_cast<R*>(s->re), static_cast<R*>(s->im), s->n_qubits, basis);
+      launch_init_basis<R>(c->next_env(s->n_qubits), static_cast<R*>(s->re), static_cast<R*>(s->im), s->n_qubits, basis);
     });
   });
 }
@@ -493,7 +494,7 @@ int qsvb_init_gaussian(qsvb_ctx* c, qsvb_state* s, uint64_t seed) {
       using R = decltype(r);
       R* re = static_cast<R*>(s->re);
       R* im = static_cast<R*>(s->im);
-      launch_init_gaussian<R>(c->env(), re, im, s->n_qubits, seed);
+      launch_init_gaussian<R>(c->next_env(s->n_qubits), re, im, s->n_qubits, seed);
       launch_reduce<R>(c->env(), RED_NORM, re, im, nullptr, nullptr, s->n_qubits, 0, c->d_partials, c->d_result);
       launch_scale<R>(c->env(), re, im, s->n_qubits, c->d_result);
     });
@@ -855,11 +856,11 @@ int qsvb_inner_product(qsvb_ctx* c, const qsvb_state* a, const qsvb_state* b, do
     }
     // mixed precision: complex64 against complex128, accumulated in FP64
     if (a->dtype == QSVB_C64)
-      launch_inner_mixed<float, double>(c->env(), static_cast<const float*>(a->re), static_cast<const float*>(a->im),
+      launch_inner_mixed<float, double>(c->next_env(a->n_qubits), static_cast<const float*>(a->re), static_cast<const float*>(a->im),
                                         static_cast<const double*>(b->re), static_cast<const double*>(b->im),
                                         a->n_qubits, c->d_partials, c->h_result);
     else
-      launch_inner_mixed<double, float>(c->env(), static_cast<const double*>(a->re), static_cast<const double*>(a->im),
+      launch_inner_mixed<double, float>(c->next_env(a->n_qubits), static_cast<const double*>(a->re), static_cast<const double*>(a->im),
                                         static_cast<const float*>(b->re), static_cast<const float*>(b->im),
                                         a->n_qubits, c->d_partials, c->h_result);
     wait_result(c, out);  // also reports a failure flagged by earlier device work

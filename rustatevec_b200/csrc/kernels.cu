@@ -1121,25 +1121,25 @@ void launch_pair(const LaunchEnv& env, R* re, R* im, uint32_t n, uint32_t t, con
       const uint64_t set = split(LOG, fixed, low);
       const uint64_t nwork = 1ull << (n - LOG - fixed.size());
       auto kern = t == 0 ? k_pair_invec<R, 0> : k_pair_invec<R, LOG - 1>;  // LOG is 1 or 2
-      launch_pdl(kern, grid_for(nwork, kThreads, env.num_sms), kThreads, 0, env.stream, re, im, nwork,
+      launch_pdl(kern, grid_for(nwork, kThreads, env.num_sms), kThreads, 0, env, re, im, nwork,
                  make_enum(fixed, set, env.flip(nwork)), low, g);
     } else if (t < LOG + 5) {
       const uint64_t set = split(LOG + 5, fixed, low);
       const uint64_t nwork = 1ull << (n - LOG - 5 - fixed.size());
-      launch_pdl(k_pair_shfl<R>, grid_for(nwork * 32, kThreads, env.num_sms), kThreads, 0, env.stream,
+      launch_pdl(k_pair_shfl<R>, grid_for(nwork * 32, kThreads, env.num_sms), kThreads, 0, env,
           re, im, nwork, make_enum(fixed, set, env.flip(nwork)), t, low, g);
     } else {
       const uint64_t set = split(LOG, fixed, low);
       fixed.push_back(t);
       const uint64_t nwork = 1ull << (n - LOG - fixed.size());
-      launch_pdl(k_pair_strided<R>, grid_for(nwork, kThreads, env.num_sms), kThreads, 0, env.stream,
+      launch_pdl(k_pair_strided<R>, grid_for(nwork, kThreads, env.num_sms), kThreads, 0, env,
           re, im, nwork, make_enum(fixed, set, env.flip(nwork)), t, low, g);
     }
   } else {
     std::vector<uint32_t> fixed(ctrl, ctrl + nctrl);
     fixed.push_back(t);
     const uint64_t nwork = 1ull << (n - fixed.size());
-    launch_pdl(k_pair_scalar<R>, grid_for(nwork, kThreads, env.num_sms), kThreads, 0, env.stream,
+    launch_pdl(k_pair_scalar<R>, grid_for(nwork, kThreads, env.num_sms), kThreads, 0, env,
         re, im, nwork, make_enum(fixed, cmask, env.flip(nwork)), t, g);
   }
   check_launch();
@@ -1165,11 +1165,11 @@ void launch_diag(const LaunchEnv& env, R* re, R* im, uint32_t n, const Sweep& s)
         set |= 1ull << s.ctrl[i];
       }
     const uint64_t nwork = 1ull << (n - LOG - fixed.size());
-    launch_pdl(k_diag<R>, grid_for(nwork, kThreads, env.num_sms), kThreads, 0, env.stream,
+    launch_pdl(k_diag<R>, grid_for(nwork, kThreads, env.num_sms), kThreads, 0, env,
         re, im, nwork, make_enum(fixed, set, env.flip(nwork)), p);
   } else {
     const uint64_t dim = 1ull << n;
-    launch_pdl(k_diag_scalar<R>, grid_for(dim, kThreads, env.num_sms), kThreads, 0, env.stream, re, im, dim, p);
+    launch_pdl(k_diag_scalar<R>, grid_for(dim, kThreads, env.num_sms), kThreads, 0, env, re, im, dim, p);
   }
   check_launch();
 }
@@ -1200,7 +1200,7 @@ void launch_dense_mma_shape(const LaunchEnv& env, R* re, R* im, uint64_t ngroups
   const uint64_t items = ngroups / G;
   p.flip = env.flip(items);
   static const int per_sm = resident_blocks(reinterpret_cast<const void*>(kern), TH, smem);
-  launch_pdl(kern, grid_for(items, TH / 32, env.num_sms, per_sm), TH, smem, env.stream, re, im, items, u, p, t);
+  launch_pdl(kern, grid_for(items, TH / 32, env.num_sms, per_sm), TH, smem, env, re, im, items, u, p, t);
   check_launch();
 }
 
@@ -1254,7 +1254,7 @@ void launch_dense_cols_at(const LaunchEnv& env, float* re, float* im, uint32_t n
   constexpr int TH = dense_cols_threads(K, L0 + L1, L2);
   const uint64_t items = 1ull << (n - K - 7);
   p.flip = env.flip(items);
-  launch_pdl(k_dense_cols<K, L0, L1, L2, TH, TAIL>, grid_for(items, TH / 32, env.num_sms, 1), TH, 0, env.stream, re, im,
+  launch_pdl(k_dense_cols<K, L0, L1, L2, TH, TAIL>, grid_for(items, TH / 32, env.num_sms, 1), TH, 0, env, re, im,
              items, reinterpret_cast<const float2*>(u), p, t);
   check_launch();
 }
@@ -1304,7 +1304,7 @@ void launch_dense_of(const LaunchEnv& env, R* re, R* im, uint32_t n, const Sweep
   if (n < uint32_t(K + 3)) {
     if constexpr (!TAIL) {  // (attach_diagonals leaves such states alone)
       const uint64_t nb = 1ull << (n - K);
-      launch_pdl(k_dense_small<R, K>, grid_for(nb, 128, env.num_sms), 128, 0, env.stream, re, im, nb, u, make_enum(std::vector<uint32_t>(q, q + K), 0), q[0], q[1], q[2], q[3], q[4], q[5]);
+      launch_pdl(k_dense_small<R, K>, grid_for(nb, 128, env.num_sms), 128, 0, env, re, im, nb, u, make_enum(std::vector<uint32_t>(q, q + K), 0), q[0], q[1], q[2], q[3], q[4], q[5]);
       check_launch();
       return;
     }
@@ -1481,7 +1481,7 @@ void launch_sweep(const LaunchEnv& env, R* re, R* im, uint32_t n, const Sweep& s
 
 template <class R> void launch_init_basis(const LaunchEnv& e, R* re, R* im, uint32_t n, uint64_t basis) {
   const uint64_t dim = 1ull << n;
-  launch_pdl(k_init_basis<R>, grid_for(dim / VecT<R>::N + 1, kThreads, e.num_sms), kThreads, 0, e.stream, re, im, dim, basis);
+  launch_pdl(k_init_basis<R>, grid_for(dim / VecT<R>::N + 1, kThreads, e.num_sms), kThreads, 0, e, re, im, dim, basis);
 }
 
 template <class R> void launch_init_gaussian(const LaunchEnv& e, R* re, R* im, uint32_t n, uint64_t seed) {
@@ -1508,7 +1508,7 @@ void launch_reduce(const LaunchEnv& e, int op, const R* re, const R* im, const R
                    uint32_t n, uint64_t mask, double* partials, double* d_out) {
   const uint64_t dim = 1ull << n;
   const unsigned grid = grid_for(dim / VecT<R>::N + 1, kThreads, e.num_sms, kReduceBlocksPerSM);
-  launch_pdl(k_reduce<R>, grid, kThreads, 0, e.stream, op, re, im, re2, im2, dim, mask, partials,
+  launch_pdl(k_reduce<R>, grid, kThreads, 0, e, op, re, im, re2, im2, dim, mask, partials,
              reduce_counter(e, partials), d_out, e.err_flag);
 }
 
@@ -1517,7 +1517,7 @@ void launch_inner_mixed(const LaunchEnv& e, const RA* are, const RA* aim, const 
                         double* partials, double* d_out) {
   const uint64_t dim = 1ull << n;
   const unsigned grid = grid_for(dim / 4 + 1, kThreads, e.num_sms, kReduceBlocksPerSM);
-  launch_pdl(k_inner_mixed<RA, RB>, grid, kThreads, 0, e.stream, are, aim, bre, bim, dim, partials,
+  launch_pdl(k_inner_mixed<RA, RB>, grid, kThreads, 0, e, are, aim, bre, bim, dim, partials,
              reduce_counter(e, partials), d_out, e.err_flag);
 }
 template void launch_inner_mixed<float, double>(const LaunchEnv&, const float*, const float*, const double*,

@@ -198,6 +198,8 @@ struct LaunchEnv {
   // Walk the state from its end: the contexts' sweeps alternate, so that a sweep starts on what the one
   // before it touched last, which is still in L2 (24 qubits complex64, a 134 MB state, gate by gate: 2.63 -> 2.19 ms for 71 gates).
   bool reverse = false;
+  // Whether launch_pdl launches programmatically (qsvb_ctx::next_env).
+  bool early = true;
   uint64_t flip(uint64_t items) const { return reverse ? items - 1 : 0; }  // XOR on the index (items = 2^k)
 };
 
@@ -268,9 +270,9 @@ namespace qsvb {
 __device__ __forceinline__ void early_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_prior() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Launches a kernel that calls early_next and wait_prior (see there).
+// Launches a kernel that calls early_next and wait_prior (see there), programmatically if the environment says so.
 template <class... P, class... A>
-void launch_pdl(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, A&&... args) {
+void launch_pdl(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, const LaunchEnv& env, A&&... args) {
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
@@ -278,9 +280,9 @@ void launch_pdl(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, 
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
+  cfg.stream = env.stream;
   cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = env.early ? 1 : 0;
   QSVB_CK(cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...));
 }
 #endif
@@ -333,7 +335,24 @@ struct qsvb_ctx {
   cudaEvent_t pin_ev[2] = {nullptr, nullptr};
   bool reverse = false;           // direction of the next sweep (LaunchEnv::reverse)
   bool stream_shared = false;     // qsvb_stream handed the stream out, so a caller may capture it
+  bool tensor_last = false;       // the last sweep was one of the tensor-core kernels
+  uint32_t bits_last = 0;         // and touched 2^bits_last amplitudes
   qsvb::LaunchEnv env() const { return {stream, num_sms, d_err, reverse}; }
+  // The environment of the stream's next kernel, which touches 2^bits amplitudes. tensor: k_tc_dense or k_tc_chain,
+  // whose one block an SM takes nearly all of its memory as shared memory. Next to a kernel of the other kind such
+  // a one is launched ordinarily once both are large: an SM changes its split only when it is idle, so blocks
+  // started among the last of the kernel before run with the wrong one for good, which costs a share of the
+  // sweep, where the launch saved is a few us. Two sweeps in turn, complex64, k_tc_dense (k = 6) and k_dense_cols
+  // (k = 4), programmatic -> ordinary: 28 qubits 1.61 -> 1.40 ms, 26 qubits 416 -> 371 us, 25 qubits 217 -> 193
+  // us, 24 qubits 110 -> 108 us (with k_dense_mma or k_diag there, 2 to 8 us more), 22 qubits 40 -> 42 us.
+  qsvb::LaunchEnv next_env(uint32_t bits, bool tensor = false) {
+    constexpr uint32_t kMixedOrdinary = 25;
+    qsvb::LaunchEnv e = env();
+    e.early = tensor == tensor_last || bits < kMixedOrdinary || bits_last < kMixedOrdinary;
+    tensor_last = tensor;
+    bits_last = bits;
+    return e;
+  }
 };
 
 namespace qsvb {

@@ -1233,7 +1233,7 @@ void launch_tc_chain(const LaunchEnv& env, float* re, float* im, uint32_t n, con
                                int(cudaSharedmemCarveoutMaxShared)));
   // one persistent CTA per SM (the tensor-memory allocation of 512 columns assumes it)
   const unsigned grid = unsigned(std::max<uint64_t>(1, std::min<uint64_t>(ntiles, uint64_t(env.num_sms))));
-  launch_pdl(kern, grid, kThreads, kChainSmem, env.stream, re, im, ntiles, static_cast<const uint4*>(dev_mat), p,
+  launch_pdl(kern, grid, kThreads, kChainSmem, env, re, im, ntiles, static_cast<const uint4*>(dev_mat), p,
              env.err_flag, lay.maps[0], lay.maps[1]);
 }
 
@@ -1258,7 +1258,7 @@ void launch_permute(const LaunchEnv& env, R* re, R* im, uint32_t n, const Sweep&
   QSVB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_permute_tiles<R>, kPermThreads, smem));
   QSVB_REQUIRE(occ >= 1, "permutation kernel does not fit on an SM");
   const unsigned grid = unsigned(std::max<uint64_t>(1, std::min<uint64_t>(ntiles, uint64_t(env.num_sms) * occ)));
-  launch_pdl(k_permute_tiles<R>, grid, kPermThreads, smem, env.stream, re, im, ntiles, p);
+  launch_pdl(k_permute_tiles<R>, grid, kPermThreads, smem, env, re, im, ntiles, p);
 }
 template void launch_permute<float>(const LaunchEnv&, float*, float*, uint32_t, const Sweep&);
 template void launch_permute<double>(const LaunchEnv&, double*, double*, uint32_t, const Sweep&);

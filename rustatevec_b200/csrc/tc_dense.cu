@@ -773,7 +773,7 @@ static void launch_tc_k(const LaunchEnv& env, float* re, float* im, uint32_t n, 
   long long* prof = nullptr;
   if (profile) QSVB_CK(cudaMalloc(&prof, sizeof(long long) * 12 * grid));
   if (prof) QSVB_CK(cudaMemsetAsync(prof, 0, sizeof(long long) * 12 * grid, env.stream));
-  launch_pdl(kern, grid, kTcThreads, kTcSmem, env.stream, re, im, ntiles, static_cast<const uint4*>(dev_mat), p,
+  launch_pdl(kern, grid, kTcThreads, kTcSmem, env, re, im, ntiles, static_cast<const uint4*>(dev_mat), p,
              env.err_flag, prof, lay.maps[0], lay.maps[1]);
   if (prof) {
     std::vector<long long> h(12 * size_t(grid));
