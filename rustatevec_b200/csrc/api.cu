@@ -190,7 +190,8 @@ void* ring_upload(qsvb_ctx* c, const void* src, size_t bytes) {
 }
 
 void run_sweep(qsvb_ctx* c, qsvb_state* st, const Sweep& s, const void* dev_mat, bool tail = false) {
-  const LaunchEnv env = c->next_env(st->n_qubits - s.nctrl, s.kind == SK_DENSE_TC || s.kind == SK_TC_CHAIN);
+  const LaunchEnv env = c->next_env(st->n_qubits - s.nctrl, s.kind == SK_DENSE_TC || s.kind == SK_TC_CHAIN,
+                                   s.kind == SK_DIAG);
   by_dtype(st->dtype, [&](auto r) {
     using R = decltype(r);
     launch_sweep<R>(env, static_cast<R*>(st->re), static_cast<R*>(st->im), st->n_qubits, s, dev_mat, tail);

@@ -1200,7 +1200,15 @@ void launch_dense_mma_shape(const LaunchEnv& env, R* re, R* im, uint64_t ngroups
   const uint64_t items = ngroups / G;
   p.flip = env.flip(items);
   static const int per_sm = resident_blocks(reinterpret_cast<const void*>(kern), TH, smem);
-  launch_pdl(kern, grid_for(items, TH / 32, env.num_sms, per_sm), TH, smem, env, re, im, items, u, p, t);
+  // After k_diag a large K = 4 sweep launches ordinarily: that kernel's 0.5 or 1 KB a block leave the SM a split
+  // with room for one of these blocks' matrices, not three, and an SM that holds one keeps the split, so blocks
+  // started early found SMs with one or two and the others waited for a second wave. A CZ and such a sweep,
+  // complex128, programmatic -> ordinary: 28 qubits 2.25 -> 1.81 ms, 25 qubits 267 -> 225 us, 23 qubits 67 -> 62
+  // us; at 22 qubits the saved launch counts for more (30 -> 32 us). K = 2, 3 fit as they are, K = 5, 6 not at all.
+  LaunchEnv e = env;
+  if constexpr (sizeof(R) == 8 && K == 4 && G > 1)
+    e.early = e.early && !(env.after_diag && items * G * 8 * (1u << K) >= uint64_t(1) << 23);
+  launch_pdl(kern, grid_for(items, TH / 32, env.num_sms, per_sm), TH, smem, e, re, im, items, u, p, t);
   check_launch();
 }
 

@@ -200,6 +200,7 @@ struct LaunchEnv {
   bool reverse = false;
   // Whether launch_pdl launches programmatically (qsvb_ctx::next_env).
   bool early = true;
+  bool after_diag = false;  // the kernel before is k_diag (launch_dense_mma_shape)
   uint64_t flip(uint64_t items) const { return reverse ? items - 1 : 0; }  // XOR on the index (items = 2^k)
 };
 
@@ -336,20 +337,24 @@ struct qsvb_ctx {
   bool reverse = false;           // direction of the next sweep (LaunchEnv::reverse)
   bool stream_shared = false;     // qsvb_stream handed the stream out, so a caller may capture it
   bool tensor_last = false;       // the last sweep was one of the tensor-core kernels
+  bool diag_last = false;         // or k_diag
   uint32_t bits_last = 0;         // and touched 2^bits_last amplitudes
   qsvb::LaunchEnv env() const { return {stream, num_sms, d_err, reverse}; }
-  // The environment of the stream's next kernel, which touches 2^bits amplitudes. tensor: k_tc_dense or k_tc_chain,
+  // The environment of the stream's next kernel, which touches 2^bits amplitudes. diag: k_diag (see
+  // launch_dense_mma_shape). tensor: k_tc_dense or k_tc_chain,
   // whose one block an SM takes nearly all of its memory as shared memory. Next to a kernel of the other kind such
   // a one is launched ordinarily once both are large: an SM changes its split only when it is idle, so blocks
   // started among the last of the kernel before run with the wrong one for good, which costs a share of the
   // sweep, where the launch saved is a few us. Two sweeps in turn, complex64, k_tc_dense (k = 6) and k_dense_cols
   // (k = 4), programmatic -> ordinary: 28 qubits 1.61 -> 1.40 ms, 26 qubits 416 -> 371 us, 25 qubits 217 -> 193
   // us, 24 qubits 110 -> 108 us (with k_dense_mma or k_diag there, 2 to 8 us more), 22 qubits 40 -> 42 us.
-  qsvb::LaunchEnv next_env(uint32_t bits, bool tensor = false) {
+  qsvb::LaunchEnv next_env(uint32_t bits, bool tensor = false, bool diag = false) {
     constexpr uint32_t kMixedOrdinary = 25;
     qsvb::LaunchEnv e = env();
     e.early = tensor == tensor_last || bits < kMixedOrdinary || bits_last < kMixedOrdinary;
+    e.after_diag = diag_last;
     tensor_last = tensor;
+    diag_last = diag;
     bits_last = bits;
     return e;
   }
