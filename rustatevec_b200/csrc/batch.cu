@@ -767,7 +767,7 @@ __global__ void __launch_bounds__(NT, MINB)
             const PhaseDev* __restrict__ phases, const Instr* __restrict__ prog, const R* __restrict__ coef,
             R* __restrict__ sre, R* __restrict__ sim, double* __restrict__ probs, double* __restrict__ zpart,
             uint32_t* __restrict__ done, uint32_t* __restrict__ queue, int* __restrict__ err, uint32_t lbits,
-            long long* __restrict__ prof, uint32_t fixed, const long long* __restrict__ wait_budget) {
+            long long* __restrict__ prof, uint32_t order, const long long* __restrict__ wait_budget) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   R* xr = reinterpret_cast<R*>(smem_raw);
   const uint32_t cap = TILE ? uint32_t(HI) << W : 1u << lbits;  // every pass has nlocal <= lbits
@@ -792,23 +792,27 @@ __global__ void __launch_bounds__(NT, MINB)
       if ((h >> i) & 1u) v ^= swz_col(W + i, W);
     if (QSVB_BC(h < uint32_t(HI), err)) s_swz[h] = uint16_t(v);
   }
-  long long t_wait = 0, t_fill = 0, t_gates = 0, t_out = 0, n_items = 0, t_mark = prof ? clock64() : 0;
+  const bool timed = !TILE && prof != nullptr;
+  long long t_wait = 0, t_fill = 0, t_gates = 0, t_out = 0, n_items = 0, t_mark = timed ? clock64() : 0;
   uint32_t staged_pass = ~0u;
-  // fixed != 0: one pass (passes[0]) over one state, tile i (bit 1: from the last one) handled by block i mod
-  // grid, no queue
+  // TILE: one pass (passes[0]) over one state, tile i (order 2: from the last one) handled by block i mod grid, no
+  // queue. Batches are launched with order 0, but test it at run time: knowing the queue to be the only source, the
+  // compiler keeps more of an item in registers and the 512-thread variants spill (512 ansatz circuits, complex64,
+  // 14 local and 4 register qubits: 15.6 against 18.7 ms; 13 and 3, complex128: 34.7 against 37.1). Tile sweeps
+  // without the queue's code: 30-qubit brickwork, 28 passes, 478 -> 469 ms.
   uint32_t iter = 0;
   while (true) {
-    if (!fixed && tid == 0) s_item = atomicAdd(queue, 1u);
+    if (!TILE && tid == 0) s_item = atomicAdd(queue, 1u);
     __syncthreads();
-    const uint32_t it = fixed ? blockIdx.x + (iter++) * gridDim.x : s_item;
+    const uint32_t it = (TILE || order) ? blockIdx.x + (iter++) * gridDim.x : s_item;
     if (it >= nitems) break;
-    const Item item = fixed ? Item{0u, (fixed & 2u) ? nitems - 1u - it : it} : items[it];
+    const Item item = (TILE || order) ? Item{0u, (order & 2u) ? nitems - 1u - it : it} : items[it];
     const PassDev& P = passes[item.pass];
     const uint32_t L = P.nlocal, T = 1u << L;
     [[maybe_unused]] const uint64_t gsize = 1ull << (L + P.nnon);  // the circuit's amplitudes (checked builds)
     if (tid == 0) {
       int ok = *reinterpret_cast<volatile int*>(err) == 0;
-      if (ok && P.prev != ~0u) {
+      if (!TILE && ok && P.prev != ~0u) {
         cuda::atomic_ref<uint32_t, cuda::thread_scope_device> d(done[P.prev]);
         const uint32_t need = passes[P.prev].ntiles;
         if (d.load(cuda::memory_order_acquire) < need) {
@@ -842,14 +846,14 @@ __global__ void __launch_bounds__(NT, MINB)
       }
     }
     __syncthreads();
-    if (prof) t_wait += clock64() - t_mark, t_mark = clock64(), ++n_items;
+    if (timed) t_wait += clock64() - t_mark, t_mark = clock64(), ++n_items;
     if (!s_ok) continue;
     // the pass's instructions, phases and coefficients into shared memory (kept while the next
     // item is a tile of the same pass), overlapped with the tile fill
     const uint32_t ph_bytes = P.prog_len * uint32_t(sizeof(Instr));
     const uint32_t co_bytes = (ph_bytes + P.nphase * uint32_t(sizeof(PhaseDev)) + 15u) & ~15u;  // (double2 reads)
     if (P.staged && staged_pass != item.pass &&
-        QSVB_BC(co_bytes + P.ncoef * 2u * uint32_t(sizeof(R)) <= (fixed ? kTileStageBytes : kStageBytes), err)) {
+        QSVB_BC(co_bytes + P.ncoef * 2u * uint32_t(sizeof(R)) <= (TILE ? kTileStageBytes : kStageBytes), err)) {
       const uint32_t* src0 = reinterpret_cast<const uint32_t*>(prog + P.prog_off);
       const uint32_t* src1 = reinterpret_cast<const uint32_t*>(phases + P.phase_off);
       const uint32_t* src2 = reinterpret_cast<const uint32_t*>(coef + 2 * size_t(P.coef_off));
@@ -867,7 +871,7 @@ __global__ void __launch_bounds__(NT, MINB)
     const uint32_t lowmask = L >= 5 ? 31u : (T - 1u);
     R* gre = sre + P.state_off;
     R* gim = sim + P.state_off;
-    if (P.first) {
+    if (!TILE && P.first) {
       for (uint32_t x = tid; x < T; x += NT) {
         xr[x] = R(0);
         xi[x] = R(0);
@@ -977,7 +981,7 @@ __global__ void __launch_bounds__(NT, MINB)
       }
       __syncthreads();
     }
-    if (prof) t_fill += clock64() - t_mark, t_mark = clock64();
+    if (timed) t_fill += clock64() - t_mark, t_mark = clock64();
     // register phases: each group of 2^r amplitudes (fixed non-register bits) is loaded into one
     // thread's registers, takes all of the phase's gates there, and is written back
     uint32_t k = 0;
@@ -1013,8 +1017,8 @@ __global__ void __launch_bounds__(NT, MINB)
       k = kend;
       __syncthreads();
     }
-    if (prof) t_gates += clock64() - t_mark, t_mark = clock64();
-    if (P.last) {
+    if (timed) t_gates += clock64() - t_mark, t_mark = clock64();
+    if (!TILE && P.last) {
       // FP64 probabilities and the <Z_0> partial (state bit 0 is local position 0)
       double z = 0.0;
       double* pout = probs + P.prob_off;
@@ -1061,14 +1065,14 @@ __global__ void __launch_bounds__(NT, MINB)
       }
     }
     __syncthreads();
-    if (tid == 0 && !fixed) {
+    if (!TILE && tid == 0) {
       __threadfence();
       cuda::atomic_ref<uint32_t, cuda::thread_scope_device> d(done[item.pass]);
       d.fetch_add(1u, cuda::memory_order_release);
     }
-    if (prof) t_out += clock64() - t_mark, t_mark = clock64();
+    if (timed) t_out += clock64() - t_mark, t_mark = clock64();
   }
-  if (prof && tid == 0) {
+  if (timed && tid == 0) {
     long long* o = prof + 5 * blockIdx.x;
     o[0] = t_wait;
     o[1] = t_fill;
