@@ -123,6 +123,9 @@ int qsvb_stream(qsvb_ctx* ctx, void** stream_out);
 
 /* Backend::alloc (mod.rs:36; lib.rs:100-107). Contents unspecified until init/upload. */
 int qsvb_state_alloc(qsvb_ctx* ctx, uint32_t n_qubits, int dtype, qsvb_state** out);
+/* Waits for the context's queued work. The context keeps the memory of small states for its next ones (at most
+ * 64 MB; not of states whose pointers were handed out or that another context used) and, likewise, the sampler's
+ * scratch; it frees both before an allocation of its own would fail, and when it is destroyed. */
 int qsvb_state_free(qsvb_ctx* ctx, qsvb_state* st);
 /* Shape of a state and its device SoA pointers (re[2^n], im[2^n]). */
 int qsvb_state_info(const qsvb_state* st, uint32_t* n_qubits, int* dtype, void** d_re, void** d_im);

@@ -2459,7 +2459,7 @@ void tile_prepare(Sweep& s, uint32_t n, int dtype) {
   std::vector<double> tdat;
   // per operation: type, the factors of both sides with no tile bit set, the term count, then per
   // term (tile bit k, tile bit l, factor of side 0, factor of side 1) applied when bits k and l
-  // are set, then the register-bit-0 flag
+  // are set
   for (const TphOp& op : tph) {
     toffs.push_back(uint32_t(tdat.size()));
     tdat.push_back(double(op.type));

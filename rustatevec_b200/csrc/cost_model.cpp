@@ -31,8 +31,12 @@ constexpr double kTileFp64Flops = 15.5e12;
 constexpr double kTileMemFactor32 = 1.95;
 constexpr double kTileMemFactor64 = 1.80;
 // the same form with a trained model installed, fitted to the kernels the model's records were taken on (411
-// passes of QFT, brickwork, QAOA, GHZ and random circuits at 22-30 qubits: mean |log2 error| 0.16 / 0.15, where
-// the constants above, which the planner without a model keeps, are off by 0.18 / 0.43)
+// tile passes of QFT, brickwork, QAOA, GHZ and random circuits at 22-30 qubits, each one's time from
+// qsvb_plan_profile against its bytes and flops from qsvb_plan_sweep_info: mean |log2 error| 0.16 / 0.15, where
+// the constants above are off by 0.18 / 0.43). The planner without a model keeps those above: it is what the
+// trained planner is compared with. Tile passes are no input of the network, so where plans of QAOA and GHZ
+// circuits gain from an installed model, these constants and not the network are why: with them in both, both
+// planners choose the same plans there (26 qubits complex128: QAOA 8.5 -> 7.4 ms, GHZ 2.86 -> 2.48 ms).
 constexpr double kTrainedTileFp32Flops = 31.0e12;
 constexpr double kTrainedTileFp64Flops = 19.7e12;
 constexpr double kTrainedTileMemFactor32 = 1.72;

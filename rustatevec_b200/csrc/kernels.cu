@@ -2,9 +2,9 @@
 //
 // Layout: the state is Structure-of-Arrays, re[2^n] and im[2^n] in HBM, the layout qsv's
 // StateVector uses (crates/qsv-core/src/state/mod.rs:25-29) so `download` is a straight copy.
-// Every kernel here is HBM-bound except the dense k>=4 sweeps; each moves 16-byte vectors
-// (4 x f32 or 2 x f64 amplitudes per component) and walks the state with a grid-stride loop
-// sized to a multiple of the SM count.
+// Every kernel here is HBM-bound except the dense sweeps of five and six qubits (FP64 pipe); each moves
+// whole 32-byte sectors, most of them as 16-byte vectors (4 x f32 or 2 x f64 amplitudes per component), and
+// walks the state with a grid-stride loop sized to a multiple of the SM count.
 //
 // Index math follows qsv's layout helpers (crates/qsv-core/src/state/layout.rs:22-86):
 // insert_zero_bit(s) anchors a pair/block, scatter_bits/gather_bits map a gate sub-index to
@@ -1056,8 +1056,8 @@ __global__ void k_probs(const R* __restrict__ re, const R* __restrict__ im, uint
 // ---------------------------------------------------------------------------------------------
 // Blocks of a kernel an SM holds at a time. A grid of persistent blocks launched programmatically has to fill
 // every SM: its blocks start wherever the kernel before it leaves room, so with fewer of them than fit, the SMs
-// that finish first take more than their share (26-qubit complex128 two-qubit sweeps, 3 blocks an SM where 4 or
-// fit, back to back: 413 us against 337 us alone).
+// that finish first take more than their share (26-qubit complex128 two-qubit sweeps back to back, three
+// blocks an SM where four fit: 413 us a sweep, against 337 us alone).
 inline int resident_blocks(const void* kern, int threads, size_t smem) {
   int blocks = 0;
   QSVB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, threads, smem));
