@@ -306,7 +306,7 @@ std::vector<Gate> learned_fuse(const std::vector<Gate>& seg, uint32_t n, const q
       if (s.kind != SK_NONE) sw.push_back(std::move(s));
     }
     select_engines(sw, n, o, dtype);
-    return predict_plan_seconds(sw, n, dtype, true);
+    return predict_plan_seconds(sw, n, dtype, !o.diagonals_apart);
   };
   const size_t ncand = 2 * size_t(cap);
   std::vector<double> secs(ncand, 1e300);

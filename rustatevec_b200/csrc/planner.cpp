@@ -459,7 +459,7 @@ std::vector<Sweep> plan_sweeps(const std::vector<Gate>& in, uint32_t n, const qs
     double best_t = 1e300;
     for (uint32_t m = 1; m <= uint32_t(kChainMaxMats); ++m) {
       std::vector<Sweep> cand = plan_chain(in, n, m);
-      const double t = predict_plan_seconds(cand, n, dtype, true);
+      const double t = predict_plan_seconds(cand, n, dtype, !o.diagonals_apart);
       if (t < best_t) {
         best_t = t;
         best = std::move(cand);
@@ -492,7 +492,7 @@ std::vector<Sweep> plan_sweeps(const std::vector<Gate>& in, uint32_t n, const qs
   double best_t = 1e300;
   for (size_t c = 0; c < fut.size(); ++c) {
     std::vector<Sweep> cand = fut[c].get();
-    const double t = predict_plan_seconds(cand, n, dtype, true);
+    const double t = predict_plan_seconds(cand, n, dtype, !o.diagonals_apart);
     if (t < best_t) {
       best_t = t;
       best = std::move(cand);
@@ -585,7 +585,7 @@ void tile_segment(const std::vector<Gate>& seg, uint32_t n, const qsvb_plan_opts
           std::vector<Sweep> alt = fused_sweeps(t.tile_gates, n, o, dtype);
           select_engines(alt, n, o, dtype);
           tile_prepare(t, n, dtype);
-          if (predict_plan_seconds(alt, n, dtype, true) <= predict_sweep_seconds(t, n, dtype)) {
+          if (predict_plan_seconds(alt, n, dtype, !o.diagonals_apart) <= predict_sweep_seconds(t, n, dtype)) {
             res[i] = std::move(alt);
             continue;
           }

@@ -126,3 +126,18 @@ def test_carried_diagonals_cost_nothing(built, dtype):
     pc = L.PackedCircuit(both)
     L.check(L.lib().qsvb_plan_dry_run(pc.ref(), dtype, C.byref(apart), C.byref(st)))
     assert st.to_dict() == given
+
+
+def test_learned_planner_with_diagonals_apart_charges_every_diagonal(built):
+    """With diagonals_apart the candidates are weighed as they would run, so the chosen plan is predicted no slower
+    than any of them; weighed with carried diagonals for free, a plan of 38 % more seconds won."""
+    def apart(planner, k):
+        o, st = L.make_opts(planner, k, L.ENGINE_CUDA_CORE), L.PlanStats()
+        o.diagonals_apart = 1
+        L.check(L.lib().qsvb_plan_dry_run(pc.ref(), L.C64, C.byref(o), C.byref(st)))
+        return st.to_dict()["predicted_seconds"]
+
+    tuning.install(None)
+    pc = L.PackedCircuit(qaoa_maxcut(24, 2, 3))
+    best = min([apart(L.PLAN_TILE, 4)] + [apart(p, k) for p in (L.PLAN_GREEDY, L.PLAN_WINDOW) for k in range(1, 7)])
+    assert apart(L.PLAN_LEARNED, 6) <= best
